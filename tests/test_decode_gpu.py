@@ -41,6 +41,32 @@ def test_device_packer_bit_exact():
         assert np.array_equal(scales.cpu().numpy(), want_scales), enc
 
 
+@pytest.mark.parametrize("enc", ["q4_group128", "q8_group128"])
+@pytest.mark.parametrize("groups,offset", [(1, 0), (7, 4), (64, 8), (131, 0), (1029, 4)])
+def test_device_packer_rounding_boundaries_and_layouts(enc, groups, offset):
+    """Ties and their neighbours, subnormal groups and chunks of a fused tensor; 8- and 16-byte aligned sources, group
+    counts around a block's 64: bit-exact against the oracle, which divides."""
+    ops = _ops()
+    quant, qmax = (orc.quantize_q4, 7) if enc == "q4_group128" else (orc.quantize_q8, 127)
+    rng = np.random.default_rng(groups)
+    n = groups * 128
+    v = torch.from_numpy(rng.standard_normal((2, n)).astype(np.float32)).to(torch.bfloat16)
+    flat = v.reshape(-1, 128)
+    for g in range(0, len(flat), 3):                         # scale a power of two: (k + 1/2) * scale is a tie
+        half = torch.from_numpy((rng.integers(-2 * qmax, 2 * qmax + 1, 128) / 2).astype(np.float32))
+        half[5] = qmax
+        flat[g] = (half * 2.0 ** int(rng.integers(-20, 20))).to(torch.bfloat16)
+    flat[1] = (flat[1].float() * 2.0 ** -127).to(torch.bfloat16)        # subnormal weights and scale
+    want = [quant(part.float().numpy()) for part in v]
+    store = torch.zeros(offset + 2 * (n + 128), dtype=torch.bfloat16, device=DEV)
+    chunks = torch.as_strided(store, (2, groups, 128), (n + 128, 128, 1), offset)
+    chunks.copy_(v.reshape(2, groups, 128))
+    for codes, scales in (ops.quantize_chunks(chunks, enc), ops.quantize_groups(chunks.contiguous(), enc)):
+        got = codes.cpu().numpy().view(np.uint8)
+        assert np.array_equal(got, np.concatenate([np.asarray(c).view(np.uint8).reshape(-1) for c, _ in want]))
+        assert np.array_equal(scales.cpu().numpy(), np.concatenate([s for _, s in want]))
+
+
 def test_olmoe_decode_golden(golden_dir):
     g = np.load(golden_dir / "olmoe_decode.npz")
     x = bits_to_bf16(g["x_bits"])

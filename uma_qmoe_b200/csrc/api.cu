@@ -105,7 +105,13 @@ int umaq_moe_decode(const umaq_layer* layer, const umaq_shared_expert* shared, c
 
 int umaq_quantize_groups(const void* src_bf16, long long elements, int encoding, void* codes, float* scales,
                          void* stream) {
-  return launch_quantize_groups(src_bf16, elements, encoding, codes, scales, static_cast<cudaStream_t>(stream));
+  return launch_quantize_groups(src_bf16, elements, 1, 0, encoding, codes, scales, static_cast<cudaStream_t>(stream));
+}
+
+int umaq_quantize_chunks(const void* src_bf16, long long chunk_elements, long long chunks, long long chunk_stride, int encoding,
+                         void* codes, float* scales, void* stream) {
+  return launch_quantize_groups(src_bf16, chunk_elements, chunks, chunk_stride, encoding, codes, scales,
+                                static_cast<cudaStream_t>(stream));
 }
 
 int umaq_route_topk(const void* hidden_bf16, const void* router_weight_bf16, int tokens, int hidden, int experts,

@@ -55,13 +55,11 @@ def encode_experts(gate_up_proj: torch.Tensor, down_proj: torch.Tensor, encoding
     inter = two_i // 2
     if down_proj.shape != (experts, hidden, inter):
         raise RuntimeError(f"down_proj has shape {tuple(down_proj.shape)}, expected {(experts, hidden, inter)}")
-    gate = gate_up_proj[:, :inter, :].contiguous()
-    up = gate_up_proj[:, inter:, :].contiguous()
-    down = down_proj.contiguous()
+    gate, up, down = gate_up_proj[:, :inter, :], gate_up_proj[:, inter:, :], down_proj
     if encoding == "bf16_le":
-        as_bytes = lambda t: t.reshape(-1).view(torch.uint8)
+        as_bytes = lambda t: t.contiguous().reshape(-1).view(torch.uint8)
         return DeviceLayer(encoding, experts, hidden, inter, as_bytes(gate), as_bytes(up), as_bytes(down), None, None, None)
-    (g, gs), (u, us), (d, ds) = (ops.quantize_groups(t.reshape(-1), encoding) for t in (gate, up, down))
+    (g, gs), (u, us), (d, ds) = (ops.quantize_chunks(t, encoding) for t in (gate, up, down))
     return DeviceLayer(encoding, experts, hidden, inter, g, u, d, gs, us, ds)
 
 

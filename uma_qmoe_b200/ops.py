@@ -379,14 +379,33 @@ def workspace_status(workspace: torch.Tensor) -> int:
 def quantize_groups(values: torch.Tensor, encoding: str) -> tuple[torch.Tensor, torch.Tensor]:
     """Device-side packer: BF16 tensor -> (canonical codes as uint8/int8, float32 scales)."""
     _require_cuda_bf16(values, "values")
+    codes, scales, enc = _packed_like(values, encoding)
+    code = _native.lib().umaq_quantize_groups(values.data_ptr(), values.numel(), enc, codes.data_ptr(), scales.data_ptr(),
+                                              _stream(values.device))
+    _native.check(code, "umaq_quantize_groups")
+    return codes, scales
+
+
+def quantize_chunks(values: torch.Tensor, encoding: str) -> tuple[torch.Tensor, torch.Tensor]:
+    """:func:`quantize_groups` of a ``[chunks, rows, k]`` view whose chunks are each contiguous (one projection inside a
+    fused tensor) without a copy of it; any other layout is copied first."""
+    chunks, rows, k = values.shape
+    if (values.stride(2) != 1 or values.stride(1) != k or values.stride(0) < rows * k or rows * k % 128 or
+            not 1 <= chunks <= 65535):
+        return quantize_groups(values.contiguous().reshape(-1), encoding)
+    _require_cuda_bf16(values[0], "values")
+    codes, scales, enc = _packed_like(values, encoding)
+    code = _native.lib().umaq_quantize_chunks(values.data_ptr(), rows * k, chunks, values.stride(0), enc, codes.data_ptr(),
+                                              scales.data_ptr(), _stream(values.device))
+    _native.check(code, "umaq_quantize_chunks")
+    return codes, scales
+
+
+def _packed_like(values: torch.Tensor, encoding: str) -> tuple[torch.Tensor, torch.Tensor, int]:
     n = values.numel()
     enc = ENCODING_ID[encoding]
     if enc == ENC_BF16:
         raise RuntimeError("bf16_le needs no quantisation")
     codes = torch.empty(n // 2 if enc == ENC_Q4 else n, dtype=torch.uint8 if enc == ENC_Q4 else torch.int8,
                         device=values.device)
-    scales = torch.empty(n // 128, dtype=torch.float32, device=values.device)
-    code = _native.lib().umaq_quantize_groups(values.data_ptr(), n, enc, codes.data_ptr(), scales.data_ptr(),
-                                              _stream(values.device))
-    _native.check(code, "umaq_quantize_groups")
-    return codes, scales
+    return codes, torch.empty(n // 128, dtype=torch.float32, device=values.device), enc
