@@ -5,6 +5,7 @@
 // accumulation order of the reference's CPU path (src/uma_qmoe/custom_op.py:312-338).
 #include "grouped.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -876,6 +877,7 @@ combine_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __restric
 // order of the routes found with shuffles.  A token with one or two present routes (an expert-parallel rank's
 // share) costs a warp a few hundred cycles instead of a block three barriers.
 constexpr int kCombineWarps = 8;
+constexpr int kCombineSpreadWarps = 4736;    // 32 warps on each of 148 SMs
 __global__ void __launch_bounds__(kCombineWarps * 32)
 combine_warp_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __restrict__ indices, int idx64,
                     const int* __restrict__ route_pos, int tokens, int top_k, int hidden, int experts,
@@ -910,7 +912,7 @@ combine_warp_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __re
     rows[s] = s < n ? (unsigned)(((size_t)qs * hidden) >> 3) : 0u;
   }
   const uint4* wbase = reinterpret_cast<const uint4*>(weighted);
-  for (int c = lane; c < (hidden >> 3); c += 32) {            // 16 bytes per lane and row
+  for (int c = blockIdx.y * 32 + lane; c < (hidden >> 3); c += 32 * gridDim.y) {   // 16 bytes per lane and row
     uint4 v[8];
 #pragma unroll
     for (int s = 0; s < 8; ++s)
@@ -1037,9 +1039,12 @@ int launch_combine(const __nv_bfloat16* weighted, const void* indices, int idx64
   if (tokens <= 0 || top_k < 1 || top_k > 8 || hidden % 8) { set_error("combine: unsupported shape"); return ERR_BAD_ARGUMENT; }
   SegmentedOut seg{};
   if (segments) seg = *segments;
-  static const int warp_path = [] { const char* v = std::getenv("UMAQ_COMBINE_WARP"); return v ? std::atoi(v) : 1; }();
-  if (!shared_out && warp_path) {
-    combine_warp_kernel<<<(tokens + kCombineWarps - 1) / kCombineWarps, kCombineWarps * 32, 0, stream>>>(
+  if (!shared_out) {
+    // A warp per token leaves the device empty when the tokens are few, and its eight column passes of 2048 wide rows are
+    // a chain of load latencies (11.5 us at 7 tokens): then a token's columns are spread over several warps.
+    const int passes = (hidden / 8 + 31) / 32;
+    const int spread = std::max(1, std::min(passes, kCombineSpreadWarps / tokens));
+    combine_warp_kernel<<<dim3((tokens + kCombineWarps - 1) / kCombineWarps, spread), kCombineWarps * 32, 0, stream>>>(
         weighted, indices, idx64, route_pos, tokens, top_k, hidden, experts, out, seg);
     return check_launch("combine");
   }
