@@ -332,3 +332,78 @@ def test_stack_shape_8192_tokens_sampled_rows():
     src = lambda e: cache.setdefault(e, staged(e))
     want = orc.moe_forward(x[rows], idx_s, w_s, src, num_experts=64, top_k=8, qwen=False)
     assert_parity(y[rows], want)
+
+
+# ---- few routes per expert: the transposed kernel (grouped_ts.cu) ------------------------------------------------
+
+def _dequantised(codes, scales, encoding, experts, rows, k):
+    """The BF16 weights the tensor cores multiply, from the staged bytes."""
+    if encoding == "bf16_le":
+        return codes.view(torch.bfloat16).reshape(experts, rows, k).float()
+    raw = codes.view(torch.uint8).reshape(-1)
+    if encoding == "q4_group128":
+        q = torch.stack((raw & 15, raw >> 4), dim=1).reshape(-1).to(torch.int16)
+        scales = scales.to(torch.bfloat16).float()                      # the kernels multiply by the BF16 scale
+    else:
+        q = raw.to(torch.int16)
+    half, full = (8, 16) if encoding == "q4_group128" else (128, 256)
+    q = torch.where(q >= half, q - full, q).float().reshape(-1, 128)
+    return (q * scales.reshape(-1, 1)).to(torch.bfloat16).float().reshape(experts, rows, k)
+
+
+def _reference_layer(layer, x, expert, weight):
+    """float32 sums over the same BF16 operands, with the kernels' two roundings; one route per token."""
+    e, h, i = layer.num_experts, layer.hidden, layer.intermediate
+    gate = _dequantised(layer.gate, layer.gate_scales, layer.encoding, e, i, h)
+    up = _dequantised(layer.up, layer.up_scales, layer.encoding, e, i, h)
+    down = _dequantised(layer.down, layer.down_scales, layer.encoding, e, h, i)
+    out = torch.zeros(x.shape, dtype=torch.bfloat16, device=x.device)
+    for n in range(e):
+        rows = (expert == n).nonzero().flatten()
+        if len(rows):
+            xr = x[rows].double()
+            inter = (torch.nn.functional.silu(xr @ gate[n].double().T) * (xr @ up[n].double().T)).to(torch.bfloat16)
+            out[rows] = ((inter.double() @ down[n].double().T) * weight[rows, None]).to(torch.bfloat16)
+    return out
+
+
+@pytest.mark.parametrize("model", ["olmoe", "qwen"])
+@pytest.mark.parametrize("encoding", ["q4_group128", "q8_group128", "bf16_le"])
+@pytest.mark.parametrize("counts", [[1], [2, 0, 15], [16, 17, 1, 31, 33, 63, 64, 65], [129, 0, 7] * 4, [300, 1, 192]])
+def test_few_routes_per_expert_at_tile_edges(model, encoding, counts):
+    """Route counts around the MMA's N steps (16) and the tile (64), absent experts, experts with several tiles.  Both sides
+    round the intermediate and the output to BF16 once: they differ where a float32 sum falls on the other side of a
+    rounding boundary, by 2^-8 of the value, and by 2^-8 of single terms of a sum; a misplaced row or column is off by
+    the whole value."""
+    from uma_qmoe_b200.stack import random_layer
+    shape = syn.OLMOE if model == "olmoe" else syn.QWEN
+    layer = random_layer(shape, encoding, 3, torch.device(DEV))
+    gen = torch.Generator(device=DEV).manual_seed(sum(counts))
+    expert = torch.cat([torch.full((c,), (11 * n) % shape.experts, device=DEV) for n, c in enumerate(counts)])
+    expert = expert[torch.randperm(len(expert), device=DEV, generator=gen)]
+    x = torch.randn(len(expert), shape.hidden, device=DEV, generator=gen).to(torch.bfloat16)
+    w = torch.rand(len(expert), 1, device=DEV, generator=gen) + 0.1
+    got = _run_prefill(layer, x, expert[:, None], w).float()
+    want = _reference_layer(layer, x, expert, w[:, 0]).cpu().float()
+    assert (got - want).norm() <= 2.0 ** -8 * want.norm()
+    assert (got - want).abs().max() <= 2.0 ** -7 * want.abs().max()
+
+
+def test_few_routes_kernel_takes_tables_of_wider_tiles():
+    """The exported stage calls hand the transposed kernel tables of up to 256 routes per entry: it cuts them itself, and a
+    gathered copy of the rows gives the bits that rows fetched by index give."""
+    from uma_qmoe_b200 import ops
+    from uma_qmoe_b200.stack import random_layer
+    layer = random_layer(syn.OLMOE, "q4_group128", 4, torch.device(DEV))
+    gen = torch.Generator(device=DEV).manual_seed(2)
+    counts = [256, 257, 100, 64, 1, 80]
+    idx = torch.cat([torch.full((c, 1), 5 * n, device=DEV) for n, c in enumerate(counts)])
+    x = torch.randn(len(idx), 2048, device=DEV, generator=gen).to(torch.bfloat16)
+    w = torch.rand(len(idx), 1, device=DEV, generator=gen)
+    routes = ops.route_sort(idx, w, 64)
+    xp = ops.gather_rows(x, None, 1, permute=True)
+    xs = ops.gather_rows(x, routes.sorted_route, 1, permute=True)
+    inter = ops.grouped_gemm_by_index(layer, xp, routes, 1, permute_out=True)
+    assert torch.equal(inter, ops.grouped_gemm(layer, 0, xs, routes, permute_out=True))
+    y = ops.grouped_gemm(layer, 1, inter, routes, routes.sorted_weight)
+    assert torch.equal(ops.combine_routes(y, idx, routes.route_pos).cpu(), _run_prefill(layer, x, idx, w))

@@ -145,7 +145,7 @@ int umaq_route_sort(const void* expert_indices, int indices_are_int64, const flo
   a.counts = counts; a.offsets = offsets; a.sorted_route = sorted_route; a.route_pos = route_pos;
   a.sorted_weight = sorted_weight; a.num_tiles = num_tiles;
   a.tile_expert = tile_table; a.tile_row0 = tile_table + max_tiles; a.tile_rows = tile_table + 2 * max_tiles;
-  a.max_tiles = max_tiles; a.status = status;
+  a.max_tiles = max_tiles; a.tile_cap = kTileCapMax; a.status = status;
   a.scratch = scratch; a.scratch_ints = scratch ? scratch_ints : 0;
   return launch_route_sort(a, static_cast<cudaStream_t>(stream));
 }
@@ -173,7 +173,7 @@ int umaq_grouped_gemm(const umaq_layer* layer, int mode, const void* act_bf16, l
   if (mode == 0) { g.w0 = layer->gate; g.s0 = layer->gate_scales; g.w1 = layer->up; g.s1 = layer->up_scales; }
   else { g.w0 = layer->down; g.s0 = layer->down_scales; }
   g.num_tiles = num_tiles; g.tile_expert = tile_table; g.tile_row0 = tile_table + max_tiles;
-  g.tile_rows = tile_table + 2 * max_tiles; g.max_tiles = max_tiles;
+  g.tile_rows = tile_table + 2 * max_tiles; g.max_tiles = max_tiles; g.tile_cap = kTileCapMax;
   g.out = static_cast<__nv_bfloat16*>(out_bf16); g.out_stride = g.n_rows;
   g.route_weight = route_weight; g.permute_out = permute_out; g.status = status; g.variant = variant;
   return launch_grouped_gemm(g, static_cast<cudaStream_t>(stream));
@@ -192,7 +192,7 @@ int umaq_grouped_gemm_by_index(const umaq_layer* layer, const void* hidden_bf16,
   g.act = hidden_bf16; g.total_rows = routes;
   g.w0 = layer->gate; g.s0 = layer->gate_scales; g.w1 = layer->up; g.s1 = layer->up_scales;
   g.num_tiles = num_tiles; g.tile_expert = tile_table; g.tile_row0 = tile_table + max_tiles;
-  g.tile_rows = tile_table + 2 * max_tiles; g.max_tiles = max_tiles;
+  g.tile_rows = tile_table + 2 * max_tiles; g.max_tiles = max_tiles; g.tile_cap = kTileCapMax;
   g.out = static_cast<__nv_bfloat16*>(out_bf16); g.out_stride = g.n_rows;
   g.permute_out = permute_out; g.status = status; g.variant = 1;
   g.gather_route = sorted_route; g.gather_top_k = top_k;
@@ -260,8 +260,8 @@ size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 PrefillPlan prefill_plan(long long tokens, int top_k, int experts, int hidden, int inter, int shared_inter) {
   PrefillPlan p{};
   const size_t routes = (size_t)tokens * top_k;
-  p.max_tiles = (int)((routes + 127) / 128) + experts;
-  p.s_max_tiles = (int)((tokens + 127) / 128);
+  p.max_tiles = (int)((routes + kTileCapMin - 1) / kTileCapMin) + experts;
+  p.s_max_tiles = (int)((tokens + kTileCapMin - 1) / kTileCapMin);
   size_t cur = 0;
   auto take = [&](size_t bytes) { const size_t at = cur; cur = align256(cur + bytes); return at; };
   p.status = take(256);
@@ -328,24 +328,30 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   sa.sorted_weight = reinterpret_cast<float*>(at(pl.sorted_weight));
   sa.num_tiles = reinterpret_cast<int*>(at(pl.num_tiles));
   sa.tile_expert = tiles; sa.tile_row0 = tiles + pl.max_tiles; sa.tile_rows = tiles + 2 * pl.max_tiles;
-  sa.max_tiles = pl.max_tiles; sa.status = status;
+  sa.max_tiles = pl.max_tiles; sa.tile_cap = grouped_gemm_tile_cap(layer->encoding, routes, E, 0); sa.status = status;
   sa.scratch = reinterpret_cast<int*>(at(pl.sort_scratch)); sa.scratch_ints = pl.sort_ints;
-  int rc = launch_route_sort(sa, stream);
-  if (rc) return rc;
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(at(pl.xs));
   GroupedGemmArgs g{};
   g.mode = 0; g.enc = layer->encoding; g.num_experts = E; g.n_rows = I; g.k = H;
   g.total_rows = routes;
   g.w0 = layer->gate; g.s0 = layer->gate_scales; g.w1 = layer->up; g.s1 = layer->up_scales;
   g.num_tiles = sa.num_tiles; g.tile_expert = sa.tile_expert; g.tile_row0 = sa.tile_row0; g.tile_rows = sa.tile_rows;
-  g.max_tiles = pl.max_tiles;
+  g.max_tiles = pl.max_tiles; g.tile_cap = sa.tile_cap;
   g.out = reinterpret_cast<__nv_bfloat16*>(at(pl.inter)); g.out_stride = I; g.permute_out = quant; g.status = status;
-  if (grouped_gemm_can_gather(g)) {
+  const bool by_index = grouped_gemm_can_gather(g);
+  if (by_index && quant && !rows_k_permuted && H % 8 == 0 && !(reinterpret_cast<uintptr_t>(hidden_bf16) & 15)) {
+    sa.permute_src = static_cast<const __nv_bfloat16*>(hidden_bf16);
+    sa.permute_dst = xs;
+    sa.permute_chunks = tokens * (H / 8);
+  }
+  int rc = launch_route_sort(sa, stream);
+  if (rc) return rc;
+  if (by_index) {
     // The gate/up GEMM fetches its activation rows by index: no [routes, H] copy of the activations exists.  The
     // quantised kernels want k in the order their conversion produces, so x is permuted once (tokens rows, not routes).
     const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(hidden_bf16);
     if (quant && !rows_k_permuted) {
-      rc = launch_gather_rows(src, nullptr, 1, tokens, H, 1, xs, nullptr, stream);
+      if (!sa.permute_dst) rc = launch_gather_rows(src, nullptr, 1, tokens, H, 1, xs, nullptr, stream);
       if (rc) return rc;
       src = xs;
     }
@@ -369,14 +375,15 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   if (shared) {
     int* st = reinterpret_cast<int*>(at(pl.s_tiles));
     int* snt = reinterpret_cast<int*>(at(pl.s_num_tiles));
-    rc = launch_dense_tiles((int)tokens, snt, st, st + pl.s_max_tiles, st + 2 * pl.s_max_tiles, stream);
+    const int s_cap = grouped_gemm_tile_cap(ENC_BF16, tokens, 1, 0);
+    rc = launch_dense_tiles((int)tokens, s_cap, snt, st, st + pl.s_max_tiles, st + 2 * pl.s_max_tiles, stream);
     if (rc) return rc;
     GroupedGemmArgs d{};
     d.mode = 0; d.enc = ENC_BF16; d.num_experts = 1; d.n_rows = S; d.k = H;
     d.act = hidden_bf16; d.total_rows = tokens;
     d.w0 = shared->gate; d.w1 = shared->up;
     d.num_tiles = snt; d.tile_expert = st; d.tile_row0 = st + pl.s_max_tiles; d.tile_rows = st + 2 * pl.s_max_tiles;
-    d.max_tiles = pl.s_max_tiles;
+    d.max_tiles = pl.s_max_tiles; d.tile_cap = s_cap;
     d.out = reinterpret_cast<__nv_bfloat16*>(at(pl.s_inter)); d.out_stride = S; d.status = status;
     rc = launch_grouped_gemm(d, stream);
     if (rc) return rc;

@@ -546,11 +546,36 @@ constexpr long long kPairMinRows = 16384;
 static bool takes_pair_kernel(const GroupedGemmArgs& a) {
   return a.variant == 2 || (a.variant == 0 && a.enc == ENC_BF16 && a.total_rows >= kPairMinRows);
 }
+// Few routes per expert: the transposed kernel of grouped_ts.cu, whose time follows the routes.  The line lies where the two
+// kernels cross on B200 (both GEMMs of a layer, all experts used, us, this kernel | grouped_ts.cu):
+//   OLMoE Q4   8 routes per expert 163 | 77    64: 165 | 123    96: 167 | 166   128: 198 | 201
+//   OLMoE Q8   8 routes per expert 209 | 112   64: 212 | 184    96: 215 | 234
+//   Qwen  Q8  34 routes per expert 267 | 150   51: 268 | 172    68: 268 | 236
+//   Qwen BF16  4 routes per expert 202 | 171   51: 207 | 186    68: 208 | 209
+//   one dense BF16 expert (the shared one), 128 tokens: 39 | 31   192: 48 | 33   256: 52 | 48   512: 55 | 72
+constexpr int kTsMaxRoutesQ4 = 88, kTsMaxRoutesQ8 = 76, kTsMaxRoutesBf16 = 64, kTsMaxRowsDense = 192;
+static bool takes_ts_kernel(int enc, long long rows, int experts, int variant) {
+  if (variant == 2) return false;
+  if (enc == ENC_BF16) return rows <= (experts == 1 ? kTsMaxRowsDense : (long long)experts * kTsMaxRoutesBf16);
+  return rows <= (long long)experts * (enc == ENC_Q8 ? kTsMaxRoutesQ8 : kTsMaxRoutesQ4);
+}
+int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant) {
+  return takes_ts_kernel(enc, rows, num_experts, variant) ? kTileCapMin : kTileCapMax;
+}
 bool grouped_gemm_can_gather(const GroupedGemmArgs& a) { return a.mode == 0 && !takes_pair_kernel(a); }
 int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
   if (takes_pair_kernel(a)) {
     if (a.gather_route) { set_error("grouped: the CTA-pair kernel takes gathered activation rows"); return ERR_BAD_ARGUMENT; }
     return launch_grouped_gemm_pair(a, stream);
+  }
+  if (takes_ts_kernel(a.enc, a.total_rows, a.num_experts, a.variant)) {
+    if (a.k % 128 || a.n_rows % (a.mode == 0 ? BN / 2 : BN) || a.total_rows <= 0 || a.max_tiles <= 0 ||
+        (a.enc != ENC_BF16 && a.k > kMaxGroups * 128)) {
+      set_error("grouped: unsupported shape (k %d, rows per expert %d)", a.k, a.n_rows);
+      return ERR_BAD_ARGUMENT;
+    }
+    if (a.gather_route && (a.mode != 0 || a.gather_top_k < 1)) { set_error("grouped: rows are fetched by index only for the gate/up GEMM"); return ERR_BAD_ARGUMENT; }
+    return launch_grouped_gemm_ts(a, stream);
   }
   return launch_grouped_gemm_single(a, stream);
 }

@@ -20,6 +20,7 @@ struct GroupedParams {
   const int* tile_row0;       // first sorted route row of the tile
   const int* tile_rows;       // valid rows (<= 128)
   int max_tiles;
+  int subs;                   // grouped_ts.cu: parts a table entry may be cut into
   __nv_bfloat16* out;         // mode 0: intermediate [routes, n_rows]; mode 1: weighted outputs [routes, n_rows]
   long long out_stride;       // elements
   const float* route_weight;  // mode 1: routing weight per sorted route
@@ -46,6 +47,7 @@ struct GroupedGemmArgs {
   const void* w1; const float* s1;   // up
   const int* num_tiles; const int* tile_expert; const int* tile_row0; const int* tile_rows;
   int max_tiles;
+  int tile_cap;               // most routes of a table entry
   __nv_bfloat16* out; long long out_stride;
   const float* route_weight;
   int permute_out;
@@ -63,6 +65,11 @@ bool grouped_gemm_can_gather(const GroupedGemmArgs& a);
 int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream);        // picks the variant
 int launch_grouped_gemm_single(const GroupedGemmArgs& a, cudaStream_t stream);
 int launch_grouped_gemm_pair(const GroupedGemmArgs& a, cudaStream_t stream);
+int launch_grouped_gemm_ts(const GroupedGemmArgs& a, cudaStream_t stream);
+
+// Routes per tile that suit the kernel launch_grouped_gemm picks for a layer: the cap to build the tile table with.
+int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant);
+constexpr int kTileCapMin = 64, kTileCapMax = 256;
 
 // ---- routing (route.cu) ---------------------------------------------------------------------------
 struct RouterArgs {
@@ -86,13 +93,16 @@ struct SortArgs {
   float* sorted_weight;            // [routes]
   int* num_tiles; int* tile_expert; int* tile_row0; int* tile_rows;   // 128-route tiles
   int max_tiles;
+  int tile_cap;                    // routes per tile
   unsigned* status;
+  // optional: rows of x in the k order of the quantised GEMMs, written by further CTAs of the first launch
+  const __nv_bfloat16* permute_src; __nv_bfloat16* permute_dst; long long permute_chunks;   // 16-byte chunks
   int* scratch;                    // optional: ceil(routes / 2048) * experts ints let the sort use many CTAs
   long long scratch_ints;
 };
 int launch_route_sort(const SortArgs& a, cudaStream_t stream);
 
-int launch_dense_tiles(int rows, int* num_tiles, int* tile_expert, int* tile_row0, int* tile_rows, cudaStream_t stream);
+int launch_dense_tiles(int rows, int tile_cap, int* num_tiles, int* tile_expert, int* tile_row0, int* tile_rows, cudaStream_t stream);
 
 // rows of x gathered into sorted order; `permute` writes each run of 8 as [0,4,1,5,2,6,3,7]
 // valid_rows (device, may be null): only the first *valid_rows sorted routes exist

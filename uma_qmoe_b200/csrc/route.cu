@@ -531,30 +531,40 @@ __global__ void __launch_bounds__(256) router_mma_kernel(const RouterArgs a) {
 // a scan over (expert, warp) give every warp its first position inside each expert's run, and ranks
 // inside a 32-route batch come from __match_any_sync, so equal experts keep their route order.
 constexpr int kSortThreads = 1024;
-constexpr int kTileRows = 256;       // routes per grouped-GEMM tile (two M = 128 accumulators)
 constexpr int kMaxSortExperts = 128;
 
 __device__ __forceinline__ int load_expert(const void* idx, int idx64, long long i) {
   return idx64 ? (int)reinterpret_cast<const long long*>(idx)[i] : reinterpret_cast<const int*>(idx)[i];
 }
 
-// Offsets and the tile list from the per-expert counts in count[] (shared memory).  Thread 0 scans the counts
-// in shared memory only; the global stores (offsets, a few tiles per expert) are then spread over the threads.
+// Offsets and the tile list from the per-expert counts in count[] (shared memory).  Warp 0 scans the counts; the global
+// stores (offsets, a few tiles per expert) are then spread over the threads.
 // start[e] receives the first sorted position of expert e.  All threads of the CTA call it.
 __device__ __forceinline__ void emit_offsets_and_tiles(const SortArgs& a, const int* count, int* start, int* tile_base,
                                                        bool write, int tid, int nthreads) {
   const int E = a.experts;
-  if (tid == 0) {
-    int run = 0, tiles = 0;
-    for (int e = 0; e < E; ++e) {
-      const int c = count[e];
-      start[e] = run;
-      tile_base[e] = tiles;
-      run += c;
-      tiles += (c + kTileRows - 1) / kTileRows;
+  if (tid < 32) {                                // four experts per lane, scanned across the warp
+    static_assert(kMaxSortExperts == 128, "four experts per lane");
+    int run[5], tiles[5];
+    run[0] = tiles[0] = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int e = 4 * tid + i, c = e < E ? count[e] : 0;
+      run[i + 1] = run[i] + c;
+      tiles[i + 1] = tiles[i] + (c + a.tile_cap - 1) / a.tile_cap;
     }
-    start[E] = run;
-    tile_base[E] = tiles;
+    int run_in = run[4], tiles_in = tiles[4];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int r = __shfl_up_sync(0xffffffffu, run_in, o), t = __shfl_up_sync(0xffffffffu, tiles_in, o);
+      if (tid >= o) { run_in += r; tiles_in += t; }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int e = 4 * tid + i;
+      if (e < E) { start[e] = run_in - run[4] + run[i]; tile_base[e] = tiles_in - tiles[4] + tiles[i]; }
+    }
+    if (tid == 31) { start[E] = run_in; tile_base[E] = tiles_in; }
   }
   __syncthreads();
   if (write) {
@@ -562,15 +572,25 @@ __device__ __forceinline__ void emit_offsets_and_tiles(const SortArgs& a, const 
     for (int e = tid; e < E; e += nthreads) {
       const int c = start[e + 1] - start[e];
       int t = tile_base[e];
-      for (int r = 0; r < c && t < a.max_tiles; r += kTileRows, ++t) {
-        a.tile_expert[t] = e; a.tile_row0[t] = start[e] + r; a.tile_rows[t] = min(kTileRows, c - r);
+      for (int r = 0; r < c && t < a.max_tiles; r += a.tile_cap, ++t) {
+        a.tile_expert[t] = e; a.tile_row0[t] = start[e] + r; a.tile_rows[t] = min(a.tile_cap, c - r);
       }
     }
     if (tid == 0) *a.num_tiles = min(tile_base[E], a.max_tiles);
   }
 }
 
+// Rows of x in the k order of the quantised GEMMs ([k0,k4,k1,k5,k2,k6,k3,k7] in every run of 8), 16 bytes per thread: the
+// sort needs one CTA (or a few), the rest of the device does this beside it instead of in a launch of its own.
+__device__ __forceinline__ void permute_chunk(const SortArgs& a, long long i) {
+  if (i >= a.permute_chunks) return;
+  const uint4 w = reinterpret_cast<const uint4*>(a.permute_src)[i];
+  reinterpret_cast<uint4*>(a.permute_dst)[i] =
+      make_uint4(prmt(w.x, w.z, 0x5410), prmt(w.x, w.z, 0x7632), prmt(w.y, w.w, 0x5410), prmt(w.y, w.w, 0x7632));
+}
+
 __global__ void __launch_bounds__(kSortThreads) route_sort_kernel(const SortArgs a) {
+  if (blockIdx.x > 0) return permute_chunk(a, (long long)(blockIdx.x - 1) * kSortThreads + threadIdx.x);
   __shared__ int hist[32][kMaxSortExperts];     // per-warp counts, then per-warp running positions
   __shared__ int total[kMaxSortExperts + 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -629,7 +649,8 @@ __global__ void __launch_bounds__(kSortThreads) route_sort_kernel(const SortArgs
 // the tile list.
 constexpr int kChunk = 2048;
 
-__global__ void __launch_bounds__(kSortThreads) route_hist_kernel(const SortArgs a, int* __restrict__ chunk_hist) {
+__global__ void __launch_bounds__(kSortThreads) route_hist_kernel(const SortArgs a, int* __restrict__ chunk_hist, int chunks) {
+  if ((int)blockIdx.x >= chunks) return permute_chunk(a, (long long)(blockIdx.x - chunks) * kSortThreads + threadIdx.x);
   __shared__ int hist[kMaxSortExperts];
   const int tid = threadIdx.x, E = a.experts;
   const long long routes = (long long)a.tokens * a.top_k;
@@ -941,10 +962,10 @@ combine_warp_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __re
 }
 
 // tile table of a dense [rows, k] matrix treated as one expert (the Qwen shared expert in prefill)
-__global__ void dense_tiles_kernel(int rows, int* num_tiles, int* tile_expert, int* tile_row0, int* tile_rows) {
-  const int tiles = (rows + 255) / 256;
+__global__ void dense_tiles_kernel(int rows, int cap, int* num_tiles, int* tile_expert, int* tile_row0, int* tile_rows) {
+  const int tiles = (rows + cap - 1) / cap;
   for (int t = threadIdx.x; t < tiles; t += blockDim.x) {
-    tile_expert[t] = 0; tile_row0[t] = t * 256; tile_rows[t] = min(256, rows - t * 256);
+    tile_expert[t] = 0; tile_row0[t] = t * cap; tile_rows[t] = min(cap, rows - t * cap);
   }
   if (threadIdx.x == 0) *num_tiles = tiles;
 }
@@ -957,8 +978,8 @@ int check_launch(const char* what) {
 
 }  // namespace
 
-int launch_dense_tiles(int rows, int* num_tiles, int* tile_expert, int* tile_row0, int* tile_rows, cudaStream_t stream) {
-  dense_tiles_kernel<<<1, 256, 0, stream>>>(rows, num_tiles, tile_expert, tile_row0, tile_rows);
+int launch_dense_tiles(int rows, int tile_cap, int* num_tiles, int* tile_expert, int* tile_row0, int* tile_rows, cudaStream_t stream) {
+  dense_tiles_kernel<<<1, 256, 0, stream>>>(rows, tile_cap, num_tiles, tile_expert, tile_row0, tile_rows);
   return check_launch("dense tiles");
 }
 
@@ -1015,11 +1036,12 @@ int launch_route_sort(const SortArgs& a, cudaStream_t stream) {
   }
   const long long routes = (long long)a.tokens * a.top_k;
   const int chunks = (int)((routes + kChunk - 1) / kChunk);
+  const unsigned permute_blocks = a.permute_dst ? (unsigned)((a.permute_chunks + kSortThreads - 1) / kSortThreads) : 0;
   if (chunks <= 2 || !a.scratch || a.scratch_ints < (long long)chunks * a.experts) {
-    route_sort_kernel<<<1, kSortThreads, 0, stream>>>(a);
+    route_sort_kernel<<<1 + permute_blocks, kSortThreads, 0, stream>>>(a);
     return check_launch("route sort");
   }
-  route_hist_kernel<<<chunks, kSortThreads, 0, stream>>>(a, a.scratch);
+  route_hist_kernel<<<chunks + permute_blocks, kSortThreads, 0, stream>>>(a, a.scratch, chunks);
   route_place_kernel<<<chunks, kSortThreads, 0, stream>>>(a, a.scratch, chunks);
   return check_launch("route sort");
 }
