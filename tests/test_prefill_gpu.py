@@ -407,3 +407,24 @@ def test_few_routes_kernel_takes_tables_of_wider_tiles():
     assert torch.equal(inter, ops.grouped_gemm(layer, 0, xs, routes, permute_out=True))
     y = ops.grouped_gemm(layer, 1, inter, routes, routes.sorted_weight)
     assert torch.equal(ops.combine_routes(y, idx, routes.route_pos).cpu(), _run_prefill(layer, x, idx, w))
+
+
+@pytest.mark.parametrize("tokens", [1, 5, 63, 192, 193, 600, 1030])
+def test_shared_expert_in_parts_of_its_contraction(tokens):
+    """The shared expert's down GEMM cut along k: eight parts, an uneven last part (600 tokens: 88 steps in six), the
+    transposed kernel and the wide one.  The routes weigh nothing, so the result is the shared expert's; rounding as above
+    and once more for the gate."""
+    from uma_qmoe_b200.stack import random_layer, random_shared_expert
+    dev = torch.device(DEV)
+    layer, sh = random_layer(syn.QWEN, "q4_group128", 6, dev), random_shared_expert(syn.QWEN, 6, dev)
+    gen = torch.Generator(device=DEV).manual_seed(tokens)
+    x = torch.randn(tokens, 2048, device=DEV, generator=gen).to(torch.bfloat16)
+    idx = torch.arange(tokens * 4, device=DEV).reshape(tokens, 4) % 60
+    got = _run_prefill(layer, x, idx, torch.zeros(tokens, 4, device=DEV), sh).float()
+    xd = x.double()
+    inter = (torch.nn.functional.silu(xd @ sh.gate.double().T) * (xd @ sh.up.double().T)).to(torch.bfloat16)
+    y = (inter.double() @ sh.down.double().T).to(torch.bfloat16)
+    gate = torch.sigmoid((xd @ sh.gate_vec.reshape(-1).double()).to(torch.bfloat16).float()).to(torch.bfloat16)
+    want = (gate[:, None] * y).cpu().float()
+    assert (got - want).norm() <= 2.0 ** -7 * want.norm()
+    assert (got - want).abs().max() <= 2.0 ** -6 * want.abs().max()

@@ -2,6 +2,7 @@
 // utilities the kernels' launchers share.
 #include "../../include/umaq_b200.h"
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -245,7 +246,7 @@ int umaq_combine_routes(const void* weighted_bf16, const void* expert_indices, i
     return ERR_BAD_ARGUMENT;
   }
   return launch_combine(static_cast<const __nv_bfloat16*>(weighted_bf16), expert_indices, indices_are_int64, route_pos,
-                        tokens, top_k, hidden, 0x7fffffff, nullptr, nullptr, nullptr, static_cast<__nv_bfloat16*>(out_bf16),
+                        tokens, top_k, hidden, 0x7fffffff, nullptr, nullptr, 0, nullptr, nullptr, static_cast<__nv_bfloat16*>(out_bf16),
                         static_cast<cudaStream_t>(stream));
 }
 
@@ -253,9 +254,14 @@ namespace {
 struct PrefillPlan {
   size_t status, counts, offsets, num_tiles, tiles, sort_scratch, sorted_route, route_pos, sorted_weight, xs, inter, yw;
   long long sort_ints;
-  size_t s_num_tiles, s_tiles, s_inter, s_out, total;
+  size_t s_num_tiles, s_tiles, s_inter, s_out, s_part, total;
   int max_tiles, s_max_tiles;
 };
+// Room for the float32 parts of the shared expert's down GEMM: up to eight of them while the tokens are few (a tile of the
+// wide kernel is 256 x 256, so at most one part per SM has been cut from 2368 tokens on).
+size_t s_part_bytes(long long tokens, int hidden) {
+  return (size_t)std::min<long long>(tokens * kMaxDenseSplits, 8192) * hidden * 4;
+}
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 PrefillPlan prefill_plan(long long tokens, int top_k, int experts, int hidden, int inter, int shared_inter) {
   PrefillPlan p{};
@@ -282,6 +288,8 @@ PrefillPlan prefill_plan(long long tokens, int top_k, int experts, int hidden, i
     p.s_tiles = take((size_t)p.s_max_tiles * 12);
     p.s_inter = take((size_t)tokens * shared_inter * 2);
     p.s_out = take((size_t)tokens * hidden * 2);
+    // at most one part of 128 rows x 64 tokens for each of two CTAs of an SM: see grouped_gemm_dense_splits
+    p.s_part = take(s_part_bytes(tokens, hidden));
   }
   p.total = cur;
   return p;
@@ -372,6 +380,8 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   if (rc) return rc;
 
   const __nv_bfloat16* shared_out = nullptr;
+  const float* shared_part = nullptr;
+  int shared_parts = 0;
   if (shared) {
     int* st = reinterpret_cast<int*>(at(pl.s_tiles));
     int* snt = reinterpret_cast<int*>(at(pl.s_num_tiles));
@@ -389,12 +399,16 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
     if (rc) return rc;
     d.mode = 1; d.n_rows = H; d.k = S; d.act = d.out; d.w0 = shared->down; d.w1 = nullptr;
     d.out = reinterpret_cast<__nv_bfloat16*>(at(pl.s_out)); d.out_stride = H; d.route_weight = nullptr;
+    d.k_splits = grouped_gemm_dense_splits(tokens, H, S);
+    d.part = reinterpret_cast<float*>(at(pl.s_part));
+    if ((size_t)d.k_splits * tokens * H * 4 > s_part_bytes(tokens, H)) d.k_splits = 1;
     rc = launch_grouped_gemm(d, stream);
     if (rc) return rc;
-    shared_out = d.out;
+    if (d.k_splits > 1) { shared_part = d.part; shared_parts = d.k_splits; }
+    else shared_out = d.out;
   }
   return launch_combine(reinterpret_cast<const __nv_bfloat16*>(at(pl.yw)), expert_indices, indices_are_int64, sa.route_pos,
-                        (int)tokens, top_k, H, E, shared_out, static_cast<const __nv_bfloat16*>(hidden_bf16),
+                        (int)tokens, top_k, H, E, shared_out, shared_part, shared_parts, static_cast<const __nv_bfloat16*>(hidden_bf16),
                         shared ? static_cast<const __nv_bfloat16*>(shared->gate_vec) : nullptr,
                         static_cast<__nv_bfloat16*>(out_bf16), stream, segments);
 }

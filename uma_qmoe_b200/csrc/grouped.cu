@@ -27,6 +27,8 @@
 
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "tc.cuh"
 
@@ -67,7 +69,7 @@ struct GemmShared {
 };
 
 struct TileInfo {
-  int tile_n, expert, row0, nrows;
+  int tile_n, expert, row0, nrows, k0, k1;   // k0, k1: first and end step of the contraction
 };
 
 // Persistent: one CTA per SM walks the (row tile, column tile) list, column tile fastest, so that the
@@ -102,7 +104,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const int nk = K / BK;
   const int groups = K >> 7;
   const int n_col = p.n_rows / (MODE == 0 ? BN / 2 : BN);
-  const int total = *p.num_tiles * n_col;
+  constexpr bool kSplit = ENC == ENC_BF16 && MODE == 1;      // may run on parts of the contraction
+  const int splits = kSplit ? p.k_splits : 1;
+  const int total = *p.num_tiles * n_col * splits;
   const int first = blockIdx.x, step = gridDim.x;
   volatile int* abort_flag = &sh.abort_flag;
   // Gather mode (gate/up GEMM only): the activation tile of a stage is written by kGatherThreads threads with
@@ -132,6 +136,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
   auto tile_of = [&](int it) {
     TileInfo t;
+    t.k0 = 0; t.k1 = nk;
+    if (kSplit && splits > 1) {
+      const int part = it % splits, each = (nk + splits - 1) / splits;
+      it /= splits;
+      t.k0 = min(nk, part * each); t.k1 = min(nk, t.k0 + each);
+    }
     const int tile_m = it / n_col;
     t.tile_n = it - tile_m * n_col;
     t.expert = p.tile_expert[tile_m]; t.row0 = p.tile_row0[tile_m]; t.nrows = p.tile_rows[tile_m];
@@ -154,7 +164,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const bool two = t.nrows > BM;
         const long long wrow0 = weight_row(t);
         bool ok = true;
-        for (int kc = 0; kc < nk; ++kc, ++kidx) {
+        for (int kc = t.k0; kc < t.k1; ++kc, ++kidx) {
           const uint32_t s = kidx % kInStages, use = kidx / kInStages;
           if (use > 0 && !mbar_wait(&sh.in_empty[s], (use - 1) & 1)) { ok = false; break; }
           const uint32_t bytes = (gather ? 0 : (two ? kATile : kAHalf)) + (ENC == ENC_BF16 ? kBTile : 0);
@@ -278,11 +288,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       uint32_t kidx = 0;
       int seq = 0;
       for (int it = first; it < total && !*abort_flag; it += step, ++seq) {
-        const bool two = p.tile_rows[it / n_col] > BM;
+        const TileInfo t = tile_of(it);
+        const bool two = t.nrows > BM;
         if (seq >= 1 && !mbar_wait(&sh.acc_empty, (seq - 1) & 1)) { fail(); break; }
         tc_fence_after();
         bool ok = true;
-        for (int kc = 0; kc < nk; ++kc, ++kidx) {
+        for (int kc = t.k0; kc < t.k1; ++kc, ++kidx) {
           const uint32_t s = kidx % kInStages;
           const uint32_t sb = ENC == ENC_BF16 ? s : kidx % kBStages;
           ok = mbar_wait(&sh.in_full[s], (kidx / kInStages) & 1);
@@ -293,8 +304,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
             const uint64_t bdesc = smem_desc_sw128(b_addr + k * 32);
-            tc_mma_bf16(tmem, smem_desc_sw128(a_addr + k * 32), bdesc, kInstrDesc, (kc | k) ? 1u : 0u);
-            if (two) tc_mma_bf16(tmem + BN, smem_desc_sw128(a_addr + kAHalf + k * 32), bdesc, kInstrDesc, (kc | k) ? 1u : 0u);
+            const uint32_t accumulate = kc != t.k0 || k ? 1u : 0u;
+            tc_mma_bf16(tmem, smem_desc_sw128(a_addr + k * 32), bdesc, kInstrDesc, accumulate);
+            if (two) tc_mma_bf16(tmem + BN, smem_desc_sw128(a_addr + kAHalf + k * 32), bdesc, kInstrDesc, accumulate);
           }
           tc_commit(&sh.in_empty[s]);                 // A tile (and a BF16 B tile) may be overwritten
           if (ENC != ENC_BF16) tc_commit(&sh.b_empty[sb]);
@@ -427,7 +439,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (c + 1 < nchunks) tmem_ld32(tq + ((c + 1) >> 2) * BN + ch * 128 + ((c + 1) & 3) * 32, acc[(c + 1) & 1]);
             else release();
             const int row = (c >> 2) * BM + quarter * 32 + lane;
-            if ((kStaged || row < t.nrows) && !(p.debug & 2)) {
+            if (kSplit && splits > 1) {
+              if (row < t.nrows) {                           // float32 sums of this part: a lane writes 128 contiguous bytes
+                const uint32_t (&a)[32] = acc[c & 1];
+                uint4* dst = reinterpret_cast<uint4*>(p.part + (it % splits) * p.part_stride + ((long long)t.row0 + row) * p.n_rows +
+                                                      f0 + ch * 128 + (c & 3) * 32);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) dst[i] = make_uint4(a[4 * i], a[4 * i + 1], a[4 * i + 2], a[4 * i + 3]);
+              }
+            } else if ((kStaged || row < t.nrows) && !(p.debug & 2)) {
               const long long grow = (long long)t.row0 + row;
               const float wr = row < t.nrows && p.route_weight ? p.route_weight[grow] : 1.f;
               const uint32_t (&a)[32] = acc[c & 1];
@@ -559,6 +579,17 @@ static bool takes_ts_kernel(int enc, long long rows, int experts, int variant) {
   if (enc == ENC_BF16) return rows <= (experts == 1 ? kTsMaxRowsDense : (long long)experts * kTsMaxRoutesBf16);
   return rows <= (long long)experts * (enc == ENC_Q8 ? kTsMaxRoutesQ8 : kTsMaxRoutesQ4);
 }
+// The shared expert's down GEMM has few tiles and a long contraction (Qwen: 2048 rows, k 5632): without parts it runs on 16
+// CTAs at up to 64 tokens and on 48 at 1531.  Parts until the CTAs that fit the device have a tile each.
+// Down GEMM plus the combine that adds the parts, Qwen shape, us, before | now: 24 tokens 52 | 15, 128: 54 | 17, 1531: 76 | 62.
+int grouped_gemm_dense_splits(long long rows, int n_rows, int k) {
+  const bool ts = takes_ts_kernel(ENC_BF16, rows, 1, 0);
+  if (!ts && rows >= kPairMinRows) return 1;
+  const long long tiles = ts ? (rows + kTileCapMin - 1) / kTileCapMin * (n_rows / 128) : (rows + kTileCapMax - 1) / kTileCapMax * (n_rows / BN);
+  const long long slots = (long long)sm_count() * (ts ? 2 : 1);
+  const long long want = tiles > 0 ? slots / tiles : 1;
+  return (int)std::max(1ll, std::min({want, (long long)kMaxDenseSplits, (long long)(k / 512)}));
+}
 int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant) {
   return takes_ts_kernel(enc, rows, num_experts, variant) ? kTileCapMin : kTileCapMax;
 }
@@ -620,6 +651,7 @@ int launch_grouped_gemm_single(const GroupedGemmArgs& a, cudaStream_t stream) {
   p.scales0 = a.s0; p.scales1 = a.s1;
   p.num_tiles = a.num_tiles; p.tile_expert = a.tile_expert; p.tile_row0 = a.tile_row0; p.tile_rows = a.tile_rows;
   p.max_tiles = a.max_tiles;
+  p.k_splits = a.k_splits > 1 ? a.k_splits : 1; p.part = a.part; p.part_stride = a.total_rows * a.n_rows;
   p.out = a.out; p.out_stride = a.out_stride; p.route_weight = a.route_weight; p.permute_out = a.permute_out;
   { static const int dbg = [] { const char* v = std::getenv("UMAQ_GEMM_DEBUG"); return v ? std::atoi(v) : 0; }(); p.debug = dbg; }
   p.tma_out = tma_out;

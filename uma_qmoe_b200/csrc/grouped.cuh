@@ -21,6 +21,9 @@ struct GroupedParams {
   const int* tile_rows;       // valid rows (<= 128)
   int max_tiles;
   int subs;                   // grouped_ts.cu: parts a table entry may be cut into
+  int k_splits;               // BF16 down GEMM: the contraction is cut into this many parts, each a tile of its own
+  float* part;                // k_splits > 1: float32 sums [k_splits, total rows, n_rows] instead of `out`
+  long long part_stride;      // elements of one split
   __nv_bfloat16* out;         // mode 0: intermediate [routes, n_rows]; mode 1: weighted outputs [routes, n_rows]
   long long out_stride;       // elements
   const float* route_weight;  // mode 1: routing weight per sorted route
@@ -48,6 +51,8 @@ struct GroupedGemmArgs {
   const int* num_tiles; const int* tile_expert; const int* tile_row0; const int* tile_rows;
   int max_tiles;
   int tile_cap;               // most routes of a table entry
+  int k_splits;               // > 1 (BF16 down GEMM without routing weights): partial sums into `part`, `out` is not written
+  float* part;                // [k_splits, total_rows, n_rows] float32
   __nv_bfloat16* out; long long out_stride;
   const float* route_weight;
   int permute_out;
@@ -69,6 +74,9 @@ int launch_grouped_gemm_ts(const GroupedGemmArgs& a, cudaStream_t stream);
 
 // Routes per tile that suit the kernel launch_grouped_gemm picks for a layer: the cap to build the tile table with.
 int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant);
+// Parts the contraction of a dense BF16 down GEMM (the shared expert's) is cut into
+int grouped_gemm_dense_splits(long long rows, int n_rows, int k);
+constexpr int kMaxDenseSplits = 8;
 constexpr int kTileCapMin = 64, kTileCapMax = 256;
 
 // ---- routing (route.cu) ---------------------------------------------------------------------------
@@ -130,10 +138,11 @@ struct SegmentedOut {
   int row0;
   int skip_empty;
 };
-// experts: ids outside [0, experts) are treated as absent routes
+// experts: ids outside [0, experts) are treated as absent routes.  The shared expert's rows come as BF16 (shared_out) or
+// as shared_parts float32 partial sums [shared_parts, tokens, hidden] that are added here and rounded once.
 int launch_combine(const __nv_bfloat16* weighted, const void* indices, int idx64, const int* route_pos, int tokens,
-                   int top_k, int hidden, int experts, const __nv_bfloat16* shared_out, const __nv_bfloat16* x,
-                   const __nv_bfloat16* gate_vec, __nv_bfloat16* out, cudaStream_t stream,
+                   int top_k, int hidden, int experts, const __nv_bfloat16* shared_out, const float* shared_part,
+                   int shared_parts, const __nv_bfloat16* x, const __nv_bfloat16* gate_vec, __nv_bfloat16* out, cudaStream_t stream,
                    const SegmentedOut* segments = nullptr);
 
 }  // namespace umaq

@@ -120,11 +120,20 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 
 struct TsTile {
   int col, expert, row0, nrows;
+  int part, k0, k1;                         // part of the contraction, its first and end step
 };
 
 // tile table entry -> one of its `subs` parts of at most NMAX routes (equal parts, multiples of 16); nrows 0: no such part
-__device__ __forceinline__ TsTile ts_tile(const GroupedParams& p, int it, int n_col) {
+template <bool SPLIT>
+__device__ __forceinline__ TsTile ts_tile(const GroupedParams& p, int it, int n_col, int nk) {
   TsTile t;
+  t.part = 0; t.k0 = 0; t.k1 = nk;
+  if (SPLIT && p.k_splits > 1) {
+    const int each = (nk + p.k_splits - 1) / p.k_splits;
+    t.part = it % p.k_splits;
+    it /= p.k_splits;
+    t.k0 = min(nk, t.part * each); t.k1 = min(nk, t.k0 + each);
+  }
   const int m = it / n_col;
   t.col = it - m * n_col;
   const int tm = p.subs == 1 ? m : m / p.subs, sub = m - tm * p.subs;
@@ -157,7 +166,8 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
   const int nk = K / S::kStepK;
   const int groups = K >> 7;
   const int n_col = p.n_rows / kFeatures;
-  const int total = *p.num_tiles * p.subs * n_col;
+  constexpr bool kSplit = !kQuant && MODE == 1;
+  const int total = *p.num_tiles * p.subs * n_col * (kSplit ? p.k_splits : 1);
   const int first = blockIdx.x, step = gridDim.x;
   volatile int* abort_flag = &sh.abort_flag;
   const bool gather = MODE == 0 && p.gather_route != nullptr;
@@ -190,7 +200,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     uint32_t seq = 0;
     for (int it = first; it < total; it += step) {
       if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
-      const TsTile t = ts_tile(p, it, n_col);
+      const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
       if (t.nrows == 0) continue;
       const uint32_t buf = seq % kAccBufs, use = seq / kAccBufs;
       ++seq;
@@ -199,7 +209,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
       // kind::f16, BF16 x BF16 -> FP32, K-major operands, M = 128, N = the tile's routes
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n16 >> 3) << 17) | (8u << 24);
       const uint32_t acc = tmem + buf * NMAX;
-      for (int kc = 0; kc < nk; ++kc) {
+      for (int kc = t.k0; kc < t.k1; ++kc) {
         ok = ok && mbar_wait(&sh.in_full[rb.slot], rb.phase);
         ok = ok && (kQuant ? mbar_wait(&sh.a_full[ra.slot], ra.phase) : mbar_wait(&sh.p_full[rp.slot], rp.phase));
         if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
@@ -211,13 +221,13 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
 #pragma unroll
           for (int k = 0; k < S::kStepK / 16; ++k) {
             const uint64_t bdesc = bd + (k >> 2) * (S::kBAtom >> 4) + (k & 3) * 2;
-            const uint32_t accumulate = k ? 1u : (uint32_t)(kc != 0);
+            const uint32_t accumulate = k ? 1u : (uint32_t)(kc != t.k0);
             if (kQuant) tc_mma_bf16_ts(acc, a_tmem + k * 8, bdesc, idesc, accumulate);
             else tc_mma_bf16(acc, wd + k * 2, bdesc, idesc, accumulate);
           }
           tc_commit(&sh.in_empty[rb.slot]);
           tc_commit(kQuant ? &sh.a_empty[ra.slot] : &sh.p_empty[rp.slot]);
-          if (kc == nk - 1) tc_commit(&sh.acc_full[buf]);
+          if (kc == t.k1 - 1) tc_commit(&sh.acc_full[buf]);
         }
         __syncwarp();
         rb.next();
@@ -231,7 +241,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
       uint32_t kidx = 0, seq = 0;
       Ring<kPStages> rp;
       for (int it = first; it < total && !*abort_flag; it += step) {
-        const TsTile t = ts_tile(p, it, n_col);
+        const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
         if (t.nrows == 0) continue;
         const long long wrow0 = (long long)t.expert * p.n_rows + t.col * kFeatures;
         if (kQuant) {
@@ -245,7 +255,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
         }
         ++seq;
         bool ok = true;
-        for (int kc = 0; kc < nk; ++kc, ++kidx, rp.next()) {
+        for (int kc = t.k0; kc < t.k1; ++kc, ++kidx, rp.next()) {
           const uint32_t s = rp.slot;
           if (kidx >= (uint32_t)kPStages && !mbar_wait(&sh.p_empty[s], rp.phase ^ 1)) { ok = false; break; }
           mbar_expect_tx(&sh.p_full[s], S::kWeightBytes);
@@ -280,11 +290,11 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
         uint32_t kidx = 0;
         Ring<kBStages> rb;
         for (int it = first; it < total && !*abort_flag; it += step) {
-          const TsTile t = ts_tile(p, it, n_col);
+          const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
           if (t.nrows == 0) continue;
           const int boxes = (t.nrows + kActBox - 1) / kActBox;
           bool ok = true;
-          for (int kc = 0; kc < nk; ++kc, ++kidx, rb.next()) {
+          for (int kc = t.k0; kc < t.k1; ++kc, ++kidx, rb.next()) {
             const uint32_t s = rb.slot;
             if (kidx >= (uint32_t)kBStages && !mbar_wait(&sh.in_empty[s], rb.phase ^ 1)) { ok = false; break; }
             mbar_expect_tx(&sh.in_full[s], S::kAtoms * boxes * kActBox * 128);
@@ -320,7 +330,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
       for (int it = first; it < total; it += step) {
         // everybody has read the previous tile's table, and the threads agree whether to go on
         if (named_bar_or(1, kTsGatherThreads, !ok || *abort_flag != 0)) break;
-        const TsTile t = ts_tile(p, it, n_col);
+        const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
         const int n8 = ((t.nrows + 15) & ~15) >> 3;         // runs of 8 rows
         sh.gather_token[pt] = pt < t.nrows ? p.gather_route[t.row0 + pt] / p.gather_top_k : -1;
         named_bar_sync(1, kTsGatherThreads);
@@ -360,7 +370,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     Ring<kPStages> rp;
     Ring<kAStages> ra;
     for (int it = first; it < total && !*abort_flag; it += step) {
-      const TsTile t = ts_tile(p, it, n_col);
+      const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
       if (t.nrows == 0) continue;
       const uint32_t sbuf = seq & 1;
       bool ok = mbar_wait(&sh.sc_full[sbuf], (seq >> 1) & 1);
@@ -408,7 +418,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
     uint32_t seq = 0;
     for (int it = first; it < total && !*abort_flag; it += step) {
-      const TsTile t = ts_tile(p, it, n_col);
+      const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
       if (t.nrows == 0) continue;
       const uint32_t buf = seq % kAccBufs, use = seq / kAccBufs;
       ++seq;
@@ -445,6 +455,12 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
             if (2 * j + r0 < left)
               *reinterpret_cast<uint32_t*>(dst + (long long)(2 * j) * p.out_stride) = hi ? pack_bf16(other, v[j + 1]) : pack_bf16(v[j], other);
           }
+        } else if (kSplit && p.k_splits > 1) {
+          // float32 sums of this part of the contraction
+          float* dst = p.part + t.part * p.part_stride + ((long long)t.row0 + c * 16) * p.n_rows + t.col * kFeatures + quarter * 32 + lane;
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (j < left) dst[(long long)j * p.n_rows] = __uint_as_float(a[j]);
         } else {
           const int hi = lane & 1;
           const float* wr = p.route_weight ? p.route_weight + t.row0 + c * 16 : nullptr;
@@ -521,6 +537,7 @@ int launch_grouped_gemm_ts(const GroupedGemmArgs& a, cudaStream_t stream) {
   p.scales0 = a.s0; p.scales1 = a.s1;
   p.num_tiles = a.num_tiles; p.tile_expert = a.tile_expert; p.tile_row0 = a.tile_row0; p.tile_rows = a.tile_rows;
   p.max_tiles = a.max_tiles;
+  p.k_splits = a.k_splits > 1 ? a.k_splits : 1; p.part = a.part; p.part_stride = a.total_rows * a.n_rows;
   p.out = a.out; p.out_stride = a.out_stride; p.route_weight = a.route_weight; p.permute_out = a.permute_out;
   p.status = a.status;
   p.gather_route = a.gather_route; p.gather_top_k = a.gather_top_k; p.gather_src = static_cast<const __nv_bfloat16*>(a.act);

@@ -799,11 +799,12 @@ __global__ void ep_pack_kernel(const __nv_bfloat16* __restrict__ x, const int* _
 // contributions are already BF16 (GEMM 2 epilogue).  With a shared expert: + bf16(sigmoid(bf16(x . wg))
 // * shared_out[t]), as QuantizedQwenMoEBlock does after the operator
 // (src/uma_qmoe/qwen_compressed_loader.py:82-85).
-__global__ void __launch_bounds__(256, 4)
+template <bool PARTS>                             // the shared expert's rows come as float32 partial sums
+__global__ void __launch_bounds__(256, PARTS ? 2 : 4)
 combine_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __restrict__ indices, int idx64,
                const int* __restrict__ route_pos, int top_k, int hidden, int experts,
-               const __nv_bfloat16* __restrict__ shared_out, const __nv_bfloat16* __restrict__ x,
-               const __nv_bfloat16* __restrict__ gate_vec, __nv_bfloat16* __restrict__ out, const __grid_constant__ SegmentedOut seg) {
+               const __nv_bfloat16* __restrict__ shared_out, const float* __restrict__ shared_part, int shared_parts,
+               const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate_vec, __nv_bfloat16* __restrict__ out, const __grid_constant__ SegmentedOut seg) {
   __shared__ int order_pos[8];
   __shared__ int present;
   __shared__ float red[8];
@@ -830,7 +831,8 @@ combine_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __restric
     const unsigned m = __ballot_sync(0xffu, valid);
     if (tid == 0) present = __popc(m);
   }
-  if (shared_out) {
+  const bool has_shared = PARTS || shared_out;
+  if (has_shared) {
     float acc = 0.f;
     for (int k = tid; k < hidden; k += 256)
       acc += __bfloat162float(x[(size_t)t * hidden + k]) * __bfloat162float(gate_vec[k]);
@@ -839,7 +841,7 @@ combine_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __restric
     if ((tid & 31) == 0) red[tid >> 5] = acc;
   }
   __syncthreads();
-  if (shared_out && tid == 0) {
+  if (has_shared && tid == 0) {
     float s = 0.f;
     for (int i = 0; i < 8; ++i) s += red[i];
     s = bf16_round(s);
@@ -876,14 +878,38 @@ combine_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __restric
         }
       }
     }
-    if (shared_out) {
-      const uint4 sv = *reinterpret_cast<const uint4*>(shared_out + (size_t)t * hidden + c);
-      const uint32_t w[4] = {sv.x, sv.y, sv.z, sv.w};
+    if (has_shared) {
+      float sv[8];
+      if (PARTS) {                                  // added in order and rounded where the BF16 row was
+        const float4* at = reinterpret_cast<const float4*>(shared_part + (size_t)t * hidden + c);
+        const size_t stride = (size_t)gridDim.x * hidden / 4;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        r[2 * e] = bf16_round(r[2 * e] + bf16_round(gate * __uint_as_float(w[e] << 16)));
-        r[2 * e + 1] = bf16_round(r[2 * e + 1] + bf16_round(gate * __uint_as_float(w[e] & 0xffff0000u)));
+        for (int e = 0; e < 8; ++e) sv[e] = 0.f;
+        for (int q = 0; q < shared_parts; q += 4) {  // four parts' loads in flight
+          float4 lo[4], hi[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (q + i < shared_parts) { lo[i] = at[(q + i) * stride]; hi[i] = at[(q + i) * stride + 1]; }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (q + i < shared_parts) {
+              sv[0] += lo[i].x; sv[1] += lo[i].y; sv[2] += lo[i].z; sv[3] += lo[i].w;
+              sv[4] += hi[i].x; sv[5] += hi[i].y; sv[6] += hi[i].z; sv[7] += hi[i].w;
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sv[e] = bf16_round(sv[e]);
+      } else {
+        const uint4 raw = *reinterpret_cast<const uint4*>(shared_out + (size_t)t * hidden + c);
+        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          sv[2 * e] = __uint_as_float(w[e] << 16);
+          sv[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+        }
       }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) r[e] = bf16_round(r[e] + bf16_round(gate * sv[e]));
     }
     uint4 o;
     __nv_bfloat162 p0 = __floats2bfloat162_rn(r[0], r[1]), p1 = __floats2bfloat162_rn(r[2], r[3]);
@@ -1055,13 +1081,13 @@ int launch_gather_rows(const __nv_bfloat16* x, const int* sorted_route, int top_
 }
 
 int launch_combine(const __nv_bfloat16* weighted, const void* indices, int idx64, const int* route_pos, int tokens,
-                   int top_k, int hidden, int experts, const __nv_bfloat16* shared_out, const __nv_bfloat16* x,
-                   const __nv_bfloat16* gate_vec, __nv_bfloat16* out, cudaStream_t stream,
+                   int top_k, int hidden, int experts, const __nv_bfloat16* shared_out, const float* shared_part,
+                   int shared_parts, const __nv_bfloat16* x, const __nv_bfloat16* gate_vec, __nv_bfloat16* out, cudaStream_t stream,
                    const SegmentedOut* segments) {
   if (tokens <= 0 || top_k < 1 || top_k > 8 || hidden % 8) { set_error("combine: unsupported shape"); return ERR_BAD_ARGUMENT; }
   SegmentedOut seg{};
   if (segments) seg = *segments;
-  if (!shared_out) {
+  if (!shared_out && shared_parts == 0) {
     // A warp per token leaves the device empty when the tokens are few, and its eight column passes of 2048 wide rows are
     // a chain of load latencies (11.5 us at 7 tokens): then a token's columns are spread over several warps.
     const int passes = (hidden / 8 + 31) / 32;
@@ -1070,7 +1096,8 @@ int launch_combine(const __nv_bfloat16* weighted, const void* indices, int idx64
         weighted, indices, idx64, route_pos, tokens, top_k, hidden, experts, out, seg);
     return check_launch("combine");
   }
-  combine_kernel<<<tokens, 256, 0, stream>>>(weighted, indices, idx64, route_pos, top_k, hidden, experts, shared_out, x, gate_vec, out, seg);
+  auto kernel = shared_parts > 0 ? combine_kernel<true> : combine_kernel<false>;
+  kernel<<<tokens, 256, 0, stream>>>(weighted, indices, idx64, route_pos, top_k, hidden, experts, shared_out, shared_part, shared_parts, x, gate_vec, out, seg);
   return check_launch("combine");
 }
 
