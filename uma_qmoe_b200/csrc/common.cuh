@@ -106,6 +106,13 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// ---- programmatic stream serialisation ---------------------------------------
+// A kernel launched with launch_chained may become resident while the kernel before it on the stream still runs.  Its
+// threads call pdl_wait before they read or write global memory: it returns when that kernel has finished and its writes
+// are visible (at once if the launch was an ordinary one).  Since every kernel of a chain waits, so does everything before.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- named barrier ------------------------------------------------------------
 // Barrier over `threads` threads that also returns the OR of their predicates: every participant gets the same
 // answer, so a group can agree to stop without anybody being left waiting at the next barrier.
@@ -180,6 +187,17 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
 __device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 // MUFU reciprocal: 2 ulp in float32, far below the BF16 rounding that follows every use
 __device__ __forceinline__ float silu_f32(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
+
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
 
 #endif  // __CUDACC__
 

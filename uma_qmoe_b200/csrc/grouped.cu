@@ -106,7 +106,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const int n_col = p.n_rows / (MODE == 0 ? BN / 2 : BN);
   constexpr bool kSplit = ENC == ENC_BF16 && MODE == 1;      // may run on parts of the contraction
   const int splits = kSplit ? p.k_splits : 1;
-  const int total = *p.num_tiles * n_col * splits;
   const int first = blockIdx.x, step = gridDim.x;
   volatile int* abort_flag = &sh.abort_flag;
   // Gather mode (gate/up GEMM only): the activation tile of a stage is written by kGatherThreads threads with
@@ -114,6 +113,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   // produces; the stage's barrier then counts those threads (plus the TMA warp for a BF16 weight tile).
   const bool gather = MODE == 0 && p.gather_route != nullptr;
 
+  pdl_launch_dependents();
   if (tid == 0) {
     const uint32_t in_count = gather ? kGatherThreads + (ENC == ENC_BF16 ? 1 : 0) : 1;
     for (int s = 0; s < kInStages; ++s) { mbar_init(&sh.in_full[s], in_count); mbar_init(&sh.in_empty[s], 1); }
@@ -133,6 +133,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh.tmem_base;
+  pdl_wait();                                        // everything above ran beside the kernel before
+  const int total = *p.num_tiles * n_col * splits;
 
   auto tile_of = [&](int it) {
     TileInfo t;
@@ -333,29 +335,33 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         for (int kc = 0; kc < nk && ok; ++kc, ++kidx) {
           const uint32_t s = kidx % kPStages, sb = kidx % kBStages, use = kidx / kBStages;
           ok = mbar_wait(&sh.p_full[s], (kidx / kPStages) & 1);
-          if (ok && use > 0) ok = mbar_wait(&sh.b_empty[sb], (use - 1) & 1);
           if (!ok) break;
           const float scale = sc[kc >> 1];
           const uint8_t* src = sP + s * kPackedBytes + r * kPackedRow;
-          uint8_t* dstrow = sB + sb * kBTile + r * 128;
+          // The arithmetic comes before the wait for a free stage: with two converted stages the round trip commit ->
+          // free -> stores -> full has to fit into the other stage's MMAs (1024 clocks), and the conversion would not.
+          uint32_t out[2][16];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {                 // the two 32-wide halves of the k chunk
-            uint32_t out[16];
             if (ENC == ENC_Q4) {
-              convert_q4(*reinterpret_cast<const uint4*>(src + h * 16), scale, out);
+              convert_q4(*reinterpret_cast<const uint4*>(src + h * 16), scale, out[h]);
             } else {
               convert_q8(*reinterpret_cast<const uint4*>(src + h * 32), *reinterpret_cast<const uint4*>(src + h * 32 + 16),
-                         scale, out);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int chunk = (h * 4 + i) ^ (r & 7);
-              *reinterpret_cast<uint4*>(dstrow + chunk * 16) = make_uint4(out[4 * i], out[4 * i + 1], out[4 * i + 2], out[4 * i + 3]);
+                         scale, out[h]);
             }
           }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh.p_empty[s]);
+          if (use > 0) ok = mbar_wait(&sh.b_empty[sb], (use - 1) & 1);
+          if (!ok) break;
+          uint8_t* dstrow = sB + sb * kBTile + r * 128;
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            *reinterpret_cast<uint4*>(dstrow + ((i ^ (r & 7)) << 4)) =
+                make_uint4(out[i >> 2][4 * (i & 3)], out[i >> 2][4 * (i & 3) + 1], out[i >> 2][4 * (i & 3) + 2], out[i >> 2][4 * (i & 3) + 3]);
           fence_proxy_async();                         // generic-proxy writes -> visible to the tensor core
           __syncwarp();
-          if (lane == 0) { mbar_arrive(&sh.b_full[sb]); mbar_arrive(&sh.p_empty[s]); }
+          if (lane == 0) mbar_arrive(&sh.b_full[sb]);
         }
         if (ok) {
           __syncwarp();
@@ -548,8 +554,8 @@ int launch_one(const GroupedParams& p, const CUtensorMap& ma, const CUtensorMap&
     configured = dev;
   }
   (void)n_tiles;
-  kernel<<<dim3(sm_count()), kGemmThreads + (MODE == 0 && p.gather_route ? kGatherThreads : 0), smem, stream>>>(ma, mb0, mb1, mo, p);
-  cudaError_t e = cudaGetLastError();
+  const int threads = kGemmThreads + (MODE == 0 && p.gather_route ? kGatherThreads : 0);
+  cudaError_t e = launch_chained(kernel, dim3(sm_count()), dim3(threads), smem, stream, ma, mb0, mb1, mo, p);
   if (e != cudaSuccess) { set_error("grouped: launch failed: %s", cudaGetErrorString(e)); return ERR_LAUNCH; }
   return ERR_NONE;
 }

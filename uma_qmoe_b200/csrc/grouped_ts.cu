@@ -167,11 +167,11 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
   const int groups = K >> 7;
   const int n_col = p.n_rows / kFeatures;
   constexpr bool kSplit = !kQuant && MODE == 1;
-  const int total = *p.num_tiles * p.subs * n_col * (kSplit ? p.k_splits : 1);
   const int first = blockIdx.x, step = gridDim.x;
   volatile int* abort_flag = &sh.abort_flag;
   const bool gather = MODE == 0 && p.gather_route != nullptr;
 
+  pdl_launch_dependents();
   if (tid == 0) {
     for (int s = 0; s < kBStages; ++s) { mbar_init(&sh.in_full[s], gather ? kTsGatherThreads : 1); mbar_init(&sh.in_empty[s], 1); }
     for (int s = 0; s < kPStages; ++s) { mbar_init(&sh.p_full[s], 1); mbar_init(&sh.p_empty[s], kQuant ? S::kConvertWarps : 1); }
@@ -189,6 +189,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh.tmem_base;
+  const int total = *p.num_tiles * p.subs * n_col * (kSplit ? p.k_splits : 1);
   auto fail = [&]() { atomicExch(p.status, (unsigned)ERR_DEVICE_TIMEOUT); *abort_flag = 1; };
 
   if (warp == 0) {
@@ -523,6 +524,9 @@ int launch_ts(const GroupedGemmArgs& a, GroupedParams p, cudaStream_t stream) {
                 kAtomK, kActBox, CU_TENSOR_MAP_SWIZZLE_128B))
     return ERR_LAUNCH;
   p.subs = (a.tile_cap + NMAX - 1) / NMAX;
+  // An ordinary launch, not a chained one: CTAs that become resident one by one as their predecessor's leave are paired on
+  // the SMs by chance, and CTAs with a tile more than the others then meet on one SM (OLMoE Q8, 96 tokens: 127 -> 140 us a
+  // layer).  Launched on an empty device, CTA b and b + SMs share an SM and the longer ones spread.
   kernel<<<dim3(2 * sm_count()), S::kThreads, smem, stream>>>(ma, m0, m1, p);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_error("grouped: launch failed: %s", cudaGetErrorString(e)); return ERR_LAUNCH; }

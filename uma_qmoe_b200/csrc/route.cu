@@ -320,9 +320,9 @@ router_small_kernel(const RouterArgs a) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint32_t cr;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(cr));
-  // A kernel launched behind this one with programmatic stream serialisation (the decode kernels are) may become
-  // resident now and run its prologue; it still waits for this grid to finish before it reads the routes.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // A kernel launched behind this one with programmatic stream serialisation (the decode kernels and the sort are) may
+  // become resident now and run its prologue; it still waits for this grid to finish before it reads the routes.
+  pdl_launch_dependents();
   // a CTA may write into another CTA's shared memory only once that CTA runs: arrive now, wait before the stores
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   const int token0 = (blockIdx.x / kRsCluster) * kRsTokens, nt = min(kRsTokens, a.tokens - token0);
@@ -411,6 +411,7 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t& r0, uint32_
 
 template <int MT>
 __global__ void __launch_bounds__(256) router_mma_kernel(const RouterArgs a) {
+  pdl_launch_dependents();
   extern __shared__ __align__(128) uint8_t rm_smem[];
   constexpr int kGroups = MT / 16;                         // token groups of 16
   constexpr int kPerGroup = 8 / kGroups;                   // warps sharing a token group
@@ -590,6 +591,8 @@ __device__ __forceinline__ void permute_chunk(const SortArgs& a, long long i) {
 }
 
 __global__ void __launch_bounds__(kSortThreads) route_sort_kernel(const SortArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (blockIdx.x > 0) return permute_chunk(a, (long long)(blockIdx.x - 1) * kSortThreads + threadIdx.x);
   __shared__ int hist[32][kMaxSortExperts];     // per-warp counts, then per-warp running positions
   __shared__ int total[kMaxSortExperts + 1];
@@ -650,6 +653,8 @@ __global__ void __launch_bounds__(kSortThreads) route_sort_kernel(const SortArgs
 constexpr int kChunk = 2048;
 
 __global__ void __launch_bounds__(kSortThreads) route_hist_kernel(const SortArgs a, int* __restrict__ chunk_hist, int chunks) {
+  pdl_launch_dependents();
+  pdl_wait();
   if ((int)blockIdx.x >= chunks) return permute_chunk(a, (long long)(blockIdx.x - chunks) * kSortThreads + threadIdx.x);
   __shared__ int hist[kMaxSortExperts];
   const int tid = threadIdx.x, E = a.experts;
@@ -670,6 +675,8 @@ __global__ void __launch_bounds__(kSortThreads) route_hist_kernel(const SortArgs
 
 __global__ void __launch_bounds__(kSortThreads) route_place_kernel(const SortArgs a, const int* __restrict__ chunk_hist,
                                                                    int chunks) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ int hist[32][kMaxSortExperts];     // per-warp counts of this chunk, then running positions
   __shared__ int total[kMaxSortExperts + 1];    // per-expert totals, then first position of this chunk
   __shared__ int before[kMaxSortExperts];       // routes of the expert in earlier chunks
@@ -805,6 +812,7 @@ combine_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __restric
                const int* __restrict__ route_pos, int top_k, int hidden, int experts,
                const __nv_bfloat16* __restrict__ shared_out, const float* __restrict__ shared_part, int shared_parts,
                const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate_vec, __nv_bfloat16* __restrict__ out, const __grid_constant__ SegmentedOut seg) {
+  pdl_wait();      // no early start for what follows: the chain ends here, the next kernel may be anybody's
   __shared__ int order_pos[8];
   __shared__ int present;
   __shared__ float red[8];
@@ -929,6 +937,7 @@ __global__ void __launch_bounds__(kCombineWarps * 32)
 combine_warp_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __restrict__ indices, int idx64,
                     const int* __restrict__ route_pos, int tokens, int top_k, int hidden, int experts,
                     __nv_bfloat16* __restrict__ out, const __grid_constant__ SegmentedOut seg) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * kCombineWarps + (threadIdx.x >> 5);
   if (t >= tokens) return;                                   // the whole warp
@@ -989,6 +998,8 @@ combine_warp_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __re
 
 // tile table of a dense [rows, k] matrix treated as one expert (the Qwen shared expert in prefill)
 __global__ void dense_tiles_kernel(int rows, int cap, int* num_tiles, int* tile_expert, int* tile_row0, int* tile_rows) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int tiles = (rows + cap - 1) / cap;
   for (int t = threadIdx.x; t < tiles; t += blockDim.x) {
     tile_expert[t] = 0; tile_row0[t] = t * cap; tile_rows[t] = min(cap, rows - t * cap);
@@ -996,6 +1007,11 @@ __global__ void dense_tiles_kernel(int rows, int cap, int* num_tiles, int* tile_
   if (threadIdx.x == 0) *num_tiles = tiles;
 }
 
+int check_launch(const char* what, cudaError_t e) {
+  if (e == cudaSuccess) return ERR_NONE;
+  set_error("%s: launch failed: %s", what, cudaGetErrorString(e));
+  return ERR_LAUNCH;
+}
 int check_launch(const char* what) {
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_error("%s: launch failed: %s", what, cudaGetErrorString(e)); return ERR_LAUNCH; }
@@ -1005,8 +1021,8 @@ int check_launch(const char* what) {
 }  // namespace
 
 int launch_dense_tiles(int rows, int tile_cap, int* num_tiles, int* tile_expert, int* tile_row0, int* tile_rows, cudaStream_t stream) {
-  dense_tiles_kernel<<<1, 256, 0, stream>>>(rows, tile_cap, num_tiles, tile_expert, tile_row0, tile_rows);
-  return check_launch("dense tiles");
+  return check_launch("dense tiles", launch_chained(dense_tiles_kernel, dim3(1), dim3(256), 0, stream, rows, tile_cap, num_tiles,
+                                                   tile_expert, tile_row0, tile_rows));
 }
 
 int launch_router_topk(const RouterArgs& a, cudaStream_t stream) {
@@ -1064,12 +1080,12 @@ int launch_route_sort(const SortArgs& a, cudaStream_t stream) {
   const int chunks = (int)((routes + kChunk - 1) / kChunk);
   const unsigned permute_blocks = a.permute_dst ? (unsigned)((a.permute_chunks + kSortThreads - 1) / kSortThreads) : 0;
   if (chunks <= 2 || !a.scratch || a.scratch_ints < (long long)chunks * a.experts) {
-    route_sort_kernel<<<1 + permute_blocks, kSortThreads, 0, stream>>>(a);
-    return check_launch("route sort");
+    return check_launch("route sort", launch_chained(route_sort_kernel, dim3(1 + permute_blocks), dim3(kSortThreads), 0, stream, a));
   }
-  route_hist_kernel<<<chunks + permute_blocks, kSortThreads, 0, stream>>>(a, a.scratch, chunks);
-  route_place_kernel<<<chunks, kSortThreads, 0, stream>>>(a, a.scratch, chunks);
-  return check_launch("route sort");
+  const int rc = check_launch("route sort", launch_chained(route_hist_kernel, dim3(chunks + permute_blocks), dim3(kSortThreads), 0,
+                                                            stream, a, a.scratch, chunks));
+  if (rc) return rc;
+  return check_launch("route sort", launch_chained(route_place_kernel, dim3(chunks), dim3(kSortThreads), 0, stream, a, a.scratch, chunks));
 }
 
 int launch_gather_rows(const __nv_bfloat16* x, const int* sorted_route, int top_k, long long routes, int hidden,
@@ -1092,13 +1108,13 @@ int launch_combine(const __nv_bfloat16* weighted, const void* indices, int idx64
     // a chain of load latencies (11.5 us at 7 tokens): then a token's columns are spread over several warps.
     const int passes = (hidden / 8 + 31) / 32;
     const int spread = std::max(1, std::min(passes, kCombineSpreadWarps / tokens));
-    combine_warp_kernel<<<dim3((tokens + kCombineWarps - 1) / kCombineWarps, spread), kCombineWarps * 32, 0, stream>>>(
-        weighted, indices, idx64, route_pos, tokens, top_k, hidden, experts, out, seg);
-    return check_launch("combine");
+    return check_launch("combine", launch_chained(combine_warp_kernel, dim3((tokens + kCombineWarps - 1) / kCombineWarps, spread),
+                                                  dim3(kCombineWarps * 32), 0, stream, weighted, indices, idx64, route_pos, tokens,
+                                                  top_k, hidden, experts, out, seg));
   }
   auto kernel = shared_parts > 0 ? combine_kernel<true> : combine_kernel<false>;
-  kernel<<<tokens, 256, 0, stream>>>(weighted, indices, idx64, route_pos, top_k, hidden, experts, shared_out, shared_part, shared_parts, x, gate_vec, out, seg);
-  return check_launch("combine");
+  return check_launch("combine", launch_chained(kernel, dim3(tokens), dim3(256), 0, stream, weighted, indices, idx64, route_pos, top_k,
+                                                hidden, experts, shared_out, shared_part, shared_parts, x, gate_vec, out, seg));
 }
 
 // ---- expert-parallel routing: global expert id -> this rank's local id, or -1 (absent) --------------------------
