@@ -409,7 +409,7 @@ def test_few_routes_kernel_takes_tables_of_wider_tiles():
     assert torch.equal(ops.combine_routes(y, idx, routes.route_pos).cpu(), _run_prefill(layer, x, idx, w))
 
 
-@pytest.mark.parametrize("tokens", [1, 5, 63, 192, 193, 600, 1030])
+@pytest.mark.parametrize("tokens", [1, 5, 63, 192, 193, 448, 449, 600, 1030])
 def test_shared_expert_in_parts_of_its_contraction(tokens):
     """The shared expert's down GEMM cut along k: eight parts, an uneven last part (600 tokens: 88 steps in six), the
     transposed kernel and the wide one.  The routes weigh nothing, so the result is the shared expert's; rounding as above

@@ -578,18 +578,19 @@ static bool takes_pair_kernel(const GroupedGemmArgs& a) {
 //   OLMoE Q8   8 routes per expert 209 | 112   64: 212 | 184    96: 215 | 234
 //   Qwen  Q8  34 routes per expert 267 | 150   51: 268 | 172    68: 268 | 236
 //   Qwen BF16  4 routes per expert 202 | 171   51: 207 | 186    68: 208 | 209
-//   one dense BF16 expert (the shared one), 128 tokens: 39 | 31   192: 48 | 33   256: 52 | 48   512: 55 | 72
-constexpr int kTsMaxRoutesQ4 = 88, kTsMaxRoutesQ8 = 76, kTsMaxRoutesBf16 = 64, kTsMaxRowsDense = 192;
-static bool takes_ts_kernel(int enc, long long rows, int experts, int variant) {
+//   one dense BF16 expert (the shared one), gate/up, 128 tokens: 23 | 20   192: 28 | 20   256: 29 | 33   512: 31 | 48
+//   the same, down GEMM, 192 tokens: 20 | 13   256: 23 | 15   384: 23 | 18   512: 24 | 24
+constexpr int kTsMaxRoutesQ4 = 88, kTsMaxRoutesQ8 = 76, kTsMaxRoutesBf16 = 64, kTsMaxRowsDense[2] = {192, 448};
+static bool takes_ts_kernel(int enc, long long rows, int experts, int variant, int mode) {
   if (variant == 2) return false;
-  if (enc == ENC_BF16) return rows <= (experts == 1 ? kTsMaxRowsDense : (long long)experts * kTsMaxRoutesBf16);
+  if (enc == ENC_BF16) return rows <= (experts == 1 ? kTsMaxRowsDense[mode] : (long long)experts * kTsMaxRoutesBf16);
   return rows <= (long long)experts * (enc == ENC_Q8 ? kTsMaxRoutesQ8 : kTsMaxRoutesQ4);
 }
 // The shared expert's down GEMM has few tiles and a long contraction (Qwen: 2048 rows, k 5632): without parts it runs on 16
 // CTAs at up to 64 tokens and on 48 at 1531.  Parts until the CTAs that fit the device have a tile each.
 // Down GEMM plus the combine that adds the parts, Qwen shape, us, before | now: 24 tokens 52 | 15, 128: 54 | 17, 1531: 76 | 62.
 int grouped_gemm_dense_splits(long long rows, int n_rows, int k) {
-  const bool ts = takes_ts_kernel(ENC_BF16, rows, 1, 0);
+  const bool ts = takes_ts_kernel(ENC_BF16, rows, 1, 0, 1);
   if (!ts && rows >= kPairMinRows) return 1;
   const long long tiles = ts ? (rows + kTileCapMin - 1) / kTileCapMin * (n_rows / 128) : (rows + kTileCapMax - 1) / kTileCapMax * (n_rows / BN);
   const long long slots = (long long)sm_count() * (ts ? 2 : 1);
@@ -597,7 +598,7 @@ int grouped_gemm_dense_splits(long long rows, int n_rows, int k) {
   return (int)std::max(1ll, std::min({want, (long long)kMaxDenseSplits, (long long)(k / 512)}));
 }
 int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant) {
-  return takes_ts_kernel(enc, rows, num_experts, variant) ? kTileCapMin : kTileCapMax;
+  return takes_ts_kernel(enc, rows, num_experts, variant, 0) ? kTileCapMin : kTileCapMax;
 }
 bool grouped_gemm_can_gather(const GroupedGemmArgs& a) { return a.mode == 0 && !takes_pair_kernel(a); }
 int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
@@ -605,7 +606,7 @@ int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
     if (a.gather_route) { set_error("grouped: the CTA-pair kernel takes gathered activation rows"); return ERR_BAD_ARGUMENT; }
     return launch_grouped_gemm_pair(a, stream);
   }
-  if (takes_ts_kernel(a.enc, a.total_rows, a.num_experts, a.variant)) {
+  if (takes_ts_kernel(a.enc, a.total_rows, a.num_experts, a.variant, a.mode)) {
     if (a.k % 128 || a.n_rows % (a.mode == 0 ? BN / 2 : BN) || a.total_rows <= 0 || a.max_tiles <= 0 ||
         (a.enc != ENC_BF16 && a.k > kMaxGroups * 128)) {
       set_error("grouped: unsupported shape (k %d, rows per expert %d)", a.k, a.n_rows);
