@@ -21,10 +21,10 @@ either mode -- instead of running a reference path.
 
 from __future__ import annotations
 
+import functools
 import itertools
 import threading
-from contextlib import contextmanager
-from typing import Any, Callable, Iterator
+from typing import Any, Callable
 
 from .formats import ContractError
 
@@ -41,6 +41,41 @@ class _Entry:
         self.reader = reader
         self.in_flight = 0
         self.closing = False
+
+
+class _Lease:
+    """One lease of a handle, taken on entry and given back on exit (a class, not a generator: every call of the operator
+    takes two)."""
+
+    __slots__ = ("_registry", "_handle", "_entry", "_depths")
+
+    def __init__(self, registry: "PackRegistry", handle: int) -> None:
+        self._registry, self._handle, self._entry, self._depths = registry, handle, None, None
+
+    def __enter__(self) -> Any:
+        if self._depths is not None:
+            raise RuntimeError("a lease is entered once")
+        registry, handle = self._registry, self._handle
+        depths = registry._depths()
+        depth = depths.get(handle, 0)
+        with registry._cv:
+            entry = registry._entries.get(handle)
+            if entry is None or (entry.closing and depth == 0):
+                raise RuntimeError(f"unknown or closed ExpertPack handle {handle}")
+            if depth == 0:
+                entry.in_flight += 1
+        depths[handle] = depth + 1
+        self._entry, self._depths = entry, depths
+        return entry.reader
+
+    def __exit__(self, *_: Any) -> None:
+        registry, handle, depths = self._registry, self._handle, self._depths
+        depths[handle] -= 1
+        if depths[handle] == 0:
+            del depths[handle]
+            with registry._cv:
+                self._entry.in_flight -= 1
+                registry._cv.notify_all()
 
 
 class PackRegistry:
@@ -94,26 +129,8 @@ class PackRegistry:
         for backend in listeners:
             backend.release_pack(handle)
 
-    @contextmanager
-    def lease(self, handle: int) -> Iterator[Any]:
-        depths = self._depths()
-        outermost = depths.get(handle, 0) == 0
-        with self._cv:
-            entry = self._entries.get(handle)
-            if entry is None or (entry.closing and outermost):
-                raise RuntimeError(f"unknown or closed ExpertPack handle {handle}")
-            if outermost:
-                entry.in_flight += 1
-        depths[handle] = depths.get(handle, 0) + 1
-        try:
-            yield entry.reader
-        finally:
-            depths[handle] -= 1
-            if depths[handle] == 0:
-                del depths[handle]
-                with self._cv:
-                    entry.in_flight -= 1
-                    self._cv.notify_all()
+    def lease(self, handle: int) -> "_Lease":
+        return _Lease(self, handle)
 
     def reader(self, handle: int) -> Any:
         if not self._depths().get(handle):
@@ -174,6 +191,11 @@ def expert_pack_for_handle(handle: int) -> Any:
     return _REGISTRY.reader(handle)
 
 
+@functools.lru_cache(maxsize=None)
+def _capability(torch: Any, index: int) -> tuple[int, int]:
+    return torch.cuda.get_device_capability(index)                # a device's capability does not change
+
+
 def platform_of(torch: Any, hidden_states: Any) -> str:
     """``cpu`` or ``cuda_sm100``; any other device raises, as the reference's
     ``_platform`` does for devices it does not know (``custom_op.py:149-169``)."""
@@ -182,7 +204,7 @@ def platform_of(torch: Any, hidden_states: Any) -> str:
         return "cpu"
     if kind != "cuda" or torch.version.hip:
         raise RuntimeError(f"uma_qmoe::moe_forward does not support {hidden_states.device}")
-    capability = torch.cuda.get_device_capability(hidden_states.device)
+    capability = _capability(torch, hidden_states.device.index)
     if capability != (10, 0):
         raise RuntimeError(f"CUDA implementation requires SM100, observed sm_{capability[0]}{capability[1]}")
     return PLATFORM

@@ -74,12 +74,13 @@ class _Workspace:
     `cache_summary()` and `release_pack()` look at the copy once the event has completed.  Nothing on the hot
     path waits for the device."""
 
-    __slots__ = ("kind", "buffer", "host", "event", "tokens")
+    __slots__ = ("kind", "buffer", "status", "host", "event", "tokens")
 
     def __init__(self, kind: str, buffer: Any, tokens: int) -> None:
         import torch
 
         self.kind, self.buffer, self.tokens = kind, buffer, tokens
+        self.status = buffer[:16].view(torch.int32)
         self.host = torch.zeros(4, dtype=torch.int32).pin_memory()
         self.event: Any = None
 
@@ -88,7 +89,7 @@ class _Workspace:
 
         if torch.cuda.is_current_stream_capturing():
             return                                   # a captured call reports through the workspace only
-        self.host.copy_(self.buffer[:16].view(torch.int32), non_blocking=True)
+        self.host.copy_(self.status, non_blocking=True)
         if self.event is None:
             self.event = torch.cuda.Event()
         self.event.record(stream)

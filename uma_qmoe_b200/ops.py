@@ -60,7 +60,9 @@ class DeviceSharedExpert:
 
 
 def _stream(device: torch.device) -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    # the handle alone: building a torch.cuda.Stream object for it costs a call 5 us
+    index = device.index
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index))
 
 
 def _require_cuda_bf16(t: torch.Tensor, what: str) -> None:
