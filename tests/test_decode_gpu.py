@@ -67,6 +67,28 @@ def test_device_packer_rounding_boundaries_and_layouts(enc, groups, offset):
         assert np.array_equal(scales.cpu().numpy(), np.concatenate([s for _, s in want]))
 
 
+@pytest.mark.parametrize("enc", ["q4_group128", "q8_group128"])
+def test_device_packer_every_ratio_of_bf16_mantissas(enc):
+    """Every BF16 mantissa against every BF16 maximum over the exponents whose codes are not all zero: every quotient a group
+    of normal weights can have, exact ties between two codes among them."""
+    ops = _ops()
+    quant = orc.quantize_q4 if enc == "q4_group128" else orc.quantize_q8
+    m = 1 + np.arange(128, dtype=np.float32) / 128
+    rows = []
+    for am in m:
+        for e in range(10):
+            g = m * np.float32(2.0 ** -e)
+            g[g > am] /= 2
+            rows.append(np.concatenate(([am], g[1:])).astype(np.float32))
+            rows.append(np.concatenate(([am], -g[:-1])).astype(np.float32))
+    v = torch.from_numpy(np.stack(rows)).to(torch.bfloat16)
+    assert np.array_equal(v.float().numpy(), np.stack(rows))
+    codes, scales = ops.quantize_groups((v * 2.0 ** -7).to(DEV), enc)
+    want_codes, want_scales = quant(v.float().numpy() * np.float32(2.0 ** -7))
+    assert np.array_equal(codes.cpu().numpy().view(np.uint8), np.asarray(want_codes).view(np.uint8).reshape(-1))
+    assert np.array_equal(scales.cpu().numpy(), want_scales)
+
+
 def test_olmoe_decode_golden(golden_dir):
     g = np.load(golden_dir / "olmoe_decode.npz")
     x = bits_to_bf16(g["x_bits"])

@@ -11,12 +11,12 @@ namespace {
 // all-zero group), code = clip(rint(g / scale), -qmax, qmax)
 // (src/uma_qmoe/q4.py:136-165, src/uma_qmoe/target_pack.py:92-112 in the reference).
 //
-// The bound is the stream: 2 bytes read and 0.53 (Q4) or 1.03 (Q8) written per weight.  A correctly rounded division per
-// weight cost more issue slots than that takes, so the quotient is multiplied out: with inv = 1/scale correctly rounded,
-// r = g * inv is within 2^-23 |r| of the exact quotient, less than 4e-5 for |r| <= 256.  Unless r lies within 1e-4 of a
-// rounding boundary, the integer nearest to r is the one the divided and rounded quotient has; lanes with such an r, and
-// groups with an infinite inv (a scale below 2^-128), an infinity or a NaN, divide.
-// Measured, 134 M weights to Q4: 130 us (2.6 TB/s); a warp per group with 8-byte loads and four divisions a lane took 170.
+// The bound is the stream: 2 bytes read and 0.53 (Q4) or 1.03 (Q8) written per weight; what has to stay below it is the
+// number of instructions per weight.  The quotient g / scale is v * inv with inv = 1/scale correctly rounded, corrected once by
+// its exact remainder (Markstein, IBM J. Res. Dev. 34, 1990): the correctly rounded quotient, with three operations.  Quotients
+// on the boundary between two codes are common, not rare (BF16 weights over a BF16 maximum: one weight in 200), so a path that
+// divides next to a boundary is taken by three warps in four.  Groups with a scale below 2^-100 (the remainder would
+// underflow), a scale whose mantissa is all ones (excepted by the theorem), an infinity or a NaN divide.
 constexpr int kQgLoads = 4, kQgWarps = 8;
 template <int QMAX, bool NIBBLES, bool WIDE>
 __global__ void __launch_bounds__(kQgWarps * 32)
@@ -64,20 +64,24 @@ quantize_groups_kernel(const __nv_bfloat16* __restrict__ src, long long groups, 
     if (scale == 0.f) scale = 1.f;
     const float inv = __frcp_rn(scale);
     constexpr float kMagic = 12582912.f;                                    // 1.5 * 2^23: the ulp of a sum with it is 1
-    float n[8], worst = 0.f;                                                // n = minus the nearest integer
+    divide = divide || !(scale > 7.8886091e-31f) || !(am < 3.0e38f) || (__float_as_uint(scale) & 0x7fffffu) == 0x7fffffu;
+    float n[8];                                                             // minus the code
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float v = __uint_as_float(j & 1 ? w[j >> 1] & 0xffff0000u : w[j >> 1] << 16);
-      n[j] = kMagic - __fmaf_rn(v, inv, kMagic);
-      const float d = fabsf(__fmaf_rn(v, inv, n[j]));
-      worst = fmaxf(worst, d);
+      const float q0 = __fmul_rn(v, inv);
+      const float q = __fmaf_rn(__fmaf_rn(-q0, scale, v), inv, q0);
+      n[j] = kMagic - __fadd_rn(q, kMagic);                                 // nearest integer, ties to even
     }
-    divide = divide || !(inv < 3.0e38f) || !(am < 3.0e38f) || !(worst < 0.4999f);
     if (divide) {
-#pragma unroll
+#pragma unroll 1
       for (int j = 0; j < 8; ++j) {
-        float r = rintf(__fdiv_rn(__uint_as_float(j & 1 ? w[j >> 1] & 0xffff0000u : w[j >> 1] << 16), scale));
-        n[j] = -fminf(fmaxf(r, (float)-QMAX), (float)QMAX);
+        const uint32_t word = j < 4 ? (j < 2 ? w[0] : w[1]) : (j < 6 ? w[2] : w[3]);
+        float r = rintf(__fdiv_rn(__uint_as_float(j & 1 ? word & 0xffff0000u : word << 16), scale));
+        r = -fminf(fmaxf(r, (float)-QMAX), (float)QMAX);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (k == j) n[k] = r;
       }
     }
     if (g >= groups) continue;
