@@ -989,8 +989,9 @@ def main() -> None:
                     help="expert encoding of the --only decode / gemm cases (default: q4 for olmoe, q8 for qwen)")
     ap.add_argument("--by-index", action="store_true",
                     help="--only gemm: the gate/up GEMM fetches its activation rows by index (as the operator runs it)")
-    ap.add_argument("--variant", type=int, default=0, choices=(0, 1, 2),
-                    help="grouped GEMM kernel of the --only gemm case: 0/1 one CTA per tile (default), 2 CTA pairs")
+    ap.add_argument("--variant", type=int, default=0, choices=(0, 1, 2, 3),
+                    help="grouped GEMM kernel of the --only gemm case: 0 the library picks (default), 1 one CTA per tile, 2 CTA pairs, "
+                         "3 transposed tiles")
     args = ap.parse_args()
     if args.only != "all":
         kernel_case(args)

@@ -428,3 +428,52 @@ def test_shared_expert_in_parts_of_its_contraction(tokens):
     want = (gate[:, None] * y).cpu().float()
     assert (got - want).norm() <= 2.0 ** -7 * want.norm()
     assert (got - want).abs().max() <= 2.0 ** -6 * want.abs().max()
+
+
+def _kernels(call, tmp_path):
+    """Which grouped GEMM kernels a call launches, from the nodes of a graph it is captured into."""
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        call()                                                   # whatever a first call sets up, outside the capture
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        graph.enable_debug_mode()
+        with torch.cuda.graph(graph, stream=stream):
+            call()
+    graph.debug_dump(str(tmp_path / "graph.dot"))
+    text = (tmp_path / "graph.dot").read_text()
+    names = ("grouped_gemm_kernel", "grouped_pair_kernel", "grouped_ts_kernel")
+    assert any(name in text for name in names), text[:2000]
+    return {name for name in names if name in text}
+
+
+@pytest.mark.parametrize("encoding,line", [("q4_group128", 88), ("q8_group128", 76), ("bf16_le", 64)])
+def test_variants_name_their_kernels_on_both_sides_of_the_line(encoding, line, tmp_path):
+    """Variants 1, 2 and 3 run the kernel they name at any size, variant 0 changes over at `line` routes per expert.  One-CTA
+    and transposed tiles multiply the same BF16 operands and add the same 16-k steps in the same order: equal bits."""
+    from uma_qmoe_b200 import ops
+    from uma_qmoe_b200.stack import random_layer
+    layer = random_layer(syn.OLMOE, encoding, 8, torch.device(DEV), experts=range(16))
+    gen = torch.Generator(device=DEV).manual_seed(line)
+    quant = encoding != "bf16_le"
+    for routes in (16 * line, 16 * line + 1):
+        idx = (torch.arange(routes, device=DEV) % 16)[:, None]
+        x = torch.randn(routes, 2048, device=DEV, generator=gen).to(torch.bfloat16)
+        w = torch.rand(routes, 1, device=DEV, generator=gen)
+        inter1, y1 = _stagewise(layer, x, idx, w, variant=1)
+        inter3, y3 = _stagewise(layer, x, idx, w, variant=3)
+        assert torch.equal(inter1, inter3) and torch.equal(y1, y3)
+        by_size = "grouped_ts_kernel" if routes == 16 * line else "grouped_gemm_kernel"
+        for variant, want in enumerate((by_size, "grouped_gemm_kernel", "grouped_pair_kernel", "grouped_ts_kernel")):
+            assert _kernels(lambda: _stagewise_launches(layer, x, idx, w, variant), tmp_path) == {want}, (routes, variant)
+        source = ops.gather_rows(x, None, 1, permute=True) if quant else x
+        table = ops.route_sort(idx, w, layer.num_experts)
+        assert _kernels(lambda: ops.grouped_gemm_by_index(layer, source, table, 1, permute_out=quant), tmp_path) == {by_size}
+
+
+def _stagewise_launches(layer, x, idx, w, variant):
+    """:func:`_stagewise` without its checks, so that it can be captured."""
+    from uma_qmoe_b200 import ops
+    r = ops.route_sort(idx, w, layer.num_experts)
+    xs = ops.gather_rows(x, r.sorted_route, idx.shape[1], permute=layer.encoding != "bf16_le")
+    inter = ops.grouped_gemm(layer, 0, xs, r, permute_out=layer.encoding != "bf16_le", variant=variant)
+    return ops.grouped_gemm(layer, 1, inter, r, route_weight=r.sorted_weight, variant=variant)

@@ -162,7 +162,7 @@ int umaq_grouped_gemm(const umaq_layer* layer, int mode, const void* act_bf16, l
                       const int* tile_table, int max_tiles, const float* route_weight, int permute_out, void* out_bf16,
                       unsigned* status, int variant, void* stream) {
   if (!layer || !act_bf16 || !num_tiles || !tile_table || !out_bf16 || !status || (mode != 0 && mode != 1) ||
-      variant < 0 || variant > 2) {
+      variant < 0 || variant > 3) {
     set_error("umaq_grouped_gemm: bad argument");
     return ERR_BAD_ARGUMENT;
   }
@@ -195,7 +195,8 @@ int umaq_grouped_gemm_by_index(const umaq_layer* layer, const void* hidden_bf16,
   g.num_tiles = num_tiles; g.tile_expert = tile_table; g.tile_row0 = tile_table + max_tiles;
   g.tile_rows = tile_table + 2 * max_tiles; g.max_tiles = max_tiles; g.tile_cap = kTileCapMax;
   g.out = static_cast<__nv_bfloat16*>(out_bf16); g.out_stride = g.n_rows;
-  g.permute_out = permute_out; g.status = status; g.variant = 1;
+  g.permute_out = permute_out; g.status = status;
+  g.variant = grouped_gemm_can_gather(g) ? 0 : 1;          // the pair kernel takes gathered rows only
   g.gather_route = sorted_route; g.gather_top_k = top_k;
   return launch_grouped_gemm(g, static_cast<cudaStream_t>(stream));
 }

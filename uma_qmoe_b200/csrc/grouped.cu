@@ -582,7 +582,7 @@ static bool takes_pair_kernel(const GroupedGemmArgs& a) {
 //   the same, down GEMM, 192 tokens: 20 | 13   256: 23 | 15   384: 23 | 18   512: 24 | 24
 constexpr int kTsMaxRoutesQ4 = 88, kTsMaxRoutesQ8 = 76, kTsMaxRoutesBf16 = 64, kTsMaxRowsDense[2] = {192, 448};
 static bool takes_ts_kernel(int enc, long long rows, int experts, int variant, int mode) {
-  if (variant == 2) return false;
+  if (variant != 0) return variant == 3;
   if (enc == ENC_BF16) return rows <= (experts == 1 ? kTsMaxRowsDense[mode] : (long long)experts * kTsMaxRoutesBf16);
   return rows <= (long long)experts * (enc == ENC_Q8 ? kTsMaxRoutesQ8 : kTsMaxRoutesQ4);
 }

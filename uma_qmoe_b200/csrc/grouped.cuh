@@ -57,8 +57,9 @@ struct GroupedGemmArgs {
   const float* route_weight;
   int permute_out;
   unsigned* status;
-  int variant;                // 0: by size; 1: one CTA per tile (grouped.cu); 2: persistent CTA pairs (grouped_pair.cu)
-  // mode 0 on the one-CTA kernel, optional: act = [tokens, k] and the kernel fetches row sorted_route[r] / top_k
+  int variant;                // 0: by size; 1: one CTA per tile (grouped.cu); 2: persistent CTA pairs (grouped_pair.cu);
+                              // 3: transposed tiles (grouped_ts.cu)
+  // mode 0 on the one-CTA and the transposed kernel, optional: act = [tokens, k] and the kernel fetches row sorted_route[r] / top_k
   // for sorted route r itself (no gathered copy of the activations)
   const int* gather_route;
   int gather_top_k;

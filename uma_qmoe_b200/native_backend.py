@@ -400,7 +400,7 @@ class MixedTargetNativeBackend:
         ones = torch.ones((n, 1), dtype=torch.float32, device=device)
         routes = ops.route_sort(torch.zeros((n, 1), dtype=torch.int32, device=device), ones, 1)
         act = ops.gather_rows(input_tensor.contiguous(), None, 1, permute=True)      # the k order of the quantised GEMM
-        return ops.grouped_gemm(hit, 1, act, routes, variant=1)
+        return ops.grouped_gemm(hit, 1, act, routes)
 
     def q4_linear(self, input_tensor: Any, pack_handle: int, tensor_name: str):
         return self._linear(input_tensor, pack_handle, tensor_name, "q4_group128")

@@ -216,7 +216,7 @@ def grouped_gemm(layer: DeviceLayer, mode: int, act: torch.Tensor, routes: Sorte
                  route_weight: Optional[torch.Tensor] = None, permute_out: bool = False,
                  out: Optional[torch.Tensor] = None, variant: int = 0) -> torch.Tensor:
     """One grouped GEMM launch (mode 0: gate/up + SwiGLU, mode 1: down * routing weight).
-    ``variant``: 0/1 the default one-CTA-per-tile kernel, 2 the CTA-pair (cta_group::2) kernel."""
+    ``variant``: 0 the library picks, 1 one-CTA tiles, 2 the CTA-pair (cta_group::2) kernel, 3 transposed tiles."""
     _require_cuda_bf16(act, "activations")
     n = layer.intermediate if mode == 0 else layer.hidden
     if out is None:
