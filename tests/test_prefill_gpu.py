@@ -462,12 +462,13 @@ def test_variants_name_their_kernels_on_both_sides_of_the_line(encoding, line, t
         inter1, y1 = _stagewise(layer, x, idx, w, variant=1)
         inter3, y3 = _stagewise(layer, x, idx, w, variant=3)
         assert torch.equal(inter1, inter3) and torch.equal(y1, y3)
-        by_size = "grouped_ts_kernel" if routes == 16 * line else "grouped_gemm_kernel"
-        for variant, want in enumerate((by_size, "grouped_gemm_kernel", "grouped_pair_kernel", "grouped_ts_kernel")):
-            assert _kernels(lambda: _stagewise_launches(layer, x, idx, w, variant), tmp_path) == {want}, (routes, variant)
+        one_cta, pair, transposed = {"grouped_gemm_kernel"}, {"grouped_pair_kernel"}, {"grouped_ts_kernel"}
+        by_size = one_cta | transposed if routes == 16 * line else one_cta        # below the line the counts decide
+        for variant, want in enumerate((by_size, one_cta, pair, transposed)):
+            assert _kernels(lambda: _stagewise_launches(layer, x, idx, w, variant), tmp_path) == want, (routes, variant)
         source = ops.gather_rows(x, None, 1, permute=True) if quant else x
         table = ops.route_sort(idx, w, layer.num_experts)
-        assert _kernels(lambda: ops.grouped_gemm_by_index(layer, source, table, 1, permute_out=quant), tmp_path) == {by_size}
+        assert _kernels(lambda: ops.grouped_gemm_by_index(layer, source, table, 1, permute_out=quant), tmp_path) == by_size
 
 
 def _stagewise_launches(layer, x, idx, w, variant):
@@ -477,3 +478,35 @@ def _stagewise_launches(layer, x, idx, w, variant):
     xs = ops.gather_rows(x, r.sorted_route, idx.shape[1], permute=layer.encoding != "bf16_le")
     inter = ops.grouped_gemm(layer, 0, xs, r, permute_out=layer.encoding != "bf16_le", variant=variant)
     return ops.grouped_gemm(layer, 1, inter, r, route_weight=r.sorted_weight, variant=variant)
+
+
+@pytest.mark.parametrize("model,encoding,tokens", [("olmoe", "q4_group128", 384), ("olmoe", "q4_group128", 704),
+                                                   ("olmoe", "q8_group128", 512), ("olmoe", "bf16_le", 224), ("olmoe", "bf16_le", 512),
+                                                   ("qwen", "q8_group128", 960), ("qwen", "bf16_le", 900)])
+def test_concentrated_routes_take_the_one_cta_kernel(model, encoding, tokens):
+    """Below the line of routes per expert the kernel is picked from the counts on the device: few experts in use -> one-CTA
+    tiles, all of them -> transposed ones.  Either way and through the exported stages (which pick from the table), the bits are
+    those of the stages run on the one-CTA kernel; an absent route counts like one that weighs nothing."""
+    from uma_qmoe_b200 import ops
+    from uma_qmoe_b200.stack import random_layer
+    shape = syn.OLMOE if model == "olmoe" else syn.QWEN
+    layer = random_layer(shape, encoding, 5, torch.device(DEV))
+    gen = torch.Generator(device=DEV).manual_seed(tokens)
+    k = shape.top_k
+    x = torch.randn(tokens, shape.hidden, device=DEV, generator=gen).to(torch.bfloat16)
+    w = torch.rand(tokens, k, device=DEV, generator=gen)
+    spread = (torch.arange(tokens * k, device=DEV) % shape.experts).reshape(tokens, k)     # as even as routes can be
+    narrow = (torch.arange(tokens * k, device=DEV) % (k + k // 2)).reshape(tokens, k)
+    absent = spread.clone()
+    absent[::3, 1] = -1
+    present = torch.where(absent >= 0, w, 0.0)
+    for idx, routes, weights, transposed in ((narrow, narrow, w, 0), (spread, spread, w, 1), (absent, spread, present, None)):
+        ws = ops.prefill_workspace(layer, tokens, k, None, torch.device(DEV))
+        y = ops.moe_prefill(layer, x, idx, w, ws)
+        assert ops.prefill_status(ws) == 0
+        if transposed is not None:
+            assert int(ws[64:68].view(torch.int32).item()) == transposed
+        _, want = _stagewise(layer, x, routes, weights, variant=1)       # the gather stage takes present routes only
+        assert torch.equal(y, want)
+        _, picked = _stagewise(layer, x, routes, weights, variant=0)
+        assert torch.equal(picked, want)

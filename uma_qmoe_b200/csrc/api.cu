@@ -197,7 +197,7 @@ int umaq_grouped_gemm_by_index(const umaq_layer* layer, const void* hidden_bf16,
   g.out = static_cast<__nv_bfloat16*>(out_bf16); g.out_stride = g.n_rows;
   g.permute_out = permute_out; g.status = status;
   g.variant = grouped_gemm_can_gather(g) ? 0 : 1;          // the pair kernel takes gathered rows only
-  g.gather_route = sorted_route; g.gather_top_k = top_k;
+  g.gather_route = sorted_route; g.gather_top_k = top_k; g.most = (routes + top_k - 1) / top_k;
   return launch_grouped_gemm(g, static_cast<cudaStream_t>(stream));
 }
 
@@ -338,6 +338,10 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   sa.num_tiles = reinterpret_cast<int*>(at(pl.num_tiles));
   sa.tile_expert = tiles; sa.tile_row0 = tiles + pl.max_tiles; sa.tile_rows = tiles + 2 * pl.max_tiles;
   sa.max_tiles = pl.max_tiles; sa.tile_cap = grouped_gemm_tile_cap(layer->encoding, routes, E, 0); sa.status = status;
+  if (grouped_gemm_choice_on_device(layer->encoding, routes, E, tokens, 0)) {
+    sa.use_ts = reinterpret_cast<int*>(at(pl.status) + 64);
+    sa.choice = grouped_gemm_choice(layer->encoding, I, H);
+  }
   sa.scratch = reinterpret_cast<int*>(at(pl.sort_scratch)); sa.scratch_ints = pl.sort_ints;
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(at(pl.xs));
   GroupedGemmArgs g{};
@@ -345,7 +349,7 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   g.total_rows = routes;
   g.w0 = layer->gate; g.s0 = layer->gate_scales; g.w1 = layer->up; g.s1 = layer->up_scales;
   g.num_tiles = sa.num_tiles; g.tile_expert = sa.tile_expert; g.tile_row0 = sa.tile_row0; g.tile_rows = sa.tile_rows;
-  g.max_tiles = pl.max_tiles; g.tile_cap = sa.tile_cap;
+  g.max_tiles = pl.max_tiles; g.tile_cap = sa.tile_cap; g.most = tokens; g.use_ts = sa.use_ts;
   g.out = reinterpret_cast<__nv_bfloat16*>(at(pl.inter)); g.out_stride = I; g.permute_out = quant; g.status = status;
   const bool by_index = grouped_gemm_can_gather(g);
   if (by_index && quant && !rows_k_permuted && H % 8 == 0 && !(reinterpret_cast<uintptr_t>(hidden_bf16) & 15)) {

@@ -114,6 +114,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const bool gather = MODE == 0 && p.gather_route != nullptr;
 
   pdl_launch_dependents();
+  if (p.conditional && !launch_runs(p)) return pdl_wait();    // read before the wait: see launch_grouped_gemm
   if (tid == 0) {
     const uint32_t in_count = gather ? kGatherThreads + (ENC == ENC_BF16 ? 1 : 0) : 1;
     for (int s = 0; s < kInStages; ++s) { mbar_init(&sh.in_full[s], in_count); mbar_init(&sh.in_empty[s], 1); }
@@ -600,6 +601,27 @@ int grouped_gemm_dense_splits(long long rows, int n_rows, int k) {
 int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant) {
   return takes_ts_kernel(enc, rows, num_experts, variant, 0) ? kTileCapMin : kTileCapMax;
 }
+// The lines above suppose that the routes spread over the experts.  Where they concentrate on a few, the transposed kernel
+// converts an expert's weights once per 64 routes and the one-CTA kernel once per 256, and the one-CTA kernel wins: 512 tokens
+// on 8 of 64 experts, whole operator, us, one-CTA | transposed: OLMoE Q4 65 | 100, Q8 77 | 132, BF16 67 | 109.  The counts
+// are on the device, so both kernels are launched and the one that is not wanted returns.  That costs a call 2.5 us where the
+// transposed kernel runs and 8 us where the other one does.  What decides is the number of waves (gate/up counted twice; half
+// ones where two CTAs share an SM): with these costs, over 400 routings (tokens 80 to 1320, all experts down to top-k of
+// them, the skewed router), the transposed kernel is the better one below 2 (Q4), 9/5 (Q8) and 7/4 (BF16) times the other's
+// waves; that pick is 0.1 to 0.9 % off the better one on average.  Up to 192 routes for any expert it could not win back what
+// it costs: 160 tokens on 16 experts, OLMoE Q4, one-CTA | transposed 56 | 65 (on all 64: 165 | 90).
+constexpr long long kChoiceMinRoutes = 192;
+bool grouped_gemm_choice_on_device(int enc, long long rows, int num_experts, long long most, int variant) {
+  return variant == 0 && num_experts > 1 && takes_ts_kernel(enc, rows, num_experts, 0, 0) &&
+         (most > 0 ? std::min(most, rows) : rows) > kChoiceMinRoutes;
+}
+TileChoice grouped_gemm_choice(int enc, int inter, int hidden) {
+  TileChoice c{};
+  c.cols_gate = inter / (BN / 2); c.cols_down = hidden / BN; c.sms = sm_count();
+  c.num = enc == ENC_Q4 ? 2 : enc == ENC_Q8 ? 9 : 7;
+  c.den = enc == ENC_Q4 ? 1 : enc == ENC_Q8 ? 5 : 4;
+  return c;
+}
 bool grouped_gemm_can_gather(const GroupedGemmArgs& a) { return a.mode == 0 && !takes_pair_kernel(a); }
 int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
   if (takes_pair_kernel(a)) {
@@ -613,7 +635,17 @@ int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
       return ERR_BAD_ARGUMENT;
     }
     if (a.gather_route && (a.mode != 0 || a.gather_top_k < 1)) { set_error("grouped: rows are fetched by index only for the gate/up GEMM"); return ERR_BAD_ARGUMENT; }
-    return launch_grouped_gemm_ts(a, stream);
+    if (!grouped_gemm_choice_on_device(a.enc, a.total_rows, a.num_experts, a.most, a.variant)) return launch_grouped_gemm_ts(a, stream);
+    // The one-CTA kernel second: where it is not wanted its CTAs start under the end of the other one and leave with it.  It
+    // may look at the counts before its programmatic wait: the transposed kernel, an ordinary launch, started after they
+    // were written.
+    GroupedGemmArgs b = a;
+    b.conditional = 1;
+    if (a.use_ts) b.tile_cap = kTileCapMin;
+    const int rc = launch_grouped_gemm_ts(b, stream);
+    if (rc) return rc;
+    b.conditional = 2;
+    return launch_grouped_gemm_single(b, stream);
   }
   return launch_grouped_gemm_single(a, stream);
 }
@@ -663,6 +695,8 @@ int launch_grouped_gemm_single(const GroupedGemmArgs& a, cudaStream_t stream) {
   { static const int dbg = [] { const char* v = std::getenv("UMAQ_GEMM_DEBUG"); return v ? std::atoi(v) : 0; }(); p.debug = dbg; }
   p.tma_out = tma_out;
   p.status = a.status;
+  p.conditional = a.conditional; p.use_ts = a.use_ts;
+  if (a.conditional) p.choice = grouped_gemm_choice(a.enc, a.mode == 0 ? a.n_rows : a.k, a.mode == 0 ? a.k : a.n_rows);
   p.gather_route = a.gather_route; p.gather_top_k = a.gather_top_k; p.gather_src = static_cast<const __nv_bfloat16*>(a.act);
   const int n_tiles = a.n_rows / (a.mode == 0 ? BN / 2 : BN);
 #define UMAQ_DISPATCH(E)                                                                       \

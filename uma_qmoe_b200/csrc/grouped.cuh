@@ -9,6 +9,21 @@
 
 namespace umaq {
 
+constexpr int kTileCapMin = 64, kTileCapMax = 256;   // routes of a tile: transposed kernel (grouped_ts.cu), the others
+
+// The choice between the one-CTA and the transposed kernel when routes concentrate on some experts: see grouped.cu.
+struct TileChoice {
+  int cols_gate, cols_down;   // column tiles of a row tile of the one-CTA kernel in either GEMM; the transposed one has twice as many
+  int sms;
+  int num, den;               // transposed tiles while den * their waves < num * the waves of one-CTA tiles
+};
+#ifdef __CUDACC__
+__host__ __device__ inline bool transposed_is_faster(const TileChoice& c, int tiles64, int tiles256) {
+  auto waves = [&](int t) { return 2 * ((t * c.cols_gate + c.sms - 1) / c.sms) + (t * c.cols_down + c.sms - 1) / c.sms; };
+  return c.den * waves(2 * tiles64) < c.num * 2 * waves(tiles256);        // in half waves: two transposed CTAs share an SM
+}
+#endif
+
 // Device-side view handed to the grouped GEMM kernel.
 struct GroupedParams {
   int k;                      // contraction length
@@ -34,6 +49,11 @@ struct GroupedParams {
   const int* gather_route;
   int gather_top_k;
   const __nv_bfloat16* gather_src;
+  // 1: this launch runs if transposed tiles are wanted, 2: if one-CTA tiles are, 0: always.  The answer is *use_ts, or
+  // follows from the tile table (entries of up to 256 routes) where use_ts is null
+  int conditional;
+  const int* use_ts;
+  TileChoice choice;
   int debug;
   int tma_out;                // mode 1, staged results: map_b1 describes `out` and whole 32-row groups leave by tensor store
 };
@@ -51,6 +71,9 @@ struct GroupedGemmArgs {
   const int* num_tiles; const int* tile_expert; const int* tile_row0; const int* tile_rows;
   int max_tiles;
   int tile_cap;               // most routes of a table entry
+  long long most;             // most routes an expert can have (0: total_rows)
+  const int* use_ts;          // device word of the sort whose table was cut for either kernel (null: decided from the table)
+  int conditional;            // set by launch_grouped_gemm: see GroupedParams
   int k_splits;               // > 1 (BF16 down GEMM without routing weights): partial sums into `part`, `out` is not written
   float* part;                // [k_splits, total_rows, n_rows] float32
   __nv_bfloat16* out; long long out_stride;
@@ -75,10 +98,12 @@ int launch_grouped_gemm_ts(const GroupedGemmArgs& a, cudaStream_t stream);
 
 // Routes per tile that suit the kernel launch_grouped_gemm picks for a layer: the cap to build the tile table with.
 int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant);
+// Whether that pick has to be made on the device, from the routes that the experts have; `most`: the most one can have
+bool grouped_gemm_choice_on_device(int enc, long long rows, int num_experts, long long most, int variant);
+TileChoice grouped_gemm_choice(int enc, int inter, int hidden);
 // Parts the contraction of a dense BF16 down GEMM (the shared expert's) is cut into
 int grouped_gemm_dense_splits(long long rows, int n_rows, int k);
 constexpr int kMaxDenseSplits = 8;
-constexpr int kTileCapMin = 64, kTileCapMax = 256;
 
 // ---- routing (route.cu) ---------------------------------------------------------------------------
 struct RouterArgs {
@@ -102,7 +127,8 @@ struct SortArgs {
   float* sorted_weight;            // [routes]
   int* num_tiles; int* tile_expert; int* tile_row0; int* tile_rows;   // 128-route tiles
   int max_tiles;
-  int tile_cap;                    // routes per tile
+  int tile_cap;                    // routes per tile, unless use_ts is given
+  int* use_ts; TileChoice choice;  // optional: the sort picks the kernel, cuts the table for it and writes 1 (transposed) or 0
   unsigned* status;
   // optional: rows of x in the k order of the quantised GEMMs, written by further CTAs of the first launch
   const __nv_bfloat16* permute_src; __nv_bfloat16* permute_dst; long long permute_chunks;   // 16-byte chunks

@@ -123,8 +123,10 @@ struct TsTile {
   int part, k0, k1;                         // part of the contraction, its first and end step
 };
 
-// tile table entry -> one of its `subs` parts of at most NMAX routes (equal parts, multiples of 16); nrows 0: no such part
-template <bool SPLIT>
+// tile table entry -> one of its `subs` parts of at most NMAX routes (equal parts, multiples of 16); nrows 0: no such part.
+// WIDE: entries may have more than NMAX routes (a table cut for the other kernels).  A template parameter, since the branch
+// costs every role of every tile 2 % of a small batch.
+template <bool SPLIT, bool WIDE>
 __device__ __forceinline__ TsTile ts_tile(const GroupedParams& p, int it, int n_col, int nk) {
   TsTile t;
   t.part = 0; t.k0 = 0; t.k1 = nk;
@@ -136,9 +138,14 @@ __device__ __forceinline__ TsTile ts_tile(const GroupedParams& p, int it, int n_
   }
   const int m = it / n_col;
   t.col = it - m * n_col;
-  const int tm = p.subs == 1 ? m : m / p.subs, sub = m - tm * p.subs;
+  // every entry's first part, then every entry's second one: the parts that exist spread evenly over the CTAs
+  int sub = 0, tm = m;
+  if (WIDE) {
+    const int entries = *p.num_tiles;
+    sub = m / entries; tm = m - sub * entries;
+  }
   t.expert = p.tile_expert[tm]; t.row0 = p.tile_row0[tm]; t.nrows = p.tile_rows[tm];
-  if (p.subs > 1) {
+  if (WIDE) {
     const int parts = (t.nrows + NMAX - 1) / NMAX;
     const int each = ((t.nrows + parts - 1) / parts + 15) & ~15;
     t.row0 += sub * each;
@@ -147,7 +154,7 @@ __device__ __forceinline__ TsTile ts_tile(const GroupedParams& p, int it, int n_
   return t;
 }
 
-template <int ENC, int MODE>
+template <int ENC, int MODE, bool WIDE>
 __global__ void __launch_bounds__(TsShape<ENC>::kThreads, 2)
 grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant__ CUtensorMap map_w0,
                   const __grid_constant__ CUtensorMap map_w1, const GroupedParams p) {
@@ -172,6 +179,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
   const bool gather = MODE == 0 && p.gather_route != nullptr;
 
   pdl_launch_dependents();
+  if (p.conditional && !launch_runs(p)) return;                        // an ordinary launch: what it reads here was written before
   if (tid == 0) {
     for (int s = 0; s < kBStages; ++s) { mbar_init(&sh.in_full[s], gather ? kTsGatherThreads : 1); mbar_init(&sh.in_empty[s], 1); }
     for (int s = 0; s < kPStages; ++s) { mbar_init(&sh.p_full[s], 1); mbar_init(&sh.p_empty[s], kQuant ? S::kConvertWarps : 1); }
@@ -189,7 +197,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh.tmem_base;
-  const int total = *p.num_tiles * p.subs * n_col * (kSplit ? p.k_splits : 1);
+  const int total = *p.num_tiles * (WIDE ? p.subs : 1) * n_col * (kSplit ? p.k_splits : 1);
   auto fail = [&]() { atomicExch(p.status, (unsigned)ERR_DEVICE_TIMEOUT); *abort_flag = 1; };
 
   if (warp == 0) {
@@ -201,7 +209,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     uint32_t seq = 0;
     for (int it = first; it < total; it += step) {
       if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
-      const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
+      const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
       if (t.nrows == 0) continue;
       const uint32_t buf = seq % kAccBufs, use = seq / kAccBufs;
       ++seq;
@@ -242,7 +250,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
       uint32_t kidx = 0, seq = 0;
       Ring<kPStages> rp;
       for (int it = first; it < total && !*abort_flag; it += step) {
-        const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
+        const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
         if (t.nrows == 0) continue;
         const long long wrow0 = (long long)t.expert * p.n_rows + t.col * kFeatures;
         if (kQuant) {
@@ -291,7 +299,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
         uint32_t kidx = 0;
         Ring<kBStages> rb;
         for (int it = first; it < total && !*abort_flag; it += step) {
-          const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
+          const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
           if (t.nrows == 0) continue;
           const int boxes = (t.nrows + kActBox - 1) / kActBox;
           bool ok = true;
@@ -331,7 +339,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
       for (int it = first; it < total; it += step) {
         // everybody has read the previous tile's table, and the threads agree whether to go on
         if (named_bar_or(1, kTsGatherThreads, !ok || *abort_flag != 0)) break;
-        const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
+        const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
         const int n8 = ((t.nrows + 15) & ~15) >> 3;         // runs of 8 rows
         sh.gather_token[pt] = pt < t.nrows ? p.gather_route[t.row0 + pt] / p.gather_top_k : -1;
         named_bar_sync(1, kTsGatherThreads);
@@ -371,7 +379,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     Ring<kPStages> rp;
     Ring<kAStages> ra;
     for (int it = first; it < total && !*abort_flag; it += step) {
-      const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
+      const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
       if (t.nrows == 0) continue;
       const uint32_t sbuf = seq & 1;
       bool ok = mbar_wait(&sh.sc_full[sbuf], (seq >> 1) & 1);
@@ -419,7 +427,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
     uint32_t seq = 0;
     for (int it = first; it < total && !*abort_flag; it += step) {
-      const TsTile t = ts_tile<kSplit>(p, it, n_col, nk);
+      const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
       if (t.nrows == 0) continue;
       const uint32_t buf = seq % kAccBufs, use = seq / kAccBufs;
       ++seq;
@@ -490,10 +498,10 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
   }
 }
 
-template <int ENC, int MODE>
+template <int ENC, int MODE, bool WIDE>
 int launch_ts(const GroupedGemmArgs& a, GroupedParams p, cudaStream_t stream) {
   using S = TsShape<ENC>;
-  auto kernel = grouped_ts_kernel<ENC, MODE>;
+  auto kernel = grouped_ts_kernel<ENC, MODE, WIDE>;
   constexpr size_t smem = ts_smem_bytes<ENC>();
   static_assert(smem <= 113 * 1024, "two CTAs share an SM");
   static thread_local int configured = -1;
@@ -533,6 +541,12 @@ int launch_ts(const GroupedGemmArgs& a, GroupedParams p, cudaStream_t stream) {
   return ERR_NONE;
 }
 
+template <int ENC>
+int launch_ts(const GroupedGemmArgs& a, const GroupedParams& p, cudaStream_t stream) {
+  if (a.tile_cap > NMAX) return a.mode == 0 ? launch_ts<ENC, 0, true>(a, p, stream) : launch_ts<ENC, 1, true>(a, p, stream);
+  return a.mode == 0 ? launch_ts<ENC, 0, false>(a, p, stream) : launch_ts<ENC, 1, false>(a, p, stream);
+}
+
 }  // namespace
 
 int launch_grouped_gemm_ts(const GroupedGemmArgs& a, cudaStream_t stream) {
@@ -544,10 +558,12 @@ int launch_grouped_gemm_ts(const GroupedGemmArgs& a, cudaStream_t stream) {
   p.k_splits = a.k_splits > 1 ? a.k_splits : 1; p.part = a.part; p.part_stride = a.total_rows * a.n_rows;
   p.out = a.out; p.out_stride = a.out_stride; p.route_weight = a.route_weight; p.permute_out = a.permute_out;
   p.status = a.status;
+  p.conditional = a.conditional; p.use_ts = a.use_ts;
+  if (a.conditional) p.choice = grouped_gemm_choice(a.enc, a.mode == 0 ? a.n_rows : a.k, a.mode == 0 ? a.k : a.n_rows);
   p.gather_route = a.gather_route; p.gather_top_k = a.gather_top_k; p.gather_src = static_cast<const __nv_bfloat16*>(a.act);
-  if (a.enc == ENC_Q4) return a.mode == 0 ? launch_ts<ENC_Q4, 0>(a, p, stream) : launch_ts<ENC_Q4, 1>(a, p, stream);
-  if (a.enc == ENC_Q8) return a.mode == 0 ? launch_ts<ENC_Q8, 0>(a, p, stream) : launch_ts<ENC_Q8, 1>(a, p, stream);
-  if (a.enc == ENC_BF16) return a.mode == 0 ? launch_ts<ENC_BF16, 0>(a, p, stream) : launch_ts<ENC_BF16, 1>(a, p, stream);
+  if (a.enc == ENC_Q4) return launch_ts<ENC_Q4>(a, p, stream);
+  if (a.enc == ENC_Q8) return launch_ts<ENC_Q8>(a, p, stream);
+  if (a.enc == ENC_BF16) return launch_ts<ENC_BF16>(a, p, stream);
   set_error("grouped: unknown encoding %d", a.enc);
   return ERR_BAD_ARGUMENT;
 }

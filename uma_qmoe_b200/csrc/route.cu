@@ -544,15 +544,29 @@ __device__ __forceinline__ int load_expert(const void* idx, int idx64, long long
 __device__ __forceinline__ void emit_offsets_and_tiles(const SortArgs& a, const int* count, int* start, int* tile_base,
                                                        bool write, int tid, int nthreads) {
   const int E = a.experts;
+  __shared__ int tile_cap;
   if (tid < 32) {                                // four experts per lane, scanned across the warp
     static_assert(kMaxSortExperts == 128, "four experts per lane");
-    int run[5], tiles[5];
+    int run[5], tiles[5], cap = a.tile_cap;
     run[0] = tiles[0] = 0;
+    if (a.use_ts) {                              // the kernel that suits these counts, and its table
+      int small = 0, wide = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int e = 4 * tid + i, c = e < E ? count[e] : 0;
+        small += (c + kTileCapMin - 1) / kTileCapMin;
+        wide += (c + kTileCapMax - 1) / kTileCapMax;
+      }
+      const bool ts = transposed_is_faster(a.choice, __reduce_add_sync(0xffffffffu, small), __reduce_add_sync(0xffffffffu, wide));
+      cap = ts ? kTileCapMin : kTileCapMax;
+      if (write && tid == 0) *a.use_ts = ts;
+    }
+    if (tid == 0) tile_cap = cap;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int e = 4 * tid + i, c = e < E ? count[e] : 0;
       run[i + 1] = run[i] + c;
-      tiles[i + 1] = tiles[i] + (c + a.tile_cap - 1) / a.tile_cap;
+      tiles[i + 1] = tiles[i] + (c + cap - 1) / cap;
     }
     int run_in = run[4], tiles_in = tiles[4];
 #pragma unroll
@@ -573,8 +587,8 @@ __device__ __forceinline__ void emit_offsets_and_tiles(const SortArgs& a, const 
     for (int e = tid; e < E; e += nthreads) {
       const int c = start[e + 1] - start[e];
       int t = tile_base[e];
-      for (int r = 0; r < c && t < a.max_tiles; r += a.tile_cap, ++t) {
-        a.tile_expert[t] = e; a.tile_row0[t] = start[e] + r; a.tile_rows[t] = min(a.tile_cap, c - r);
+      for (int r = 0; r < c && t < a.max_tiles; r += tile_cap, ++t) {
+        a.tile_expert[t] = e; a.tile_row0[t] = start[e] + r; a.tile_rows[t] = min(tile_cap, c - r);
       }
     }
     if (tid == 0) *a.num_tiles = min(tile_base[E], a.max_tiles);

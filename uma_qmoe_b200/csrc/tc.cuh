@@ -6,9 +6,29 @@
 #include <stdint.h>
 
 #include "common.cuh"
+#include "grouped.cuh"
 
 namespace umaq {
 namespace {
+
+// Whether a conditional launch runs (every warp of it calls this and gets the same answer).
+__device__ __forceinline__ bool launch_runs(const GroupedParams& p) {
+  if (p.conditional == 0) return true;
+  bool ts;
+  if (p.use_ts) {
+    ts = *p.use_ts != 0;
+  } else {
+    int small = 0, wide = 0;
+    const int n = *p.num_tiles;
+    for (int t = threadIdx.x & 31; t < n; t += 32) {
+      const int rows = p.tile_rows[t];
+      small += (rows + kTileCapMin - 1) / kTileCapMin;
+      wide += (rows + kTileCapMax - 1) / kTileCapMax;
+    }
+    ts = transposed_is_faster(p.choice, __reduce_add_sync(0xffffffffu, small), __reduce_add_sync(0xffffffffu, wide));
+  }
+  return ts == (p.conditional == 1);
+}
 
 // ---- tcgen05 / TMA wrappers ---------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
