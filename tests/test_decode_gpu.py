@@ -68,6 +68,23 @@ def test_device_packer_rounding_boundaries_and_layouts(enc, groups, offset):
 
 
 @pytest.mark.parametrize("enc", ["q4_group128", "q8_group128"])
+@pytest.mark.parametrize("experts,offset,pad", [(3, 1, 0), (3, 2, 0), (3, 0, 1), (2, 3, 6), (1, 1, 0)])
+def test_encode_experts_takes_any_offset_and_expert_stride(enc, experts, offset, pad):
+    """A fused gate/up tensor that starts off an 8-byte boundary, or whose experts are padded to an odd stride, packs to the
+    bytes of an aligned copy of it."""
+    from uma_qmoe_b200.host import encode_experts
+    hidden, inter = 256, 128
+    gen = torch.Generator(device=DEV).manual_seed(offset + 8 * pad)
+    def view(rows, k):
+        store = torch.randn(offset + experts * (rows * k + pad), device=DEV, generator=gen).to(torch.bfloat16)
+        return torch.as_strided(store, (experts, rows, k), (rows * k + pad, k, 1), offset)
+    gate_up, down = view(2 * inter, hidden), view(hidden, inter)
+    got = encode_experts(gate_up, down, enc)
+    want = encode_experts(gate_up.clone(memory_format=torch.contiguous_format), down.clone(memory_format=torch.contiguous_format), enc)
+    assert got.tensors and all(torch.equal(a, b) for a, b in zip(got.tensors, want.tensors))
+
+
+@pytest.mark.parametrize("enc", ["q4_group128", "q8_group128"])
 def test_device_packer_every_ratio_of_bf16_mantissas(enc):
     """Every BF16 mantissa against every BF16 maximum over the exponents whose codes are not all zero: every quotient a group
     of normal weights can have, exact ties between two codes among them."""

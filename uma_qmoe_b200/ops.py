@@ -390,11 +390,13 @@ def quantize_groups(values: torch.Tensor, encoding: str) -> tuple[torch.Tensor, 
 
 def quantize_chunks(values: torch.Tensor, encoding: str) -> tuple[torch.Tensor, torch.Tensor]:
     """:func:`quantize_groups` of a ``[chunks, rows, k]`` view whose chunks are each contiguous (one projection inside a
-    fused tensor) without a copy of it; any other layout is copied first."""
+    fused tensor) without a copy of it; any other layout, and chunks off the kernel's 8-byte boundaries, are copied first."""
     chunks, rows, k = values.shape
+    misaligned = values.data_ptr() % 8 or values.stride(0) % 4
     if (values.stride(2) != 1 or values.stride(1) != k or values.stride(0) < rows * k or rows * k % 128 or
-            not 1 <= chunks <= 65535):
-        return quantize_groups(values.contiguous().reshape(-1), encoding)
+            not 1 <= chunks <= 65535 or misaligned):
+        dense = values.contiguous()
+        return quantize_groups((dense.clone() if dense.data_ptr() % 8 else dense).reshape(-1), encoding)
     _require_cuda_bf16(values[0], "values")
     codes, scales, enc = _packed_like(values, encoding)
     code = _native.lib().umaq_quantize_chunks(values.data_ptr(), rows * k, chunks, values.stride(0), enc, codes.data_ptr(),
