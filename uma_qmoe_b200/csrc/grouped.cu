@@ -336,33 +336,29 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         for (int kc = 0; kc < nk && ok; ++kc, ++kidx) {
           const uint32_t s = kidx % kPStages, sb = kidx % kBStages, use = kidx / kBStages;
           ok = mbar_wait(&sh.p_full[s], (kidx / kPStages) & 1);
+          if (ok && use > 0) ok = mbar_wait(&sh.b_empty[sb], (use - 1) & 1);
           if (!ok) break;
           const float scale = sc[kc >> 1];
           const uint8_t* src = sP + s * kPackedBytes + r * kPackedRow;
-          // The arithmetic comes before the wait for a free stage: with two converted stages the round trip commit ->
-          // free -> stores -> full has to fit into the other stage's MMAs (1024 clocks), and the conversion would not.
-          uint32_t out[2][16];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {                 // the two 32-wide halves of the k chunk
-            if (ENC == ENC_Q4) {
-              convert_q4(*reinterpret_cast<const uint4*>(src + h * 16), scale, out[h]);
-            } else {
-              convert_q8(*reinterpret_cast<const uint4*>(src + h * 32), *reinterpret_cast<const uint4*>(src + h * 32 + 16),
-                         scale, out[h]);
-            }
-          }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sh.p_empty[s]);
-          if (use > 0) ok = mbar_wait(&sh.b_empty[sb], (use - 1) & 1);
-          if (!ok) break;
           uint8_t* dstrow = sB + sb * kBTile + r * 128;
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            *reinterpret_cast<uint4*>(dstrow + ((i ^ (r & 7)) << 4)) =
-                make_uint4(out[i >> 2][4 * (i & 3)], out[i >> 2][4 * (i & 3) + 1], out[i >> 2][4 * (i & 3) + 2], out[i >> 2][4 * (i & 3) + 3]);
+          for (int h = 0; h < 2; ++h) {                 // the two 32-wide halves of the k chunk
+            uint32_t out[16];
+            if (ENC == ENC_Q4) {
+              convert_q4(*reinterpret_cast<const uint4*>(src + h * 16), scale, out);
+            } else {
+              convert_q8(*reinterpret_cast<const uint4*>(src + h * 32), *reinterpret_cast<const uint4*>(src + h * 32 + 16),
+                         scale, out);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int chunk = (h * 4 + i) ^ (r & 7);
+              *reinterpret_cast<uint4*>(dstrow + chunk * 16) = make_uint4(out[4 * i], out[4 * i + 1], out[4 * i + 2], out[4 * i + 3]);
+            }
+          }
           fence_proxy_async();                         // generic-proxy writes -> visible to the tensor core
           __syncwarp();
-          if (lane == 0) mbar_arrive(&sh.b_full[sb]);
+          if (lane == 0) { mbar_arrive(&sh.b_full[sb]); mbar_arrive(&sh.p_empty[s]); }
         }
         if (ok) {
           __syncwarp();
