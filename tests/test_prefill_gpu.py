@@ -510,3 +510,30 @@ def test_concentrated_routes_take_the_one_cta_kernel(model, encoding, tokens):
         assert torch.equal(y, want)
         _, picked = _stagewise(layer, x, routes, weights, variant=0)
         assert torch.equal(picked, want)
+
+
+def test_a_failed_launch_is_reported_once():
+    """A launch that the runtime refuses (into the legacy stream while a blocking stream is being captured: an error on the host,
+    nothing runs) fails its own call and no later one."""
+    import ctypes as C
+    from uma_qmoe_b200 import _native, ops
+    runtime = C.CDLL("libcudart.so.12")
+    x = torch.zeros(1, 2048, dtype=torch.bfloat16, device=DEV)
+    idx = torch.zeros(1, 1, dtype=torch.int32, device=DEV)
+    pos, out = torch.zeros(1, dtype=torch.int32, device=DEV), torch.empty_like(x)
+    combine = lambda: _native.lib().umaq_combine_routes(x.data_ptr(), idx.data_ptr(), 0, pos.data_ptr(), 1, 1, 2048,
+                                                        out.data_ptr(), None)
+    torch.cuda.synchronize()
+    stream, graph = C.c_void_p(), C.c_void_p()
+    assert runtime.cudaStreamCreate(C.byref(stream)) == 0
+    try:
+        assert runtime.cudaStreamBeginCapture(stream, 2) == 0
+        refused = combine()
+        runtime.cudaStreamEndCapture(stream, C.byref(graph))         # invalidated by the refused launch
+    finally:
+        runtime.cudaStreamDestroy(stream)
+        runtime.cudaGetLastError()
+    assert refused != 0
+    ops.quantize_groups(x.reshape(-1), "q4_group128")
+    assert combine() == 0
+    torch.cuda.synchronize()

@@ -196,7 +196,9 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t s
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
   cfg.attrs = attr; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();     // reported here: the next launch's check must not find it again
+  return e;
 }
 
 #endif  // __CUDACC__
