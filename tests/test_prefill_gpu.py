@@ -537,3 +537,19 @@ def test_a_failed_launch_is_reported_once():
     ops.quantize_groups(x.reshape(-1), "q4_group128")
     assert combine() == 0
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("encoding", ["q4_group128", "q8_group128"])
+def test_wide_packed_linear_takes_the_one_cta_kernel_above_one_tile(encoding, tmp_path):
+    """A single matrix of many columns: two transposed tiles would take twice the waves of a one-CTA tile.  Narrow ones and
+    64 rows keep the transposed kernel; the bits are the same."""
+    from uma_qmoe_b200 import ops
+    from uma_qmoe_b200.ops import DeviceLayer
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    for out, rows, want in ((32768, 64, "grouped_ts_kernel"), (32768, 65, "grouped_gemm_kernel"), (2048, 65, "grouped_ts_kernel")):
+        codes, scales = ops.quantize_groups((torch.randn(out * 256, device=DEV, generator=gen) * 0.02).to(torch.bfloat16), encoding)
+        layer = DeviceLayer(encoding, 1, out, 256, codes, codes, codes, scales, scales, scales)
+        x = torch.randn(rows, 256, device=DEV, generator=gen).to(torch.bfloat16)
+        routes = ops.route_sort(torch.zeros(rows, 1, dtype=torch.int32, device=DEV), torch.ones(rows, 1, device=DEV), 1)
+        assert _kernels(lambda: ops.grouped_gemm(layer, 1, x, routes), tmp_path) == {want}
+        assert torch.equal(ops.grouped_gemm(layer, 1, x, routes), ops.grouped_gemm(layer, 1, x, routes, variant=1))

@@ -631,6 +631,13 @@ int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
       return ERR_BAD_ARGUMENT;
     }
     if (a.gather_route && (a.mode != 0 || a.gather_top_k < 1)) { set_error("grouped: rows are fetched by index only for the gate/up GEMM"); return ERR_BAD_ARGUMENT; }
+    // One quantised matrix (a packed linear layer): the count is known here and the waves of this GEMM alone decide.  65 to 88
+    // rows x [32768, 2048], us, one-CTA | transposed: Q4 27 | 33, Q8 35 | 45; x [8192, 2048]: 25 | 15, 32 | 19.
+    if (a.variant == 0 && a.num_experts == 1 && a.enc != ENC_BF16 && a.tile_cap > kTileCapMin) {
+      const TileChoice c = grouped_gemm_choice(a.enc, a.mode == 0 ? a.n_rows : 0, a.mode == 0 ? 0 : a.n_rows);
+      if (!transposed_is_faster(c, (int)((a.total_rows + kTileCapMin - 1) / kTileCapMin), (int)((a.total_rows + kTileCapMax - 1) / kTileCapMax)))
+        return launch_grouped_gemm_single(a, stream);
+    }
     if (!grouped_gemm_choice_on_device(a.enc, a.total_rows, a.num_experts, a.most, a.variant)) return launch_grouped_gemm_ts(a, stream);
     // The one-CTA kernel second: where it is not wanted its CTAs start under the end of the other one and leave with it.  It
     // may look at the counts before its programmatic wait: the transposed kernel, an ordinary launch, started after they
