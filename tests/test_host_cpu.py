@@ -65,6 +65,28 @@ def test_workspace_sizes_are_host_arithmetic():
     assert big >= 65536 * (2048 + 1024 + 2048) * 2
 
 
+@pytest.mark.parametrize("hidden", [512, 1024, 2048, 4096])
+def test_prefill_workspace_holds_the_shared_experts_parts_and_no_more(hidden):
+    """The parts of the shared expert's down GEMM on 148 SMs, restated: as many 256 x 256 (64 x 128 up to 448 rows, two per SM)
+    tiles as there are CTAs.  Their room is that of the largest need up to the token count, so a workspace serves smaller calls."""
+    lib = _native.lib()
+    if lib.umaq_sm_count() not in (0, 148):
+        pytest.skip("the figures are those of 148 SMs")
+    size = lambda tokens, shared: lib.umaq_prefill_workspace_bytes(tokens, 4, 60, hidden, 1408, shared)
+    up = lambda v: (v + 255) // 256 * 256
+    parts = lambda t: max(1, min(8, 296 // (-(-t // 64) * (hidden // 128)) if t <= 448 else 148 // (-(-t // 256) * (hidden // 256))))
+    need, before = 0, 0
+    for tokens in range(1, 9500):
+        if parts(tokens) > 1:
+            need = max(need, tokens * parts(tokens))
+        if tokens % 7 == 1 or tokens in (1366, 1536, 2304, 2305):
+            rest = up(4) + up(-(-tokens // 64) * 12) + up(tokens * 5632 * 2) + up(tokens * hidden * 2)
+            assert size(tokens, 5632) - size(tokens, 0) - rest == up(need * hidden * 4), tokens
+            assert size(tokens, 5632) >= before
+            before = size(tokens, 5632)
+    assert need * hidden * 4 <= 148 * 256 * 256 * 4
+
+
 def test_decode_launch_plans_fit_one_sm_together():
     """Host arithmetic of the decode launcher: for every shape of the benchmark configurations the two kernels'
     shared memory fits one SM side by side, every CTA's share fits its ring or the ring has at least two stages,

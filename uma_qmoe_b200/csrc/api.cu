@@ -2,7 +2,6 @@
 // utilities the kernels' launchers share.
 #include "../../include/umaq_b200.h"
 
-#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -258,11 +257,6 @@ struct PrefillPlan {
   size_t s_num_tiles, s_tiles, s_inter, s_out, s_part, total;
   int max_tiles, s_max_tiles;
 };
-// Room for the float32 parts of the shared expert's down GEMM: up to eight of them while the tokens are few (a tile of the
-// wide kernel is 256 x 256, so at most one part per SM has been cut from 2368 tokens on).
-size_t s_part_bytes(long long tokens, int hidden) {
-  return (size_t)std::min<long long>(tokens * kMaxDenseSplits, 8192) * hidden * 4;
-}
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 PrefillPlan prefill_plan(long long tokens, int top_k, int experts, int hidden, int inter, int shared_inter) {
   PrefillPlan p{};
@@ -289,8 +283,9 @@ PrefillPlan prefill_plan(long long tokens, int top_k, int experts, int hidden, i
     p.s_tiles = take((size_t)p.s_max_tiles * 12);
     p.s_inter = take((size_t)tokens * shared_inter * 2);
     p.s_out = take((size_t)tokens * hidden * 2);
-    // at most one part of 128 rows x 64 tokens for each of two CTAs of an SM: see grouped_gemm_dense_splits
-    p.s_part = take(s_part_bytes(tokens, hidden));
+    // the float32 parts of the down GEMM: at most a 256 x 256 tile for each SM (39 MB), and never less than a smaller call of
+    // the same workspace needs
+    p.s_part = take((size_t)grouped_gemm_dense_part_rows(tokens, hidden, shared_inter) * hidden * 4);
   }
   p.total = cur;
   return p;
@@ -406,7 +401,6 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
     d.out = reinterpret_cast<__nv_bfloat16*>(at(pl.s_out)); d.out_stride = H; d.route_weight = nullptr;
     d.k_splits = grouped_gemm_dense_splits(tokens, H, S);
     d.part = reinterpret_cast<float*>(at(pl.s_part));
-    if ((size_t)d.k_splits * tokens * H * 4 > s_part_bytes(tokens, H)) d.k_splits = 1;
     rc = launch_grouped_gemm(d, stream);
     if (rc) return rc;
     if (d.k_splits > 1) { shared_part = d.part; shared_parts = d.k_splits; }

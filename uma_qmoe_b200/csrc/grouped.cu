@@ -586,13 +586,29 @@ static bool takes_ts_kernel(int enc, long long rows, int experts, int variant, i
 // The shared expert's down GEMM has few tiles and a long contraction (Qwen: 2048 rows, k 5632): without parts it runs on 16
 // CTAs at up to 64 tokens and on 48 at 1531.  Parts until the CTAs that fit the device have a tile each.
 // Down GEMM plus the combine that adds the parts, Qwen shape, us, before | now: 24 tokens 52 | 15, 128: 54 | 17, 1531: 76 | 62.
-int grouped_gemm_dense_splits(long long rows, int n_rows, int k) {
+static int dense_splits(long long rows, int n_rows, int k, int sms) {
   const bool ts = takes_ts_kernel(ENC_BF16, rows, 1, 0, 1);
   if (!ts && rows >= kPairMinRows) return 1;
   const long long tiles = ts ? (rows + kTileCapMin - 1) / kTileCapMin * (n_rows / 128) : (rows + kTileCapMax - 1) / kTileCapMax * (n_rows / BN);
-  const long long slots = (long long)sm_count() * (ts ? 2 : 1);
+  const long long slots = (long long)sms * (ts ? 2 : 1);
   const long long want = tiles > 0 ? slots / tiles : 1;
   return (int)std::max(1ll, std::min({want, (long long)kMaxDenseSplits, (long long)(k / 512)}));
+}
+static int dense_sms() {
+  const int sms = sm_count();
+  return sms > 0 ? sms : 148;                               // asked for a workspace's size where there is no device
+}
+int grouped_gemm_dense_splits(long long rows, int n_rows, int k) { return dense_splits(rows, n_rows, k, dense_sms()); }
+// The most rows x parts of any call of up to `rows` rows: the parts change with the rows' tiles only, and end.
+long long grouped_gemm_dense_part_rows(long long rows, int n_rows, int k) {
+  const int sms = dense_sms();
+  long long most = 0;
+  for (long long r = kTileCapMin;; r = r < kTsMaxRowsDense[1] ? r + kTileCapMin : (r / kTileCapMax + 1) * kTileCapMax) {   // full tiles
+    const long long at = std::min(r, rows);
+    const int splits = dense_splits(at, n_rows, k, sms);
+    if (splits > 1) most = std::max(most, at * splits);
+    if (at == rows || (splits == 1 && at > kTsMaxRowsDense[1])) return most;
+  }
 }
 int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant) {
   return takes_ts_kernel(enc, rows, num_experts, variant, 0) ? kTileCapMin : kTileCapMax;

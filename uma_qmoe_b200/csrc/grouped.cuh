@@ -103,6 +103,8 @@ bool grouped_gemm_choice_on_device(int enc, long long rows, int num_experts, lon
 TileChoice grouped_gemm_choice(int enc, int inter, int hidden);
 // Parts the contraction of a dense BF16 down GEMM (the shared expert's) is cut into
 int grouped_gemm_dense_splits(long long rows, int n_rows, int k);
+// ... and the room they need, in rows of n_rows float32 sums, for every call of up to `rows` rows (0: never more than one part)
+long long grouped_gemm_dense_part_rows(long long rows, int n_rows, int k);
 constexpr int kMaxDenseSplits = 8;
 
 // ---- routing (route.cu) ---------------------------------------------------------------------------
