@@ -85,6 +85,39 @@ def test_encode_experts_takes_any_offset_and_expert_stride(enc, experts, offset,
 
 
 @pytest.mark.parametrize("enc", ["q4_group128", "q8_group128"])
+def test_device_packer_values_that_divide(enc):
+    """Groups the quantiser divides for: an infinity, a NaN (fmax passes over it, its code is -qmax), maxima near the largest
+    BF16 value, scales around 2^-100 and with the largest mantissas, next to ordinary groups in the other half of their warp."""
+    ops, qmax = _ops(), 7 if enc == "q4_group128" else 127
+    rng = np.random.default_rng(3)
+    g = rng.standard_normal((64, 128)).astype(np.float32)
+    g[1, 5], g[4, 0], g[4, 127], g[7, 9], g[8, :] = np.inf, -np.inf, np.inf, np.nan, np.nan
+    g[10, 3], g[10, 4], g[13, 64] = np.nan, np.inf, -np.nan
+    g[16] *= np.float32(3.3e38 / 4)
+    g[19, 77] = np.float32(3.3895e38)                                       # the largest finite BF16 value
+    for n, e in enumerate(range(-106, -94)):
+        g[20 + 2 * n] *= np.float32(2.0 ** e)
+    top = (1 + np.arange(128, dtype=np.float32) / 128) * 4                  # of every mantissa of the maximum, those with these scales
+    for n in range(16):
+        g[46 + n] = np.clip(g[46 + n], -3.9, 3.9)
+        g[46 + n, n] = top[np.argsort((top / np.float32(qmax)).view(np.uint32) & 0x7fffff)[-1 - n]]
+    v = torch.from_numpy(g).to(torch.bfloat16)
+    f = v.float().numpy()
+    with np.errstate(all="ignore"):
+        am = np.where(np.isnan(f), np.float32(0), np.abs(f)).max(axis=1)
+        scale = am / np.float32(qmax)
+        scale[scale == 0] = 1
+        q = np.rint(f / scale[:, None])
+    q = np.clip(np.where(np.isnan(q), -qmax, q), -qmax, qmax).astype(np.int8)
+    codes, scales = ops.quantize_groups(v.reshape(-1).to(DEV), enc)
+    want = q.reshape(-1).view(np.uint8)
+    if enc == "q4_group128":
+        want = (want[0::2] & 15) | (want[1::2] << 4)
+    assert np.array_equal(scales.cpu().numpy(), scale)
+    assert np.array_equal(codes.cpu().numpy().view(np.uint8), want)
+
+
+@pytest.mark.parametrize("enc", ["q4_group128", "q8_group128"])
 def test_device_packer_every_ratio_of_bf16_mantissas(enc):
     """Every BF16 mantissa against every BF16 maximum over the exponents whose codes are not all zero: every quotient a group
     of normal weights can have, exact ties between two codes among them."""

@@ -389,6 +389,31 @@ def test_few_routes_per_expert_at_tile_edges(model, encoding, counts):
     assert (got - want).abs().max() <= 2.0 ** -7 * want.abs().max()
 
 
+@pytest.mark.parametrize("encoding,tokens", [("q4_group128", 520), ("q4_group128", 704), ("q4_group128", 705),
+                                             ("q8_group128", 608), ("q8_group128", 609)])
+def test_top_8_prompts_around_the_line_match_float64(encoding, tokens):
+    """Prompts whose routes are sorted by several CTAs into a table of 64-route tiles (and just above the line of 256-route
+    ones), with a skewed choice of experts, absent routes and real weights.  Against :func:`_reference_layer` per route and the
+    ordered BF16 sum: 16 roundings per value, each off by one at the rare sum on a boundary; a misplaced row is off by itself."""
+    from uma_qmoe_b200.stack import random_layer
+    layer = random_layer(syn.OLMOE, encoding, 9, torch.device(DEV))
+    gen = torch.Generator(device=DEV).manual_seed(tokens)
+    popularity = 1.0 / torch.arange(1, 65, device=DEV, dtype=torch.float32) ** 0.5
+    idx = torch.multinomial(popularity.expand(tokens, 64), 8, generator=gen)
+    idx[torch.rand(tokens, 8, device=DEV, generator=gen) < 0.02] = -1
+    x = torch.randn(tokens, 2048, device=DEV, generator=gen).to(torch.bfloat16)
+    w = torch.rand(tokens, 8, device=DEV, generator=gen) + 0.1
+    got = _run_prefill(layer, x, idx, w).float()
+    per_route = _reference_layer(layer, x.repeat_interleave(8, 0), idx.reshape(-1), w.reshape(-1)).reshape(tokens, 8, 2048)
+    order = torch.where(idx < 0, 64, idx).argsort(1)                        # ascending expert; absent routes are zero rows
+    want = torch.zeros(tokens, 2048, device=DEV, dtype=torch.bfloat16)
+    for slot in range(8):
+        want = want + per_route[torch.arange(tokens, device=DEV), order[:, slot]]
+    want = want.cpu().float()
+    assert (got - want).norm() <= 2.0 ** -7 * want.norm()
+    assert (got - want).abs().max() <= 2.0 ** -5 * want.abs().max()
+
+
 def test_few_routes_kernel_takes_tables_of_wider_tiles():
     """The exported stage calls hand the transposed kernel tables of up to 256 routes per entry: it cuts them itself, and a
     gathered copy of the rows gives the bits that rows fetched by index give."""
