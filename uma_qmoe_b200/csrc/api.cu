@@ -371,13 +371,20 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
     if (rc) return rc;
     g.act = xs;
   }
-  rc = launch_grouped_gemm(g, stream);
-  if (rc) return rc;
-  g.mode = 1; g.n_rows = H; g.k = I; g.act = g.out; g.gather_route = nullptr;
-  g.w0 = layer->down; g.s0 = layer->down_scales; g.w1 = nullptr; g.s1 = nullptr;
-  g.out = reinterpret_cast<__nv_bfloat16*>(at(pl.yw)); g.out_stride = H; g.route_weight = sa.sorted_weight; g.permute_out = 0;
-  rc = launch_grouped_gemm(g, stream);
-  if (rc) return rc;
+  GroupedGemmArgs down = g;
+  down.mode = 1; down.n_rows = H; down.k = I; down.act = g.out; down.gather_route = nullptr;
+  down.w0 = layer->down; down.s0 = layer->down_scales; down.w1 = nullptr; down.s1 = nullptr;
+  down.out = reinterpret_cast<__nv_bfloat16*>(at(pl.yw)); down.out_stride = H; down.route_weight = sa.sorted_weight; down.permute_out = 0;
+  // Where the sort picks the kernel: both GEMMs on transposed tiles, then both on one-CTA tiles.  The pair that is not wanted
+  // returns, and in this order it stands between no two kernels that work.
+  for (int conditional = sa.use_ts ? 1 : 0; conditional <= (sa.use_ts ? 2 : 0); ++conditional) {
+    g.conditional = down.conditional = conditional;
+    if (conditional) g.tile_cap = down.tile_cap = conditional == 1 ? kTileCapMin : kTileCapMax;
+    rc = launch_grouped_gemm(g, stream);
+    if (rc) return rc;
+    rc = launch_grouped_gemm(down, stream);
+    if (rc) return rc;
+  }
 
   const __nv_bfloat16* shared_out = nullptr;
   const float* shared_part = nullptr;

@@ -616,7 +616,7 @@ int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant)
 // The lines above suppose that the routes spread over the experts.  Where they concentrate on a few, the transposed kernel
 // converts an expert's weights once per 64 routes and the one-CTA kernel once per 256, and the one-CTA kernel wins: 512 tokens
 // on 8 of 64 experts, whole operator, us, one-CTA | transposed: OLMoE Q4 65 | 100, Q8 77 | 132, BF16 67 | 109.  The counts
-// are on the device, so both kernels are launched and the one that is not wanted returns.  That costs a call 2.5 us where the
+// are on the device, so both kernels are launched and the one that is not wanted returns.  That costs a layer 3 us where the
 // transposed kernel runs and 8 us where the other one does.  What decides is the number of waves (gate/up counted twice; half
 // ones where two CTAs share an SM): with these costs, over 400 routings (tokens 80 to 1320, all experts down to top-k of
 // them, the skewed router), the transposed kernel is the better one below 2 (Q4), 9/5 (Q8) and 7/4 (BF16) times the other's
@@ -640,13 +640,15 @@ int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
     if (a.gather_route) { set_error("grouped: the CTA-pair kernel takes gathered activation rows"); return ERR_BAD_ARGUMENT; }
     return launch_grouped_gemm_pair(a, stream);
   }
-  if (takes_ts_kernel(a.enc, a.total_rows, a.num_experts, a.variant, a.mode)) {
+  if (a.conditional == 2) return launch_grouped_gemm_single(a, stream);
+  if (a.conditional == 1 || takes_ts_kernel(a.enc, a.total_rows, a.num_experts, a.variant, a.mode)) {
     if (a.k % 128 || a.n_rows % (a.mode == 0 ? BN / 2 : BN) || a.total_rows <= 0 || a.max_tiles <= 0 ||
         (a.enc != ENC_BF16 && a.k > kMaxGroups * 128)) {
       set_error("grouped: unsupported shape (k %d, rows per expert %d)", a.k, a.n_rows);
       return ERR_BAD_ARGUMENT;
     }
     if (a.gather_route && (a.mode != 0 || a.gather_top_k < 1)) { set_error("grouped: rows are fetched by index only for the gate/up GEMM"); return ERR_BAD_ARGUMENT; }
+    if (a.conditional == 1) return launch_grouped_gemm_ts(a, stream);
     // One quantised matrix (a packed linear layer): the count is known here and the waves of this GEMM alone decide.  65 to 88
     // rows x [32768, 2048], us, one-CTA | transposed: Q4 27 | 33, Q8 35 | 45; x [8192, 2048]: 25 | 15, 32 | 19.
     if (a.variant == 0 && a.num_experts == 1 && a.enc != ENC_BF16 && a.tile_cap > kTileCapMin) {
@@ -660,7 +662,6 @@ int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
     // were written.
     GroupedGemmArgs b = a;
     b.conditional = 1;
-    if (a.use_ts) b.tile_cap = kTileCapMin;
     const int rc = launch_grouped_gemm_ts(b, stream);
     if (rc) return rc;
     b.conditional = 2;

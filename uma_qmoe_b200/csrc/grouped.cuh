@@ -36,6 +36,7 @@ struct GroupedParams {
   const int* tile_rows;       // valid rows (<= 128)
   int max_tiles;
   int subs;                   // grouped_ts.cu: parts a table entry may be cut into
+  int part_major;             // grouped_ts.cu: order of the parts
   int k_splits;               // BF16 down GEMM: the contraction is cut into this many parts, each a tile of its own
   float* part;                // k_splits > 1: float32 sums [k_splits, total rows, n_rows] instead of `out`
   long long part_stride;      // elements of one split
@@ -73,7 +74,7 @@ struct GroupedGemmArgs {
   int tile_cap;               // most routes of a table entry
   long long most;             // most routes an expert can have (0: total_rows)
   const int* use_ts;          // device word of the sort whose table was cut for either kernel (null: decided from the table)
-  int conditional;            // set by launch_grouped_gemm: see GroupedParams
+  int conditional;            // 1: transposed tiles, 2: one-CTA tiles, if the device picks them (see GroupedParams); 0: not conditional
   int k_splits;               // > 1 (BF16 down GEMM without routing weights): partial sums into `part`, `out` is not written
   float* part;                // [k_splits, total_rows, n_rows] float32
   __nv_bfloat16* out; long long out_stride;

@@ -138,11 +138,16 @@ __device__ __forceinline__ TsTile ts_tile(const GroupedParams& p, int it, int n_
   }
   const int m = it / n_col;
   t.col = it - m * n_col;
-  // every entry's first part, then every entry's second one: the parts that exist spread evenly over the CTAs
+  // Many experts: every entry's first part, then every entry's second one.  A dense matrix, whose entries are full: entry by
+  // entry.  Either way the parts that exist come one after another and spread evenly over the CTAs.
   int sub = 0, tm = m;
   if (WIDE) {
-    const int entries = *p.num_tiles;
-    sub = m / entries; tm = m - sub * entries;
+    if (p.part_major) {
+      const int entries = *p.num_tiles;
+      sub = m / entries; tm = m - sub * entries;
+    } else {
+      tm = m / p.subs; sub = m - tm * p.subs;
+    }
   }
   t.expert = p.tile_expert[tm]; t.row0 = p.tile_row0[tm]; t.nrows = p.tile_rows[tm];
   if (WIDE) {
@@ -532,6 +537,7 @@ int launch_ts(const GroupedGemmArgs& a, GroupedParams p, cudaStream_t stream) {
                 kAtomK, kActBox, CU_TENSOR_MAP_SWIZZLE_128B))
     return ERR_LAUNCH;
   p.subs = (a.tile_cap + NMAX - 1) / NMAX;
+  p.part_major = a.num_experts > 1;
   // An ordinary launch, not a chained one: CTAs that become resident one by one as their predecessor's leave are paired on
   // the SMs by chance, and CTAs with a tile more than the others then meet on one SM (OLMoE Q8, 96 tokens: 127 -> 140 us a
   // layer).  Launched on an empty device, CTA b and b + SMs share an SM and the longer ones spread.
