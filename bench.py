@@ -318,7 +318,7 @@ def native_arm(args) -> None:
                 w, idx = stack.route(l, x)
                 x = rms_renorm(torch.ops.uma_qmoe.moe_forward(x, idx, w, l, handle, True))
             return x
-        launches_per_step = LAYERS * 7          # router, sort (2 kernels), gather, 2 grouped GEMMs, combine
+        launches_per_step = LAYERS * 6          # router, sort (2 kernels, the k permutation in the first), 2 grouped GEMMs, combine
     else:
         from uma_qmoe_b200.ep import CudaKernels, ExpertParallelMoE, PeerExchange
         dist = torch.distributed
@@ -494,7 +494,7 @@ def native_arm(args) -> None:
         line.update(kernel_objects)
         line.update(decode_objects)
         # the single-kernel legs (3 x 13 cold launches, ten kernels x 7 graph passes x 8 launches, the 512-token leg:
-        # 10 passes x 8 calls x 7 kernels) and the decode legs
+        # 10 passes x 8 calls x 7 launches: router, sort, both GEMMs on either kernel, combine) and the decode legs
         line["gpu_launches"] += 39 + 10 * 7 * 8 + 10 * 8 * 7 + decode_launches
         line["cpu_baseline"] = cpu_baseline_subprocess()
     if world > 1:
@@ -661,7 +661,7 @@ def prefill_kernel_times(stack, x, shape, dev) -> dict:
     ws = ops.prefill_workspace(layer, x.shape[0], shape.top_k, None, dev)
     phases = [("router", lambda: stack.route(0, x)),
               ("route_sort", lambda: ops.route_sort(idx, w, shape.experts)),
-              ("permute_k", lambda: ops.gather_rows(x, None, 1, permute=True)),
+              ("permute_k_inside_the_sort_launch", lambda: ops.gather_rows(x, None, 1, permute=True)),
               ("gemm_gate_up", lambda: ops.grouped_gemm_by_index(layer, x_perm, routes, shape.top_k, permute_out=True, out=inter)),
               ("gather_rows_not_on_the_path", lambda: ops.gather_rows(x, routes.sorted_route, shape.top_k, permute=True)),
               ("gemm_gate_up_on_gathered_rows", lambda: ops.grouped_gemm(layer, 0, xs, routes, permute_out=True, out=inter)),

@@ -30,10 +30,10 @@ struct GroupedParams {
   int n_rows;                 // weight rows per expert in this projection
   const float* scales0;       // [E * n_rows, k/128] (gate or down)
   const float* scales1;       // up (mode 0)
-  const int* num_tiles;       // device: number of valid 128-route tiles
+  const int* num_tiles;       // device: entries of the tile table, of up to 64 or 256 routes (SortArgs::tile_cap)
   const int* tile_expert;     // device [max_tiles]
   const int* tile_row0;       // first sorted route row of the tile
-  const int* tile_rows;       // valid rows (<= 128)
+  const int* tile_rows;       // valid rows
   int max_tiles;
   int subs;                   // grouped_ts.cu: parts a table entry may be cut into
   int part_major;             // grouped_ts.cu: order of the parts
@@ -128,7 +128,7 @@ struct SortArgs {
   int* sorted_route;               // [routes] token * top_k + slot, stable by expert
   int* route_pos;                  // [routes] inverse permutation
   float* sorted_weight;            // [routes]
-  int* num_tiles; int* tile_expert; int* tile_row0; int* tile_rows;   // 128-route tiles
+  int* num_tiles; int* tile_expert; int* tile_row0; int* tile_rows;   // tiles of up to tile_cap routes
   int max_tiles;
   int tile_cap;                    // routes per tile, unless use_ts is given
   int* use_ts; TileChoice choice;  // optional: the sort picks the kernel, cuts the table for it and writes 1 (transposed) or 0
