@@ -455,6 +455,28 @@ def test_shared_expert_in_parts_of_its_contraction(tokens):
     assert (got - want).abs().max() <= 2.0 ** -6 * want.abs().max()
 
 
+@pytest.mark.parametrize("hidden,encoding,tokens", [(1024, "q4_group128", 1400), (1024, "q4_group128", 449), (512, "q8_group128", 2100),
+                                                    (4096, "bf16_le", 5), (4096, "bf16_le", 300)])
+def test_shared_expert_in_parts_at_other_hidden_sizes(hidden, encoding, tokens):
+    """As above where the parts' room is another: six parts of 1400 tokens at hidden 1024, eight of 2100 at 512, eight of 5 and
+    one of 300 at 4096.  The bounds are those of :func:`test_shared_expert_in_parts_of_its_contraction`: the same roundings."""
+    from dataclasses import replace
+    from uma_qmoe_b200.stack import random_layer, random_shared_expert
+    dev, shape = torch.device(DEV), replace(syn.QWEN, hidden=hidden, experts=6)
+    layer, sh = random_layer(shape, encoding, 7, dev), random_shared_expert(shape, 7, dev)
+    gen = torch.Generator(device=DEV).manual_seed(tokens)
+    x = torch.randn(tokens, hidden, device=DEV, generator=gen).to(torch.bfloat16)
+    idx = torch.arange(tokens * 4, device=DEV).reshape(tokens, 4) % 6
+    got = _run_prefill(layer, x, idx, torch.zeros(tokens, 4, device=DEV), sh).float()
+    xd = x.double()
+    inter = (torch.nn.functional.silu(xd @ sh.gate.double().T) * (xd @ sh.up.double().T)).to(torch.bfloat16)
+    y = (inter.double() @ sh.down.double().T).to(torch.bfloat16)
+    gate = torch.sigmoid((xd @ sh.gate_vec.reshape(-1).double()).to(torch.bfloat16).float()).to(torch.bfloat16)
+    want = (gate[:, None] * y).cpu().float()
+    assert (got - want).norm() <= 2.0 ** -7 * want.norm()
+    assert (got - want).abs().max() <= 2.0 ** -6 * want.abs().max()
+
+
 def _kernels(call, tmp_path):
     """Which grouped GEMM kernels a call launches, from the nodes of a graph it is captured into."""
     stream = torch.cuda.Stream()
