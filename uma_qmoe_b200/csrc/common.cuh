@@ -106,6 +106,12 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// The barrier receives one arrival when all cp.async copies this thread issued so far have landed
+// (the arrival is part of the barrier's initial count).
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // ---- programmatic stream serialisation ---------------------------------------
 // A kernel launched with launch_chained may become resident while the kernel before it on the stream still runs.  Its
 // threads call pdl_wait before they read or write global memory: it returns when that kernel has finished and its writes

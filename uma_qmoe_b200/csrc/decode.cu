@@ -88,11 +88,6 @@ __device__ __forceinline__ void red_release_add_u32(unsigned* p, unsigned v) {
 __device__ __forceinline__ void cp_async8(void* dst_smem, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
 }
-// The barrier receives one arrival when all cp.async copies this thread issued so far have landed
-// (the arrival is part of the barrier's initial count).
-__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 // try_wait with a suspend-time hint: the warp sleeps in hardware until the phase completes (or the hint
 // runs out) instead of re-issuing the test -- waiting warps must not take issue slots and shared-memory

@@ -43,7 +43,6 @@ constexpr int kGemmThreads = (3 + kConvertWarps) * 32;   // + activation TMA, MM
 constexpr int kWeightWarp = 2 + kConvertWarps;
 constexpr int kGatherWarps = 4;       // launched only when the kernel fetches its activation rows by index
 constexpr int kGatherThreads = kGatherWarps * 32;
-constexpr int kGatherAhead = 2;       // a gather thread hands a stage over two steps after issuing it (< kInStages)
 constexpr int kHalves = 2;            // M = 128 accumulators per tile
 constexpr int kTmemCols = BN * kHalves;   // 512: the whole tensor memory of the SM
 constexpr int kMaxGroups = 16;        // quantised K <= 2048
@@ -159,17 +158,21 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
   if (warp == 0) {
     // ===================== TMA producer: activation tiles (and BF16 weight tiles) ==================
-    if (lane == 0 && !(gather && ENC != ENC_BF16)) {
+    // The whole warp waits (a lone lane's wait takes twice as long and slows the others'), one lane issues.
+    if (!(gather && ENC != ENC_BF16)) {
       uint32_t kidx = 0;
       int inflight_from = 0;
-      for (int it = first; it < total && !*abort_flag; it += step) {
+      for (int it = first; it < total; it += step) {
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
         const TileInfo t = tile_of(it);
         const bool two = t.nrows > BM;
         const long long wrow0 = weight_row(t);
         bool ok = true;
         for (int kc = t.k0; kc < t.k1; ++kc, ++kidx) {
           const uint32_t s = kidx % kInStages, use = kidx / kInStages;
-          if (use > 0 && !mbar_wait(&sh.in_empty[s], (use - 1) & 1)) { ok = false; break; }
+          ok = __all_sync(0xffffffffu, use == 0 || mbar_wait(&sh.in_empty[s], (use - 1) & 1));
+          if (!ok) break;
+          if (lane != 0) continue;                       // converges again at the next wait
           const uint32_t bytes = (gather ? 0 : (two ? kATile : kAHalf)) + (ENC == ENC_BF16 ? kBTile : 0);
           mbar_expect_tx(&sh.in_full[s], bytes);
           if (!gather) {
@@ -186,7 +189,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
           }
         }
-        if (!ok) { fail(); break; }
+        if (!ok) { if (lane == 0) fail(); break; }
       }
       // after an abort nobody consumes: wait (bounded) for the copies still in flight
       if (*abort_flag) {
@@ -196,23 +199,29 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
   } else if (warp == kWeightWarp) {
     // ===================== TMA producer: scales and packed weight rows, on their own deeper ring ====
-    if (lane == 0 && ENC != ENC_BF16) {
+    if (ENC != ENC_BF16) {
       uint32_t kidx = 0;
       int seq = 0;
-      for (int it = first; it < total && !*abort_flag; it += step, ++seq) {
+      for (int it = first; it < total; it += step, ++seq) {
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
         const TileInfo t = tile_of(it);
         const long long wrow0 = weight_row(t);
         const int sb = seq & 1;
-        if (seq >= 2 && !mbar_wait(&sh.sc_empty[sb], ((seq >> 1) - 1) & 1)) { fail(); break; }
-        float* dst_sc = sScales + sb * BN * kMaxGroups;
-        const uint32_t half_bytes = (uint32_t)(MODE == 0 ? BN / 2 : BN) * groups * 4;
-        mbar_expect_tx(&sh.sc_full[sb], MODE == 0 ? 2 * half_bytes : half_bytes);
-        bulk_g2s(dst_sc, p.scales0 + wrow0 * groups, half_bytes, &sh.sc_full[sb]);
-        if (MODE == 0) bulk_g2s(dst_sc + (BN / 2) * groups, p.scales1 + wrow0 * groups, half_bytes, &sh.sc_full[sb]);
+        if (!__all_sync(0xffffffffu, seq < 2 || mbar_wait(&sh.sc_empty[sb], ((seq >> 1) - 1) & 1))) { if (lane == 0) fail(); break; }
+        if (lane == 0) {
+          float* dst_sc = sScales + sb * BN * kMaxGroups;
+          const uint32_t half_bytes = (uint32_t)(MODE == 0 ? BN / 2 : BN) * groups * 4;
+          mbar_expect_tx(&sh.sc_full[sb], MODE == 0 ? 2 * half_bytes : half_bytes);
+          bulk_g2s(dst_sc, p.scales0 + wrow0 * groups, half_bytes, &sh.sc_full[sb]);
+          if (MODE == 0) bulk_g2s(dst_sc + (BN / 2) * groups, p.scales1 + wrow0 * groups, half_bytes, &sh.sc_full[sb]);
+        }
+        __syncwarp();
         bool ok = true;
         for (int kc = 0; kc < nk; ++kc, ++kidx) {
           const uint32_t s = kidx % kPStages, use = kidx / kPStages;
-          if (use > 0 && !mbar_wait(&sh.p_empty[s], (use - 1) & 1)) { ok = false; break; }
+          ok = __all_sync(0xffffffffu, use == 0 || mbar_wait(&sh.p_empty[s], (use - 1) & 1));
+          if (!ok) break;
+          if (lane != 0) continue;
           mbar_expect_tx(&sh.p_full[s], kPackedBytes);
           uint8_t* dst = sP + s * kPackedBytes;
           if (MODE == 0) {
@@ -222,7 +231,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             tma_load_2d(dst, &map_b0, kc * kPackedRow, (int)wrow0, &sh.p_full[s]);
           }
         }
-        if (!ok) { fail(); break; }
+        if (!ok) { if (lane == 0) fail(); break; }
       }
       if (*abort_flag) {
         for (int sb = 0; sb < 2; ++sb) mbar_wait(&sh.sc_full[sb], 0);   // bounded; a barrier never armed just times out
@@ -236,18 +245,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // ((c ^ (r & 7)) << 4), the 128-byte swizzle the MMA descriptors expect.  Thread j copies chunk j & 7 of
     // rows (j >> 3) + 16 i: eight neighbouring lanes read one row's 128 contiguous bytes, so every copy
     // instruction of a warp covers four whole lines.  Rows past the tile's end are zero-filled.  cp.async writes
-    // go through the generic proxy: a thread waits for its own copies of a stage (the younger stages stay in
-    // flight), fences them towards the async proxy and arrives.
+    // go through the generic proxy: the stage's barrier counts a thread's copies when they have landed, and the issuer
+    // fences them towards the async proxy before its MMAs.
     const int pt = tid - (kWeightWarp + 1) * 32;          // 0 .. 127
     const int c = pt & 7, rbase = pt >> 3;                // rows rbase, rbase + 16, ...: all have r & 7 == rbase & 7
     const uint32_t dst_off = (uint32_t)rbase * 128 + (uint32_t)((c ^ (rbase & 7)) << 4);
-    uint32_t kidx = 0, published = 0;
+    uint32_t kidx = 0;
     bool ok = true;
-    auto publish = [&]() {
-      fence_proxy_async();
-      mbar_arrive(&sh.in_full[published % kInStages]);
-      ++published;
-    };
     for (int it = first; it < total; it += step) {
       // Everybody has read the previous tile's table; and the threads agree whether to go on (a thread that gave up
       // on a wait, or saw the abort flag, must not leave the others waiting at this barrier).
@@ -263,11 +267,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       for (int i = 0; i < 2 * BM / 16; ++i) tok[i] = sh.gather_token[rbase + 16 * i];
       const uint8_t* base = reinterpret_cast<const uint8_t*>(p.gather_src) + c * 16;
       for (int kc = 0; kc < nk; ++kc, ++kidx) {
-        // first hand over the stage issued two steps ago (its copies have had two steps to land), so that the
-        // MMA issuer never waits for this thread's wait on a free slot below
-        if (kidx >= (uint32_t)kGatherAhead) { cp_async_wait<kGatherAhead - 1>(); publish(); }
         const uint32_t s = kidx % kInStages, use = kidx / kInStages;
-        if (use > 0 && !mbar_wait(&sh.in_empty[s], (use - 1) & 1)) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, use == 0 || mbar_wait(&sh.in_empty[s], (use - 1) & 1))) { ok = false; break; }
         uint8_t* dst = sA + s * kATile + dst_off;
         const uint8_t* col = base + kc * 128;
 #pragma unroll
@@ -278,44 +279,45 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           for (int i = BM / 16; i < 2 * BM / 16; ++i)
             cp_async16(dst + i * 2048, col + (size_t)(tok[i] < 0 ? 0 : tok[i]) * K * 2, tok[i] >= 0);
         }
-        cp_async_commit();
+        cp_async_arrive(&sh.in_full[s]);
       }
     }
     if (!ok && lane == 0) fail();
+    cp_async_commit();
     cp_async_wait<0>();                                  // also on the abort path: nothing of this thread stays in flight
-    if (ok && !*abort_flag)
-      while (published < kidx) publish();
   } else if (warp == 1) {
-    // ===================== MMA issuer ============================================================
-    if (lane == 0) {
+    // ===================== MMA issuer: the warp stays converged, one elected lane issues ==========
+    {
       uint32_t kidx = 0;
       int seq = 0;
-      for (int it = first; it < total && !*abort_flag; it += step, ++seq) {
+      for (int it = first; it < total; it += step, ++seq) {
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
         const TileInfo t = tile_of(it);
         const bool two = t.nrows > BM;
-        if (seq >= 1 && !mbar_wait(&sh.acc_empty, (seq - 1) & 1)) { fail(); break; }
-        tc_fence_after();
-        bool ok = true;
+        bool ok = seq == 0 || mbar_wait(&sh.acc_empty, (seq - 1) & 1);
         for (int kc = t.k0; kc < t.k1; ++kc, ++kidx) {
           const uint32_t s = kidx % kInStages;
           const uint32_t sb = ENC == ENC_BF16 ? s : kidx % kBStages;
-          ok = mbar_wait(&sh.in_full[s], (kidx / kInStages) & 1);
-          if (ok && ENC != ENC_BF16) ok = mbar_wait(&sh.b_full[sb], (kidx / kBStages) & 1);
-          if (!ok) break;
+          ok = ok && mbar_wait(&sh.in_full[s], (kidx / kInStages) & 1);
+          if (ENC != ENC_BF16) ok = ok && mbar_wait(&sh.b_full[sb], (kidx / kBStages) & 1);
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + s * kATile), b_addr = smem_u32(sB + sb * kBTile);
+          if (gather) fence_proxy_async();               // rows copied by cp.async -> visible to the tensor core
+          if (elect_one()) {
+            const uint64_t adesc = smem_desc_sw128(smem_u32(sA + s * kATile)), bdesc = smem_desc_sw128(smem_u32(sB + sb * kBTile));
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t bdesc = smem_desc_sw128(b_addr + k * 32);
-            const uint32_t accumulate = kc != t.k0 || k ? 1u : 0u;
-            tc_mma_bf16(tmem, smem_desc_sw128(a_addr + k * 32), bdesc, kInstrDesc, accumulate);
-            if (two) tc_mma_bf16(tmem + BN, smem_desc_sw128(a_addr + kAHalf + k * 32), bdesc, kInstrDesc, accumulate);
+            for (int k = 0; k < BK / 16; ++k) {            // 32 bytes along k: descriptors count 16-byte units
+              const uint32_t accumulate = k ? 1u : (uint32_t)(kc != t.k0);
+              tc_mma_bf16(tmem, adesc + k * 2, bdesc + k * 2, kInstrDesc, accumulate);
+              if (two) tc_mma_bf16(tmem + BN, adesc + (kAHalf >> 4) + k * 2, bdesc + k * 2, kInstrDesc, accumulate);
+            }
+            if (ENC != ENC_BF16) tc_commit(&sh.b_empty[sb]);
+            tc_commit(&sh.in_empty[s]);                    // A tile (and a BF16 B tile) may be overwritten
+            if (kc == t.k1 - 1) tc_commit(&sh.acc_full);
           }
-          tc_commit(&sh.in_empty[s]);                 // A tile (and a BF16 B tile) may be overwritten
-          if (ENC != ENC_BF16) tc_commit(&sh.b_empty[sb]);
+          __syncwarp();
         }
-        if (!ok) { fail(); break; }
-        tc_commit(&sh.acc_full);
+        if (!ok) { if (lane == 0) fail(); break; }
       }
     }
   } else if (warp >= 2) {

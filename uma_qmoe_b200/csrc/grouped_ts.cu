@@ -53,7 +53,6 @@ struct TsShape {
   static constexpr int kBTile = kAtoms * kBAtom;
   static constexpr int kPStages = ENC == ENC_Q4 ? 4 : ENC == ENC_Q8 ? 3 : 4;
   static constexpr int kBStages = ENC == ENC_Q4 ? 3 : ENC == ENC_Q8 ? 2 : 4;   // what 113 KB hold beside the codes
-  static constexpr int kGatherAhead = kBStages - 1;                        // steps between issuing a stage's copies and handing it over
   static constexpr int kAccCols = kAccBufs * NMAX;
   static constexpr int kAStages = kQuant ? 2 : 1;                          // BF16: no ring, one unused pair of barriers
   static constexpr int kTmemCols = kQuant ? 256 : 128;
@@ -81,37 +80,6 @@ constexpr size_t ts_smem_bytes() {
   using S = TsShape<ENC>;
   return (size_t)S::kBStages * S::kBTile + (size_t)S::kPStages * S::kWeightBytes + S::kScaleBytes + sizeof(TsShared<ENC>) + 1024;
 }
-
-// slot and phase of a ring, advanced step by step
-template <int N>
-struct Ring {
-  uint32_t slot = 0, phase = 0;
-  __device__ __forceinline__ void next() { if (++slot == N) { slot = 0; phase ^= 1; } }
-};
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
-
-// D (tensor memory) += A (tensor memory, one weight row per lane) x B (shared memory, K-major)
-__device__ __forceinline__ void tc_mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                               uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// 16 words per lane: this warp's 32 lanes, 16 consecutive columns
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -228,6 +196,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
         ok = ok && (kQuant ? mbar_wait(&sh.a_full[ra.slot], ra.phase) : mbar_wait(&sh.p_full[rp.slot], rp.phase));
         if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
         tc_fence_after();
+        if (gather) fence_proxy_async();
         if (elect_one()) {
           const uint64_t bd = b_desc0 + (uint64_t)(rb.slot * (S::kBTile >> 4));       // descriptors count 16-byte units
           const uint64_t wd = w_desc0 + (uint64_t)(rp.slot * (S::kWeightBytes >> 4));
@@ -239,8 +208,8 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
             if (kQuant) tc_mma_bf16_ts(acc, a_tmem + k * 8, bdesc, idesc, accumulate);
             else tc_mma_bf16(acc, wd + k * 2, bdesc, idesc, accumulate);
           }
-          tc_commit(&sh.in_empty[rb.slot]);
           tc_commit(kQuant ? &sh.a_empty[ra.slot] : &sh.p_empty[rp.slot]);
+          tc_commit(&sh.in_empty[rb.slot]);
           if (kc == t.k1 - 1) tc_commit(&sh.acc_full[buf]);
         }
         __syncwarp();
@@ -251,44 +220,50 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     }
   } else if (warp == 1) {
     // ===================== TMA producer: scales and weight rows ==================================
-    if (lane == 0) {
+    // The whole warp waits (a lone lane's wait takes twice as long and slows the others'), one lane issues.
+    {
       uint32_t kidx = 0, seq = 0;
       Ring<kPStages> rp;
-      for (int it = first; it < total && !*abort_flag; it += step) {
+      for (int it = first; it < total; it += step) {
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
         const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
         if (t.nrows == 0) continue;
         const long long wrow0 = (long long)t.expert * p.n_rows + t.col * kFeatures;
         if (kQuant) {
           const uint32_t sb = seq & 1;
-          if (seq >= 2 && !mbar_wait(&sh.sc_empty[sb], ((seq >> 1) - 1) & 1)) { fail(); break; }
+          if (!__all_sync(0xffffffffu, seq < 2 || mbar_wait(&sh.sc_empty[sb], ((seq >> 1) - 1) & 1))) { if (lane == 0) fail(); break; }
           float* dst = sScales + sb * kRows * kTsMaxGroups;
           const uint32_t bytes = (uint32_t)kFeatures * groups * 4;
-          mbar_expect_tx(&sh.sc_full[sb], MODE == 0 ? 2 * bytes : bytes);
-          bulk_g2s(dst, p.scales0 + wrow0 * groups, bytes, &sh.sc_full[sb]);
-          if (MODE == 0) bulk_g2s(dst + kFeatures * groups, p.scales1 + wrow0 * groups, bytes, &sh.sc_full[sb]);
+          if (lane == 0) {
+            mbar_expect_tx(&sh.sc_full[sb], MODE == 0 ? 2 * bytes : bytes);
+            bulk_g2s(dst, p.scales0 + wrow0 * groups, bytes, &sh.sc_full[sb]);
+            if (MODE == 0) bulk_g2s(dst + kFeatures * groups, p.scales1 + wrow0 * groups, bytes, &sh.sc_full[sb]);
+          }
+          __syncwarp();
         }
         ++seq;
         bool ok = true;
         for (int kc = t.k0; kc < t.k1; ++kc, ++kidx, rp.next()) {
           const uint32_t s = rp.slot;
-          if (kidx >= (uint32_t)kPStages && !mbar_wait(&sh.p_empty[s], rp.phase ^ 1)) { ok = false; break; }
-          mbar_expect_tx(&sh.p_full[s], S::kWeightBytes);
+          ok = __all_sync(0xffffffffu, kidx < (uint32_t)kPStages || mbar_wait(&sh.p_empty[s], rp.phase ^ 1));
+          if (!ok) break;
+          if (lane == 0) mbar_expect_tx(&sh.p_full[s], S::kWeightBytes);
+          __syncwarp();
           uint8_t* dst = sP + s * S::kWeightBytes;
-          if (kQuant) {
+          if (!kQuant && MODE == 0) {
+            // 16 gate rows and the 16 up rows of the same features share a lane quarter: boxes of 16 rows, a lane each
+            if (lane < 8)
+              tma_load_2d(dst + lane * 16 * 128, lane & 1 ? &map_w1 : &map_w0, kc * kAtomK, (int)wrow0 + (lane >> 1) * 16, &sh.p_full[s]);
+          } else if (lane != 0) {
+          } else if (kQuant) {
             tma_load_2d(dst, &map_w0, kc * S::kPackedRow, (int)wrow0, &sh.p_full[s]);
             if (MODE == 0) tma_load_2d(dst + kFeatures * S::kPackedRow, &map_w1, kc * S::kPackedRow, (int)wrow0, &sh.p_full[s]);
-          } else if (MODE == 1) {
-            tma_load_2d(dst, &map_w0, kc * kAtomK, (int)wrow0, &sh.p_full[s]);
           } else {
-            // 16 gate rows and the 16 up rows of the same features share a lane quarter: boxes of 16 rows
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              tma_load_2d(dst + q * 32 * 128, &map_w0, kc * kAtomK, (int)wrow0 + q * 16, &sh.p_full[s]);
-              tma_load_2d(dst + (q * 32 + 16) * 128, &map_w1, kc * kAtomK, (int)wrow0 + q * 16, &sh.p_full[s]);
-            }
+            tma_load_2d(dst, &map_w0, kc * kAtomK, (int)wrow0, &sh.p_full[s]);
           }
+          __syncwarp();
         }
-        if (!ok) { fail(); break; }
+        if (!ok) { if (lane == 0) fail(); break; }
       }
       if (*abort_flag) {                                // nobody consumes: wait (bounded) for the copies in flight
         if (kQuant)
@@ -300,25 +275,29 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
   } else if (warp < 4) {
     if (!gather) {
       // ===================== TMA producer: activation rows in sorted order =========================
-      if (warp == 2 && lane == 0) {
+      if (warp == 2) {
         uint32_t kidx = 0;
         Ring<kBStages> rb;
-        for (int it = first; it < total && !*abort_flag; it += step) {
+        for (int it = first; it < total; it += step) {
+          if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
           const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
           if (t.nrows == 0) continue;
           const int boxes = (t.nrows + kActBox - 1) / kActBox;
           bool ok = true;
           for (int kc = t.k0; kc < t.k1; ++kc, ++kidx, rb.next()) {
             const uint32_t s = rb.slot;
-            if (kidx >= (uint32_t)kBStages && !mbar_wait(&sh.in_empty[s], rb.phase ^ 1)) { ok = false; break; }
-            mbar_expect_tx(&sh.in_full[s], S::kAtoms * boxes * kActBox * 128);
-#pragma unroll
-            for (int a = 0; a < S::kAtoms; ++a)
-              for (int b = 0; b < boxes; ++b)
-                tma_load_2d(sB + s * S::kBTile + a * S::kBAtom + b * kActBox * 128, &map_act, kc * S::kStepK + a * kAtomK,
-                            t.row0 + b * kActBox, &sh.in_full[s]);
+            ok = __all_sync(0xffffffffu, kidx < (uint32_t)kBStages || mbar_wait(&sh.in_empty[s], rb.phase ^ 1));
+            if (!ok) break;
+            if (lane == 0) mbar_expect_tx(&sh.in_full[s], S::kAtoms * boxes * kActBox * 128);
+            __syncwarp();
+            if (lane < S::kAtoms * boxes) {                 // a box per lane
+              const int a = lane / boxes, b = lane - a * boxes;
+              tma_load_2d(sB + s * S::kBTile + a * S::kBAtom + b * kActBox * 128, &map_act, kc * S::kStepK + a * kAtomK,
+                          t.row0 + b * kActBox, &sh.in_full[s]);
+            }
+            __syncwarp();
           }
-          if (!ok) { fail(); break; }
+          if (!ok) { if (lane == 0) fail(); break; }
         }
         if (*abort_flag)
           for (uint32_t k2 = kidx > (uint32_t)kBStages ? kidx - kBStages : 0; k2 < kidx; ++k2)
@@ -332,15 +311,9 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
       const int pt = tid - 64;                              // 0 .. 63
       const int c = pt & 7, rbase = pt >> 3;                // rows rbase + 8 i: all have r & 7 == rbase
       const uint32_t dst_off = (uint32_t)rbase * 128 + (uint32_t)((c ^ rbase) << 4);
-      uint32_t kidx = 0, published = 0;
-      Ring<kBStages> rb, rpub;
+      uint32_t kidx = 0;
+      Ring<kBStages> rb;
       bool ok = true;
-      auto publish = [&]() {
-        fence_proxy_async();
-        mbar_arrive(&sh.in_full[rpub.slot]);
-        rpub.next();
-        ++published;
-      };
       for (int it = first; it < total; it += step) {
         // everybody has read the previous tile's table, and the threads agree whether to go on
         if (named_bar_or(1, kTsGatherThreads, !ok || *abort_flag != 0)) break;
@@ -354,8 +327,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
         for (int i = 0; i < NMAX / 8; ++i) tok[i] = sh.gather_token[rbase + 8 * i];
         const uint8_t* col = reinterpret_cast<const uint8_t*>(p.gather_src) + c * 16;
         for (int kc = 0; kc < nk; ++kc, ++kidx, rb.next(), col += S::kStepK * 2) {
-          if (kidx >= (uint32_t)S::kGatherAhead) { cp_async_wait<S::kGatherAhead - 1>(); publish(); }
-          if (kidx >= (uint32_t)kBStages && !mbar_wait(&sh.in_empty[rb.slot], rb.phase ^ 1)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, kidx < (uint32_t)kBStages || mbar_wait(&sh.in_empty[rb.slot], rb.phase ^ 1))) { ok = false; break; }
           uint8_t* dst = sB + rb.slot * S::kBTile + dst_off;
 #pragma unroll
           for (int i = 0; i < NMAX / 8; ++i) {
@@ -365,13 +337,12 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
               for (int a = 0; a < S::kAtoms; ++a) cp_async16(dst + a * S::kBAtom + i * 1024, src + a * 128, tok[i] >= 0);
             }
           }
-          cp_async_commit();
+          cp_async_arrive(&sh.in_full[rb.slot]);            // when they have landed; the issuer fences them towards the tensor core
         }
       }
       if (!ok && lane == 0) fail();
+      cp_async_commit();
       cp_async_wait<0>();                                   // also on the abort path: nothing of this thread stays in flight
-      if (ok && !*abort_flag)
-        while (published < kidx) publish();
     }
   } else if (kQuant && warp < 4 + S::kConvertWarps) {
     // ===================== conversion warps: packed codes -> BF16 rows of A in tensor memory =========
