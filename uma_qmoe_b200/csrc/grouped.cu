@@ -341,13 +341,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           if (ok && use > 0) ok = mbar_wait(&sh.b_empty[sb], (use - 1) & 1);
           if (!ok) break;
           const float scale = sc[kc >> 1];
+          const Q4Scale qs = q4_scale(scale);
+          const bool fused = ENC == ENC_Q4 && __all_sync(0xffffffffu, qs.fused);
           const uint8_t* src = sP + s * kPackedBytes + r * kPackedRow;
           uint8_t* dstrow = sB + sb * kBTile + r * 128;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {                 // the two 32-wide halves of the k chunk
             uint32_t out[16];
             if (ENC == ENC_Q4) {
-              convert_q4(*reinterpret_cast<const uint4*>(src + h * 16), scale, out);
+              const uint4 raw = *reinterpret_cast<const uint4*>(src + h * 16);
+              if (fused) convert_q4_fused(raw, qs, out);
+              else convert_q4(raw, scale, out);
             } else {
               convert_q8(*reinterpret_cast<const uint4*>(src + h * 32), *reinterpret_cast<const uint4*>(src + h * 32 + 16),
                          scale, out);

@@ -363,6 +363,8 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
       const float* sc = sScales + sbuf * kRows * kTsMaxGroups + row * groups;
       for (int kc = 0; kc < nk && ok; ++kc, ++kidx) {
         const float scale = sc[kc];
+        const Q4Scale qs = q4_scale(scale);
+        const bool fused = ENC == ENC_Q4 && __all_sync(0xffffffffu, qs.fused);
         ok = mbar_wait(&sh.p_full[rp.slot], rp.phase);
         if (!ok) break;
         const uint8_t* src = sP + rp.slot * S::kWeightBytes + row * S::kPackedRow;
@@ -370,7 +372,9 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
 #pragma unroll
         for (int j = 0; j < 2; ++j) {                       // 32 codes each
           if (ENC == ENC_Q4) {                              // 64-byte rows, TMA swizzle: 16-byte chunk ^ (row >> 1 & 3)
-            convert_q4(*reinterpret_cast<const uint4*>(src + (((2 * half + j) ^ ((row >> 1) & 3)) << 4)), scale, out[j]);
+            const uint4 raw = *reinterpret_cast<const uint4*>(src + (((2 * half + j) ^ ((row >> 1) & 3)) << 4));
+            if (fused) convert_q4_fused(raw, qs, out[j]);
+            else convert_q4(raw, scale, out[j]);
           } else {                                          // 128-byte rows: chunk ^ (row & 7)
             const int c = 4 * half + 2 * j;
             convert_q8(*reinterpret_cast<const uint4*>(src + ((c ^ (row & 7)) << 4)),

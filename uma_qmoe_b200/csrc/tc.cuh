@@ -153,6 +153,35 @@ __device__ __forceinline__ void convert_q4(const uint4 raw, float scale, uint32_
     }
   }
 }
+// The same bits with 9 instead of 15 instructions per 8 codes, for scales from 2^-100 to 2^-5 (exclusive, after rounding to BF16):
+// the nibble c + 8 in bits 0..3 (4..7) of a BF16 word is the subnormal (c + 8) * 2^-133 (2^-129), and one fused
+// multiply-add with scale * 2^133 (2^129) and -8 * scale rounds c * scale once, as the multiplication above does.
+struct Q4Scale {
+  __nv_bfloat162 low, high, bias;
+  bool fused;
+};
+__device__ __forceinline__ Q4Scale q4_scale(float scale) {
+  const float s = bf16_round(scale);
+  Q4Scale q;
+  q.fused = s >= 0x1p-100f && s < 0x1p-5f;
+  q.low = __float2bfloat162_rn(s * 0x1p100f * 0x1p33f);
+  q.high = __float2bfloat162_rn(s * 0x1p100f * 0x1p29f);
+  q.bias = __float2bfloat162_rn(-8.f * s);
+  return q;
+}
+__device__ __forceinline__ void convert_q4_fused(const uint4 raw, const Q4Scale& q, uint32_t (&out)[16]) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t m = i & 1 ? lop3<0x6A>(w[j] >> (4 * (i & 2)), 0x00F000F0u, 0x00800080u)
+                               : lop3<0x6A>(w[j] >> (4 * (i & 2)), 0x000F000Fu, 0x00080008u);
+      const __nv_bfloat162 v = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&m), i & 1 ? q.high : q.low, q.bias);
+      out[j * 4 + i] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+  }
+}
 // Q8: 32 bytes -> 16 bf16x2 words in the permuted order; code * scale in float32, one rounding.
 __device__ __forceinline__ void convert_q8(const uint4 r0, const uint4 r1, float scale, uint32_t (&out)[16]) {
   const uint32_t w[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
