@@ -333,7 +333,10 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   sa.num_tiles = reinterpret_cast<int*>(at(pl.num_tiles));
   sa.tile_expert = tiles; sa.tile_row0 = tiles + pl.max_tiles; sa.tile_rows = tiles + 2 * pl.max_tiles;
   sa.max_tiles = pl.max_tiles; sa.tile_cap = grouped_gemm_tile_cap(layer->encoding, routes, E, 0); sa.status = status;
-  if (grouped_gemm_choice_on_device(layer->encoding, routes, E, tokens, 0)) {
+  const bool wide = grouped_gemm_takes_wide(layer->encoding, routes, E, H, I);
+  if (wide) {
+    sa.tile_cap = kTileCapWide;
+  } else if (grouped_gemm_choice_on_device(layer->encoding, routes, E, tokens, 0)) {
     sa.use_ts = reinterpret_cast<int*>(at(pl.status) + 64);
     sa.choice = grouped_gemm_choice(layer->encoding, I, H);
   }
@@ -377,7 +380,13 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   down.out = reinterpret_cast<__nv_bfloat16*>(at(pl.yw)); down.out_stride = H; down.route_weight = sa.sorted_weight; down.permute_out = 0;
   // Where the sort picks the kernel: both GEMMs on transposed tiles, then both on one-CTA tiles.  The pair that is not wanted
   // returns, and in this order it stands between no two kernels that work.
-  for (int conditional = sa.use_ts ? 1 : 0; conditional <= (sa.use_ts ? 2 : 0); ++conditional) {
+  if (wide) {
+    rc = launch_grouped_gemm_wide(g, stream);
+    if (rc) return rc;
+    rc = launch_grouped_gemm_wide(down, stream);
+    if (rc) return rc;
+  }
+  for (int conditional = sa.use_ts ? 1 : 0; !wide && conditional <= (sa.use_ts ? 2 : 0); ++conditional) {
     g.conditional = down.conditional = conditional;
     if (conditional) g.tile_cap = down.tile_cap = conditional == 1 ? kTileCapMin : kTileCapMax;
     rc = launch_grouped_gemm(g, stream);

@@ -616,6 +616,18 @@ long long grouped_gemm_dense_part_rows(long long rows, int n_rows, int k) {
     if (at == rows || (splits == 1 && at > kTsMaxRowsDense[1])) return most;
   }
 }
+// Between the transposed kernel and full 256-row tiles: wide transposed tiles (grouped_wide.cu).  Whole operator, us, without |
+// with them, routes spread evenly / by the skewed router:
+//   OLMoE Q4   88 routes per expert 161 | 146 / 149 | 151   128: 197 | 159 / 199 | 186   256: 289 | 259 / 291 | 278   512: 454 | 449 / 461 | 442
+//   OLMoE Q8   88 routes per expert 217 | 182 / 234 | 188   128: 242 | 196 / 234 | 230   256: 345 | 324 / 346 | 344   512: 532 | 543 / 520 | 552
+//   Qwen  Q8  102 routes per expert 270 | 226 / 281 | 238   136: 310 | 243 / 291 | 273   273: 488 | 422 / 421 | 420   546: 814 | 724 / 715 | 746
+// Around 192 (a tile and a little more for many experts) they lose: 192, OLMoE Q4 212 | 232 / 241 | 228, Q8 258 | 288 / 290 | 284.
+constexpr long long kWideGapFrom = 160, kWideGapTo = 248, kWideMaxRoutesQ4 = 512, kWideMaxRoutesQ8 = 288;
+bool grouped_gemm_takes_wide(int enc, long long rows, int experts, int hidden, int inter) {
+  if (enc == ENC_BF16 || hidden % 256 || inter % 128 || hidden > 2048 || inter > 2048) return false;
+  if (takes_ts_kernel(enc, rows, experts, 0, 0) || rows > experts * (enc == ENC_Q4 ? kWideMaxRoutesQ4 : kWideMaxRoutesQ8)) return false;
+  return rows <= experts * kWideGapFrom || rows >= experts * kWideGapTo;
+}
 int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant) {
   return takes_ts_kernel(enc, rows, num_experts, variant, 0) ? kTileCapMin : kTileCapMax;
 }

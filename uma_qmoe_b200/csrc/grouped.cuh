@@ -10,6 +10,7 @@
 namespace umaq {
 
 constexpr int kTileCapMin = 64, kTileCapMax = 256;   // routes of a tile: transposed kernel (grouped_ts.cu), the others
+constexpr int kTileCapWide = 192;                    // wide transposed kernel (grouped_wide.cu)
 
 // The choice between the one-CTA and the transposed kernel when routes concentrate on some experts: see grouped.cu.
 struct TileChoice {
@@ -96,7 +97,10 @@ int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream);        /
 int launch_grouped_gemm_single(const GroupedGemmArgs& a, cudaStream_t stream);
 int launch_grouped_gemm_pair(const GroupedGemmArgs& a, cudaStream_t stream);
 int launch_grouped_gemm_ts(const GroupedGemmArgs& a, cudaStream_t stream);
+int launch_grouped_gemm_wide(const GroupedGemmArgs& a, cudaStream_t stream);   // only when asked for: the table is cut for it
 
+// Whether both GEMMs of a quantised layer run on wide transposed tiles (grouped_wide.cu), the sort cutting its table for them
+bool grouped_gemm_takes_wide(int enc, long long rows, int experts, int hidden, int inter);
 // Routes per tile that suit the kernel launch_grouped_gemm picks for a layer: the cap to build the tile table with.
 int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant);
 // Whether that pick has to be made on the device, from the routes that the experts have; `most`: the most one can have

@@ -587,8 +587,11 @@ __device__ __forceinline__ void emit_offsets_and_tiles(const SortArgs& a, const 
     for (int e = tid; e < E; e += nthreads) {
       const int c = start[e + 1] - start[e];
       int t = tile_base[e];
-      for (int r = 0; r < c && t < a.max_tiles; r += tile_cap, ++t) {
-        a.tile_expert[t] = e; a.tile_row0[t] = start[e] + r; a.tile_rows[t] = min(tile_cap, c - r);
+      // the time of a wide tile follows its routes: equal ones (multiples of 16) instead of full ones and a rest
+      const int parts = (c + tile_cap - 1) / tile_cap;
+      const int each = tile_cap == kTileCapWide && c > 0 ? ((c + parts - 1) / parts + 15) & ~15 : tile_cap;
+      for (int q = 0; q < parts && t < a.max_tiles; ++q, ++t) {
+        a.tile_expert[t] = e; a.tile_row0[t] = start[e] + q * each; a.tile_rows[t] = max(0, min(each, c - q * each));
       }
     }
     if (tid == 0) *a.num_tiles = min(tile_base[E], a.max_tiles);
