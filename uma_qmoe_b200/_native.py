@@ -58,6 +58,9 @@ SIGNATURES = {
                                    C.c_void_p, C.c_longlong, C.c_int, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
     "umaq_moe_prefill_digits": (C.c_int, [C.POINTER(Layer), C.POINTER(SharedExpert), C.c_void_p, C.c_void_p, C.c_int,
                                           C.c_void_p, C.c_longlong, C.c_int, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
+    "umaq_moe_step": (C.c_int, [C.POINTER(Layer), C.POINTER(SharedExpert), C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p,
+                                C.c_int, C.c_void_p, C.c_longlong, C.c_int, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p,
+                                C.c_void_p, C.c_void_p]),
     "umaq_route_sort": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p,
                                   C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p,
                                   C.c_void_p, C.c_longlong, C.c_void_p]),

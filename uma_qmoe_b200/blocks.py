@@ -2,10 +2,10 @@
 ``QuantizedMoEBlock`` (``src/uma_qmoe/compressed_loader.py:41-67``) and
 ``QuantizedQwenMoEBlock`` (``src/uma_qmoe/qwen_compressed_loader.py:46-86``).
 
-They call the same ``torch.ops.uma_qmoe`` operators; what they add is the fused path around it: the
-router runs as one kernel (softmax / top-k / renormalisation), and for Qwen the shared expert, its
-sigmoid gate and the final add run inside the expert kernels instead of as separate cuBLAS and
-element-wise launches.
+They run what the ``torch.ops.uma_qmoe`` operators run, with the path around it fused: the router
+(softmax / top-k / renormalisation) is one kernel, for Qwen the shared expert, its sigmoid gate and the
+final add run inside the expert kernels instead of as separate cuBLAS and element-wise launches, and the
+back end issues all of it from one native call.
 """
 
 from __future__ import annotations
@@ -15,7 +15,7 @@ from typing import Any
 import torch
 
 from . import ops
-from .custom_op import _backend_for, platform_of
+from .custom_op import _backend_for, acquire_expert_pack, platform_of
 from .ops import DeviceSharedExpert
 
 
@@ -36,6 +36,10 @@ class QuantizedMoEBlock(torch.nn.Module):
     def forward(self, hidden_states: torch.Tensor) -> torch.Tensor:
         weight, top_k, renorm = _router_params(self.gate)
         flat = hidden_states.reshape(-1, hidden_states.shape[-1])
+        whole = getattr(_backend_for(platform_of(torch, flat)), "block_forward", None)
+        if callable(whole):                       # router and experts in one native call
+            with acquire_expert_pack(self.pack_handle):
+                return whole("olmoe", flat, weight, top_k, renorm, self.layer_index, self.pack_handle).view(hidden_states.shape)
         routing_weights, selected = ops.route_topk(flat, weight, top_k, renorm)
         return torch.ops.uma_qmoe.moe_forward(hidden_states, selected, routing_weights, self.layer_index,
                                               self.pack_handle, self.performance_mode)
@@ -63,13 +67,17 @@ class QuantizedQwenMoEBlock(torch.nn.Module):
         batch, seq, hidden = hidden_states.shape
         flat = hidden_states.reshape(-1, hidden)
         weight, top_k, renorm = _router_params(self.gate)
-        routing_weights, selected = ops.route_topk(flat, weight, top_k, renorm)
         backend = _backend_for(platform_of(torch, flat))
+        whole = getattr(backend, "block_forward", None)
+        if callable(whole):                       # router, experts and shared expert in one native call
+            with acquire_expert_pack(self.pack_handle):
+                return whole("qwen", flat, weight, top_k, renorm, self.layer_index, self.pack_handle,
+                             self._shared()).view(batch, seq, hidden)
+        routing_weights, selected = ops.route_topk(flat, weight, top_k, renorm)
         fused = getattr(backend, "qwen_block_forward", None)
         if not callable(fused):
             raise RuntimeError("performance mode has no Qwen-capable backend with a fused shared expert; "
                                "silent reference fallback is forbidden")
-        from .custom_op import acquire_expert_pack
         with acquire_expert_pack(self.pack_handle):
             out = fused(flat, selected, routing_weights, self.layer_index, self.pack_handle, self._shared())
         return out.reshape(batch, seq, hidden)

@@ -57,9 +57,9 @@ size_t umaq_decode_workspace_bytes(int top_k, int intermediate, int shared_inter
   return decode_workspace_bytes(top_k, intermediate, shared_intermediate);
 }
 
-int umaq_moe_decode(const umaq_layer* layer, const umaq_shared_expert* shared, const void* hidden_bf16,
-                    const void* expert_indices, int indices_are_int64, const float* routing_weights, int top_k,
-                    void* out_bf16, void* workspace, size_t workspace_bytes, void* stream) {
+static int decode_impl(const umaq_layer* layer, const umaq_shared_expert* shared, const void* hidden_bf16,
+                       const void* expert_indices, int indices_are_int64, const float* routing_weights, int top_k,
+                       void* out_bf16, void* workspace, size_t workspace_bytes, unsigned* host_status, void* stream) {
   if (!layer || !hidden_bf16 || !expert_indices || !routing_weights || !out_bf16 || !workspace) {
     set_error("umaq_moe_decode: null argument");
     return ERR_BAD_ARGUMENT;
@@ -101,7 +101,15 @@ int umaq_moe_decode(const umaq_layer* layer, const umaq_shared_expert* shared, c
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   p.sync = reinterpret_cast<unsigned*>(ws);
   p.inter_buf = ws + kDecodeWsHeader;
+  p.host_status = host_status;
   return launch_moe_decode(p, static_cast<cudaStream_t>(stream));
+}
+
+int umaq_moe_decode(const umaq_layer* layer, const umaq_shared_expert* shared, const void* hidden_bf16,
+                    const void* expert_indices, int indices_are_int64, const float* routing_weights, int top_k,
+                    void* out_bf16, void* workspace, size_t workspace_bytes, void* stream) {
+  return decode_impl(layer, shared, hidden_bf16, expert_indices, indices_are_int64, routing_weights, top_k, out_bf16, workspace,
+                     workspace_bytes, nullptr, stream);
 }
 
 int umaq_quantize_groups(const void* src_bf16, long long elements, int encoding, void* codes, float* scales,
@@ -303,7 +311,7 @@ size_t umaq_prefill_workspace_bytes(long long tokens, int top_k, int num_experts
 static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* shared, const void* hidden_bf16,
                         const void* expert_indices, int indices_are_int64, const float* routing_weights, long long tokens,
                         int top_k, void* out_bf16, void* workspace, size_t workspace_bytes, void* stream_,
-                        const SegmentedOut* segments, bool rows_k_permuted = false, bool digits = false) {
+                        const SegmentedOut* segments, bool rows_k_permuted = false, bool digits = false, unsigned* host_status = nullptr) {
   if (!layer || !hidden_bf16 || !expert_indices || !routing_weights || (!out_bf16 && !segments) || !workspace || tokens <= 0) {
     set_error("umaq_moe_prefill: null argument");
     return ERR_BAD_ARGUMENT;
@@ -442,7 +450,7 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   return launch_combine(reinterpret_cast<const __nv_bfloat16*>(at(pl.yw)), expert_indices, indices_are_int64, sa.route_pos,
                         (int)tokens, top_k, H, E, shared_out, shared_part, shared_parts, static_cast<const __nv_bfloat16*>(hidden_bf16),
                         shared ? static_cast<const __nv_bfloat16*>(shared->gate_vec) : nullptr,
-                        static_cast<__nv_bfloat16*>(out_bf16), stream, segments);
+                        static_cast<__nv_bfloat16*>(out_bf16), stream, segments, StatusMirror{status, host_status});
 }
 
 int umaq_moe_prefill(const umaq_layer* layer, const umaq_shared_expert* shared, const void* hidden_bf16,
@@ -457,6 +465,30 @@ int umaq_moe_prefill_digits(const umaq_layer* layer, const umaq_shared_expert* s
                             int top_k, void* out_bf16, void* workspace, size_t workspace_bytes, void* stream_) {
   return prefill_impl(layer, shared, hidden_bf16, expert_indices, indices_are_int64, routing_weights, tokens, top_k,
                       out_bf16, workspace, workspace_bytes, stream_, nullptr, false, true);
+}
+
+int umaq_moe_step(const umaq_layer* layer, const umaq_shared_expert* shared, const void* hidden_bf16, const void* router_weight_bf16,
+                  int router_experts, int renormalize, void* expert_indices, int indices_are_int64, float* routing_weights,
+                  long long tokens, int top_k, void* out_bf16, void* workspace, size_t workspace_bytes, unsigned* host_status,
+                  void* event, void* stream) {
+  if (!layer || tokens <= 0 || tokens > 0x7fffffffLL) { set_error("umaq_moe_step: bad argument"); return ERR_BAD_ARGUMENT; }
+  int rc = ERR_NONE;
+  if (router_weight_bf16) {
+    if (!indices_are_int64) { set_error("umaq_moe_step: the router writes int64 indices"); return ERR_BAD_ARGUMENT; }
+    rc = umaq_route_topk(hidden_bf16, router_weight_bf16, (int)tokens, layer->hidden, router_experts, top_k, renormalize,
+                         routing_weights, static_cast<long long*>(expert_indices), nullptr, stream);
+    if (rc) return rc;
+  }
+  rc = tokens == 1 ? decode_impl(layer, shared, hidden_bf16, expert_indices, indices_are_int64, routing_weights, top_k, out_bf16,
+                                 workspace, workspace_bytes, host_status, stream)
+                   : prefill_impl(layer, shared, hidden_bf16, expert_indices, indices_are_int64, routing_weights, tokens, top_k,
+                                  out_bf16, workspace, workspace_bytes, stream, nullptr, false, true, host_status);
+  if (rc) return rc;
+  if (event) {
+    const cudaError_t e = cudaEventRecord(static_cast<cudaEvent_t>(event), static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) { set_error("umaq_moe_step: cudaEventRecord: %s", cudaGetErrorString(e)); return ERR_LAUNCH; }
+  }
+  return ERR_NONE;
 }
 
 int umaq_moe_prefill_to_peers(const umaq_layer* layer, const void* hidden_bf16, const void* expert_indices,

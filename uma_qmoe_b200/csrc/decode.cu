@@ -1208,6 +1208,10 @@ __global__ void __maxnreg__(96) decode_down_kernel(const DecodeParams p) {
     atomicExch(p.sync + kSyncStatus, (unsigned)ERR_DEVICE_TIMEOUT);
     __nanosleep(100000);
   }
+  if (p.host_status && blockIdx.x == 0 && tid == 0) {       // the gate/up kernel's reports are behind its counter
+    const unsigned code = *reinterpret_cast<const volatile unsigned*>(p.sync + kSyncStatus);
+    if (code) *reinterpret_cast<volatile unsigned*>(p.host_status) = code;
+  }
   stamp(p, 24, 0);
 }
 

@@ -92,6 +92,7 @@ struct DecodeParams {
                               // finished, over all calls, and sync[6] is the count the current call's down kernel
                               // waits for (every call adds its grid size; the words are never reset)
   uint8_t* inter_buf;         // intermediate fragments (after the header)
+  unsigned* host_status;      // mapped host memory that receives the status word if it is set (null: nowhere)
   // launch plans, filled by launch_moe_decode
   DecodeKernelPlan g;         // gate/up + SwiGLU kernel
   DecodeKernelPlan d;         // down + combine kernel

@@ -183,9 +183,15 @@ struct SegmentedOut {
 };
 // experts: ids outside [0, experts) are treated as absent routes.  The shared expert's rows come as BF16 (shared_out) or
 // as shared_parts float32 partial sums [shared_parts, tokens, hidden] that are added here and rounded once.
+// The sticky status word and where the host looks at it (mapped host memory, null: nowhere).  The last kernel of a call copies
+// the word there if it is set, so that a call without an error moves nothing.
+struct StatusMirror {
+  const unsigned* status;
+  unsigned* host;
+};
 int launch_combine(const __nv_bfloat16* weighted, const void* indices, int idx64, const int* route_pos, int tokens,
                    int top_k, int hidden, int experts, const __nv_bfloat16* shared_out, const float* shared_part,
                    int shared_parts, const __nv_bfloat16* x, const __nv_bfloat16* gate_vec, __nv_bfloat16* out, cudaStream_t stream,
-                   const SegmentedOut* segments = nullptr);
+                   const SegmentedOut* segments = nullptr, StatusMirror mirror = {nullptr, nullptr});
 
 }  // namespace umaq

@@ -851,13 +851,20 @@ __global__ void ep_pack_kernel(const __nv_bfloat16* __restrict__ x, const int* _
 // contributions are already BF16 (GEMM 2 epilogue).  With a shared expert: + bf16(sigmoid(bf16(x . wg))
 // * shared_out[t]), as QuantizedQwenMoEBlock does after the operator
 // (src/uma_qmoe/qwen_compressed_loader.py:82-85).
+__device__ __forceinline__ void mirror_status(const StatusMirror& m) {
+  if (m.host && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+    const unsigned code = *reinterpret_cast<const volatile unsigned*>(m.status);
+    if (code) *reinterpret_cast<volatile unsigned*>(m.host) = code;
+  }
+}
 template <bool PARTS>                             // the shared expert's rows come as float32 partial sums
 __global__ void __launch_bounds__(256, PARTS ? 2 : 4)
 combine_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __restrict__ indices, int idx64,
                const int* __restrict__ route_pos, int top_k, int hidden, int experts,
                const __nv_bfloat16* __restrict__ shared_out, const float* __restrict__ shared_part, int shared_parts,
-               const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate_vec, __nv_bfloat16* __restrict__ out, const __grid_constant__ SegmentedOut seg) {
+               const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate_vec, __nv_bfloat16* __restrict__ out, const __grid_constant__ SegmentedOut seg, const StatusMirror mirror) {
   pdl_wait();      // no early start for what follows: the chain ends here, the next kernel may be anybody's
+  mirror_status(mirror);
   __shared__ int order_pos[8];
   __shared__ int present;
   __shared__ float red[8];
@@ -981,8 +988,9 @@ constexpr int kCombineSpreadWarps = 4736;    // 32 warps on each of 148 SMs
 __global__ void __launch_bounds__(kCombineWarps * 32)
 combine_warp_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __restrict__ indices, int idx64,
                     const int* __restrict__ route_pos, int tokens, int top_k, int hidden, int experts,
-                    __nv_bfloat16* __restrict__ out, const __grid_constant__ SegmentedOut seg) {
+                    __nv_bfloat16* __restrict__ out, const __grid_constant__ SegmentedOut seg, const StatusMirror mirror) {
   pdl_wait();
+  mirror_status(mirror);
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * kCombineWarps + (threadIdx.x >> 5);
   if (t >= tokens) return;                                   // the whole warp
@@ -1144,7 +1152,7 @@ int launch_gather_rows(const __nv_bfloat16* x, const int* sorted_route, int top_
 int launch_combine(const __nv_bfloat16* weighted, const void* indices, int idx64, const int* route_pos, int tokens,
                    int top_k, int hidden, int experts, const __nv_bfloat16* shared_out, const float* shared_part,
                    int shared_parts, const __nv_bfloat16* x, const __nv_bfloat16* gate_vec, __nv_bfloat16* out, cudaStream_t stream,
-                   const SegmentedOut* segments) {
+                   const SegmentedOut* segments, StatusMirror mirror) {
   if (tokens <= 0 || top_k < 1 || top_k > 8 || hidden % 8) { set_error("combine: unsupported shape"); return ERR_BAD_ARGUMENT; }
   SegmentedOut seg{};
   if (segments) seg = *segments;
@@ -1155,11 +1163,11 @@ int launch_combine(const __nv_bfloat16* weighted, const void* indices, int idx64
     const int spread = std::max(1, std::min(passes, kCombineSpreadWarps / tokens));
     return check_launch("combine", launch_chained(combine_warp_kernel, dim3((tokens + kCombineWarps - 1) / kCombineWarps, spread),
                                                   dim3(kCombineWarps * 32), 0, stream, weighted, indices, idx64, route_pos, tokens,
-                                                  top_k, hidden, experts, out, seg));
+                                                  top_k, hidden, experts, out, seg, mirror));
   }
   auto kernel = shared_parts > 0 ? combine_kernel<true> : combine_kernel<false>;
   return check_launch("combine", launch_chained(kernel, dim3(tokens), dim3(256), 0, stream, weighted, indices, idx64, route_pos, top_k,
-                                                hidden, experts, shared_out, shared_part, shared_parts, x, gate_vec, out, seg));
+                                                hidden, experts, shared_out, shared_part, shared_parts, x, gate_vec, out, seg, mirror));
 }
 
 // ---- expert-parallel routing: global expert id -> this rank's local id, or -1 (absent) --------------------------

@@ -33,6 +33,7 @@ _MODELS = {
     "olmoe": (16, 64, 8, 2048, 1024),
     "qwen": (24, 60, 4, 2048, 1408),
 }
+_LABELS = {"olmoe": "OLMoE", "qwen": "Qwen"}
 
 
 def native_kernel_source_sha256() -> str:
@@ -67,48 +68,54 @@ class _LayerCache:
 
 
 class _Workspace:
-    """A kernel workspace owned by one (shape, device, stream) and the host's view of its sticky status word.
+    """A kernel workspace owned by one (shape, device, stream), room for the routes of a call that routes itself, and the host's
+    view of the workspace's sticky status word.
 
-    After every call the first 16 bytes of the workspace (prefill status in word 0, decode status in word 2) are
-    copied to pinned host memory on the call's stream and an event is recorded; the next call on this workspace,
-    `cache_summary()` and `release_pack()` look at the copy once the event has completed.  Nothing on the hot
-    path waits for the device."""
+    The last kernel of a call copies the word to mapped host memory if it is set, and an event is recorded behind the call;
+    the next call on this workspace looks at the host's copy, `cache_summary()` and `release_pack()` do once the event has
+    completed.  Nothing on the hot path waits for the device."""
 
-    __slots__ = ("kind", "buffer", "status", "host", "event", "tokens")
+    __slots__ = ("kind", "buffer", "host", "word", "event", "used", "tokens", "indices", "weights", "lock")
 
-    def __init__(self, kind: str, buffer: Any, tokens: int) -> None:
+    def __init__(self, kind: str, buffer: Any, tokens: int, top_k: int, stream: Any) -> None:
         import torch
 
         self.kind, self.buffer, self.tokens = kind, buffer, tokens
-        self.status = buffer[:16].view(torch.int32)
         self.host = torch.zeros(4, dtype=torch.int32).pin_memory()
-        self.event: Any = None
+        self.word = self.host.numpy()
+        self.event = torch.cuda.Event()
+        if not torch.cuda.is_current_stream_capturing():
+            self.event.record(stream)                # creates it
+        self.used = False
+        self.lock = threading.Lock()                 # the launches of a call stay together on the stream
+        self.indices = torch.empty((tokens, top_k), dtype=torch.int64, device=buffer.device)
+        self.weights = torch.empty((tokens, top_k), dtype=torch.float32, device=buffer.device)
 
-    def publish(self, stream: Any) -> None:
+    def report(self, device: Any) -> tuple[Optional[int], Optional[int]]:
+        """Where a call leaves its status and which event it records; a captured call reports through the workspace only."""
         import torch
 
         if torch.cuda.is_current_stream_capturing():
-            return                                   # a captured call reports through the workspace only
-        self.host.copy_(self.status, non_blocking=True)
-        if self.event is None:
-            self.event = torch.cuda.Event()
-        self.event.record(stream)
+            return None, None
+        if not self.event.cuda_event:                # made during a capture
+            self.event.record(torch.cuda.current_stream(device))
+        self.used = True
+        return self.host.data_ptr(), self.event.cuda_event
 
     def raise_if_failed(self, wait: bool) -> None:
+        if not self.used or not (wait or self.word[0]):
+            return
         import torch
 
-        if self.event is None or torch.cuda.is_current_stream_capturing():
+        if torch.cuda.is_current_stream_capturing():
             return
-        if wait:
-            self.event.synchronize()
-        elif not self.event.query():
-            return
-        code = int(self.host[0 if self.kind == "prefill" else 2])
+        self.event.synchronize()                     # all work on the buffer has finished
+        code = int(self.word[0])
         if code == 0:
             return
-        # sticky on the device: clear it so that the error is reported once (all work on the buffer has finished)
-        self.host.zero_()
-        self.event = None
+        # sticky on the device: clear it so that the error is reported once
+        self.word[0] = 0
+        self.used = False
         if code == -1:                               # UMAQ_ERR_BAD_ARGUMENT: the kernels skipped a route
             self.buffer[:16].zero_()
             raise RuntimeError("expert_indices contains an invalid expert")
@@ -293,68 +300,78 @@ class MixedTargetNativeBackend:
                 del self._linear_cache[key]
 
     # ---- execution ------------------------------------------------------------------------
-    def _workspace(self, kind: str, layer: Any, tokens: int, top_k: int, shared: Any, device: Any, stream: Any) -> _Workspace:
+    def _workspace(self, kind: str, layer: Any, tokens: int, top_k: int, shared: Any, device: Any, stream: int) -> _Workspace:
         """The workspace of this shape on this stream.  Calls on different streams (or threads, which have their own
         current stream only if they set one) never share a workspace, so they may overlap on the device; a stream
         keeps one prefill workspace per layer shape, grown to the largest token count seen."""
         from . import ops
 
-        family = (kind, str(device), int(stream.cuda_stream), layer.hidden, layer.intermediate, layer.num_experts, top_k,
-                  0 if shared is None else int(shared.gate.shape[0]))
+        family = (kind, device.index, stream, layer.hidden, layer.intermediate, layer.num_experts, top_k,
+                  0 if shared is None else shared.gate.shape[0])
         with self._workspace_lock:
             slot = self._workspaces.get(family)
             if slot is not None and (kind == "decode" or slot.tokens >= tokens):
                 return slot
+        import torch
         if slot is not None:
             slot.raise_if_failed(wait=True)          # the smaller buffer is about to be dropped
         if kind == "decode":
-            fresh = _Workspace(kind, ops.decode_workspace(layer, top_k, shared, device), 1)
+            buffer, tokens = ops.decode_workspace(layer, top_k, shared, device), 1
         else:
-            fresh = _Workspace(kind, ops.prefill_workspace(layer, tokens, top_k, shared, device), tokens)
+            buffer = ops.prefill_workspace(layer, tokens, top_k, shared, device)
+        fresh = _Workspace(kind, buffer, tokens, top_k, torch.cuda.current_stream(device))
         with self._workspace_lock:
             self._workspaces[family] = fresh
         return fresh
 
     def _run(self, model: str, hidden_states: Any, expert_indices: Any, routing_weights: Any, layer_index: int,
-             pack_handle: int, shared: Optional[Any] = None):
+             pack_handle: int, shared: Optional[Any] = None, router: Optional[tuple] = None):
+        """`router`: (weight, top_k, renormalise) of a call that routes itself; its routes stay in the workspace."""
         import torch
 
         from . import ops
 
         _layers, _experts, top_k, hidden, _inter = _MODELS[model]
-        label = "OLMoE" if model == "olmoe" else "Qwen"
         if hidden_states.dtype != torch.bfloat16:
-            raise RuntimeError(f"{label} native backend requires BF16 hidden states")
+            raise RuntimeError(f"{_LABELS[model]} native backend requires BF16 hidden states")
         flat = hidden_states.reshape(-1, hidden_states.shape[-1])
-        if flat.shape[-1] != hidden:
-            raise RuntimeError(f"{label} native backend requires hidden size {hidden}")
-        if tuple(expert_indices.shape) != (flat.shape[0], top_k):
-            raise RuntimeError(f"{label} native backend requires [tokens, {top_k}] routes")
-        if expert_indices.dtype not in (torch.int32, torch.int64):
-            raise RuntimeError("expert_indices must use int32 or int64")
-        if tuple(routing_weights.shape) != tuple(expert_indices.shape):
-            raise RuntimeError("expert_indices and routing_weights shapes must match")
-        with acquire_expert_pack(pack_handle) as reader:
-            layer = self._device_layer(pack_handle, layer_index, hidden_states.device, reader, model)
-        stream = torch.cuda.current_stream(hidden_states.device)
-        for tensor in layer.tensors:
-            tensor.record_stream(stream)
-        flat = flat.contiguous()
-        indices = expert_indices.contiguous()
-        weights = routing_weights.to(dtype=torch.float32).contiguous()     # float32 routing weights, no BF16 rounding
         tokens = flat.shape[0]
+        if flat.shape[1] != hidden:
+            raise RuntimeError(f"{_LABELS[model]} native backend requires hidden size {hidden}")
+        if router is not None:
+            ops._require_cuda_bf16(flat, "hidden_states")
+            ops._require_cuda_bf16(router[0], "router weight")
+            if router[1] != top_k or router[0].ndim != 2 or router[0].shape[1] != hidden:
+                raise RuntimeError(f"{_LABELS[model]} native backend requires [tokens, {top_k}] routes")
+        else:
+            if tuple(expert_indices.shape) != (tokens, top_k):
+                raise RuntimeError(f"{_LABELS[model]} native backend requires [tokens, {top_k}] routes")
+            if expert_indices.dtype not in (torch.int32, torch.int64):
+                raise RuntimeError("expert_indices must use int32 or int64")
+            if tuple(routing_weights.shape) != tuple(expert_indices.shape):
+                raise RuntimeError("expert_indices and routing_weights shapes must match")
+        device = flat.device
+        with acquire_expert_pack(pack_handle) as reader:
+            layer = self._device_layer(pack_handle, layer_index, device, reader, model)
+        stream = torch._C._cuda_getCurrentRawStream(device.index)
+        layer.used_on(stream, device)
+        flat = flat.contiguous()
         out = torch.empty_like(flat)
         if tokens == 0:                       # an empty batch has an empty result; there is nothing to launch
             return out.reshape(hidden_states.shape)
-        slot = self._workspace("decode" if tokens == 1 else "prefill", layer, tokens, top_k, shared,
-                               hidden_states.device, stream)
+        slot = self._workspace("decode" if tokens == 1 else "prefill", layer, tokens, top_k, shared, device, stream)
         slot.raise_if_failed(wait=False)      # an error an earlier call on this workspace left behind, if already known
-        slot.buffer.record_stream(stream)
-        if tokens == 1:
-            ops.moe_decode(layer, flat, indices, weights, slot.buffer, shared, out=out)
+        if router is None:
+            indices = expert_indices.contiguous()
+            weights = routing_weights.to(dtype=torch.float32).contiguous()     # float32 routing weights, no BF16 rounding
         else:
-            ops.moe_prefill(layer, flat, indices, weights, slot.buffer, shared, out=out)
-        slot.publish(stream)
+            indices, weights = slot.indices, slot.weights
+            if slot.tokens != tokens:
+                indices, weights = indices[:tokens], weights[:tokens]
+        host, event = slot.report(device)
+        with slot.lock:
+            ops.moe_step(layer, flat, indices, weights, out, slot.buffer, shared, None if router is None else router[0],
+                         router is not None and router[2], host, event, stream)
         return out.reshape(hidden_states.shape)
 
     # ---- one projection as a linear layer -----------------------------------------------------
@@ -418,6 +435,11 @@ class MixedTargetNativeBackend:
                            shared: Any):
         """Routed experts plus the shared expert and its sigmoid gate in the same kernels."""
         return self._run("qwen", hidden_states, expert_indices, routing_weights, layer_index, pack_handle, shared)
+
+    def block_forward(self, model: str, hidden_states, router_weight, top_k: int, renormalize: bool, layer_index: int,
+                      pack_handle: int, shared: Any = None):
+        """A whole MoE block: router, routed experts and (Qwen) the shared expert with its gate, in one native call."""
+        return self._run(model, hidden_states, None, None, layer_index, pack_handle, shared, (router_weight, top_k, renormalize))
 
 
 class PackedQ4NativeBackend(MixedTargetNativeBackend):

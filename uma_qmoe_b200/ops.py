@@ -31,6 +31,19 @@ class DeviceLayer:
     up_scales: Optional[torch.Tensor] = None
     down_scales: Optional[torch.Tensor] = None
 
+    def __setattr__(self, name: str, value) -> None:
+        object.__setattr__(self, name, value)
+        object.__setattr__(self, "_streams", set())          # other tensors: no stream has used them yet
+
+    def used_on(self, handle: int, device: torch.device) -> None:
+        """Tell the allocator that the stream ``handle`` uses these tensors.  A block keeps its streams until it is freed, so
+        once per stream is enough."""
+        if handle not in self._streams:
+            stream = torch.cuda.ExternalStream(handle, device=device) if handle else torch.cuda.default_stream(device)
+            for tensor in self.tensors:
+                tensor.record_stream(stream)
+            self._streams.add(handle)
+
     @property
     def tensors(self) -> tuple[torch.Tensor, ...]:
         return tuple(t for t in (self.gate, self.gate_scales, self.up, self.up_scales, self.down,
@@ -144,6 +157,21 @@ def moe_prefill(layer: DeviceLayer, hidden: torch.Tensor, indices: torch.Tensor,
         out.data_ptr(), workspace.data_ptr(), workspace.numel(), _stream(hidden.device))
     _native.check(code, "umaq_moe_prefill")
     return out.reshape(hidden.shape)
+
+
+def moe_step(layer: DeviceLayer, hidden: torch.Tensor, indices: torch.Tensor, weights: torch.Tensor, out: torch.Tensor,
+             workspace: torch.Tensor, shared: Optional[DeviceSharedExpert], router: Optional[torch.Tensor], renormalize: bool,
+             host_status: Optional[int], event: Optional[int], stream: int) -> None:
+    """One decode or prefill call, its router included, in one native call (``umaq_moe_step``).  The caller has checked the
+    shapes; every tensor is contiguous."""
+    tokens, top_k = indices.shape
+    code = _native.lib().umaq_moe_step(
+        layer.struct(), None if shared is None else shared.struct(), hidden.data_ptr(),
+        None if router is None else router.data_ptr(), 0 if router is None else router.shape[0], renormalize, indices.data_ptr(),
+        indices.dtype == torch.int64, weights.data_ptr(), tokens, top_k, out.data_ptr(), workspace.data_ptr(), workspace.numel(),
+        host_status, event, stream)
+    if code:
+        _native.check(code, "umaq_moe_step")
 
 
 def prefill_status(workspace: torch.Tensor) -> int:
