@@ -356,6 +356,12 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
     sa.choice = grouped_gemm_choice(layer->encoding, I, H);
   }
   sa.scratch = reinterpret_cast<int*>(at(pl.sort_scratch)); sa.scratch_ints = pl.sort_ints;
+  if (shared) {
+    int* st = reinterpret_cast<int*>(at(pl.s_tiles));
+    sa.dense_rows = (int)tokens; sa.dense_cap = grouped_gemm_tile_cap(ENC_BF16, tokens, 1, 0);
+    sa.dense_num_tiles = reinterpret_cast<int*>(at(pl.s_num_tiles));
+    sa.dense_expert = st; sa.dense_row0 = st + pl.s_max_tiles; sa.dense_tile_rows = st + 2 * pl.s_max_tiles;
+  }
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(at(pl.xs));
   GroupedGemmArgs g{};
   g.mode = 0; g.enc = layer->encoding; g.num_experts = E; g.n_rows = I; g.k = H;
@@ -424,17 +430,12 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   const float* shared_part = nullptr;
   int shared_parts = 0;
   if (shared) {
-    int* st = reinterpret_cast<int*>(at(pl.s_tiles));
-    int* snt = reinterpret_cast<int*>(at(pl.s_num_tiles));
-    const int s_cap = grouped_gemm_tile_cap(ENC_BF16, tokens, 1, 0);
-    rc = launch_dense_tiles((int)tokens, s_cap, snt, st, st + pl.s_max_tiles, st + 2 * pl.s_max_tiles, stream);
-    if (rc) return rc;
     GroupedGemmArgs d{};
     d.mode = 0; d.enc = ENC_BF16; d.num_experts = 1; d.n_rows = S; d.k = H;
     d.act = hidden_bf16; d.total_rows = tokens;
     d.w0 = shared->gate; d.w1 = shared->up;
-    d.num_tiles = snt; d.tile_expert = st; d.tile_row0 = st + pl.s_max_tiles; d.tile_rows = st + 2 * pl.s_max_tiles;
-    d.max_tiles = pl.s_max_tiles; d.tile_cap = s_cap;
+    d.num_tiles = sa.dense_num_tiles; d.tile_expert = sa.dense_expert; d.tile_row0 = sa.dense_row0; d.tile_rows = sa.dense_tile_rows;
+    d.max_tiles = pl.s_max_tiles; d.tile_cap = sa.dense_cap;
     d.out = reinterpret_cast<__nv_bfloat16*>(at(pl.s_inter)); d.out_stride = S; d.status = status;
     rc = launch_grouped_gemm(d, stream);
     if (rc) return rc;

@@ -148,12 +148,13 @@ struct SortArgs {
   // optional: rows of x in the k order of the quantised GEMMs, or as digits, written by further CTAs of the first launch
   const __nv_bfloat16* permute_src; __nv_bfloat16* permute_dst; long long permute_chunks;   // 16-byte chunks
   float* digit_scales;             // optional: permute_dst receives digits (digits.cuh) and this their scales [rows, hidden/128]
+  // optional: the tile table of dense_rows rows of a single further expert (the shared one), in tiles of dense_cap
+  int dense_rows, dense_cap;
+  int* dense_num_tiles; int* dense_expert; int* dense_row0; int* dense_tile_rows;
   int* scratch;                    // optional: ceil(routes / 2048) * experts ints let the sort use many CTAs
   long long scratch_ints;
 };
 int launch_route_sort(const SortArgs& a, cudaStream_t stream);
-
-int launch_dense_tiles(int rows, int tile_cap, int* num_tiles, int* tile_expert, int* tile_row0, int* tile_rows, cudaStream_t stream);
 
 // rows of x gathered into sorted order; `permute` writes each run of 8 as [0,4,1,5,2,6,3,7]
 // valid_rows (device, may be null): only the first *valid_rows sorted routes exist

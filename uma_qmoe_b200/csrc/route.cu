@@ -635,6 +635,16 @@ __device__ __forceinline__ void permute_chunk(const SortArgs& a, long long i) {
       make_uint4(prmt(w.x, w.z, 0x5410), prmt(w.x, w.z, 0x7632), prmt(w.y, w.w, 0x5410), prmt(w.y, w.w, 0x7632));
 }
 
+// The shared expert's tiles, in the sort's first launch: a launch of its own costs more than it does (mixed batch of 24 974 -> 969 us).
+__device__ __forceinline__ void dense_tiles(const SortArgs& a, int tid, int nthreads) {
+  if (a.dense_rows <= 0) return;
+  const int tiles = (a.dense_rows + a.dense_cap - 1) / a.dense_cap;
+  for (int t = tid; t < tiles; t += nthreads) {
+    a.dense_expert[t] = 0; a.dense_row0[t] = t * a.dense_cap; a.dense_tile_rows[t] = min(a.dense_cap, a.dense_rows - t * a.dense_cap);
+  }
+  if (tid == 0) *a.dense_num_tiles = tiles;
+}
+
 __global__ void __launch_bounds__(kSortThreads) route_sort_kernel(const SortArgs a) {
   pdl_launch_dependents();
   pdl_wait();
@@ -646,6 +656,7 @@ __global__ void __launch_bounds__(kSortThreads) route_sort_kernel(const SortArgs
   const long long routes = (long long)a.tokens * a.top_k;
   const long long chunk = ((routes + 31) / 32 + 31) / 32 * 32;     // routes per warp, multiple of 32
   const long long begin = min(routes, warp * chunk), end = min(routes, begin + chunk);
+  dense_tiles(a, tid, kSortThreads);
   for (int i = tid; i < 32 * kMaxSortExperts; i += kSortThreads) (&hist[0][0])[i] = 0;
   __syncthreads();
   bool bad = false;
@@ -703,6 +714,7 @@ __global__ void __launch_bounds__(kSortThreads) route_hist_kernel(const SortArgs
   if ((int)blockIdx.x >= chunks) return permute_chunk(a, (long long)(blockIdx.x - chunks) * kSortThreads + threadIdx.x);
   __shared__ int hist[kMaxSortExperts];
   const int tid = threadIdx.x, E = a.experts;
+  if (blockIdx.x == 0) dense_tiles(a, tid, kSortThreads);
   const long long routes = (long long)a.tokens * a.top_k;
   const long long begin = (long long)blockIdx.x * kChunk, end = min(routes, begin + kChunk);
   if (tid < kMaxSortExperts) hist[tid] = 0;
@@ -1049,17 +1061,6 @@ combine_warp_kernel(const __nv_bfloat16* __restrict__ weighted, const void* __re
   }
 }
 
-// tile table of a dense [rows, k] matrix treated as one expert (the Qwen shared expert in prefill)
-__global__ void dense_tiles_kernel(int rows, int cap, int* num_tiles, int* tile_expert, int* tile_row0, int* tile_rows) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int tiles = (rows + cap - 1) / cap;
-  for (int t = threadIdx.x; t < tiles; t += blockDim.x) {
-    tile_expert[t] = 0; tile_row0[t] = t * cap; tile_rows[t] = min(cap, rows - t * cap);
-  }
-  if (threadIdx.x == 0) *num_tiles = tiles;
-}
-
 int check_launch(const char* what, cudaError_t e) {
   if (e == cudaSuccess) return ERR_NONE;
   set_error("%s: launch failed: %s", what, cudaGetErrorString(e));
@@ -1072,11 +1073,6 @@ int check_launch(const char* what) {
 }
 
 }  // namespace
-
-int launch_dense_tiles(int rows, int tile_cap, int* num_tiles, int* tile_expert, int* tile_row0, int* tile_rows, cudaStream_t stream) {
-  return check_launch("dense tiles", launch_chained(dense_tiles_kernel, dim3(1), dim3(256), 0, stream, rows, tile_cap, num_tiles,
-                                                   tile_expert, tile_row0, tile_rows));
-}
 
 int launch_router_topk(const RouterArgs& a, cudaStream_t stream) {
   if (a.tokens <= 0 || a.hidden % 256 || a.experts < a.top_k || a.top_k < 1 || a.top_k > 32 || a.experts > 1024) {
