@@ -316,6 +316,9 @@ router_small_kernel(const RouterArgs a) {
   extern __shared__ __align__(16) uint8_t rs_smem[];
   __shared__ float logit[kRsTokens][kRtExperts + 1];                      // used in CTA 0 of the cluster
   __shared__ double part[kRsWarps][kRsTokens];
+  __shared__ int rank[kRsTokens][4][kRtExperts];                          // per quarter of the experts
+  __shared__ float top_p[kRsTokens][8];
+  __shared__ int top_e[kRsTokens][8];
   const int H = a.hidden, E = a.experts, chunks = H >> 3, half_chunks = chunks >> 1;   // 16-byte chunks
   uint4* xs = reinterpret_cast<uint4*>(rs_smem);                          // [kRsTokens][chunks]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -357,9 +360,11 @@ router_small_kernel(const RouterArgs a) {
   }
 #pragma unroll
   for (int t = 0; t < kRsTokens; ++t) {
+    if (t < nt) {
 #pragma unroll
-    for (int o = 16; o; o >>= 1) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], o);
-    if (lane == 0) part[warp][t] = acc[t];
+      for (int o = 16; o; o >>= 1) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], o);
+      if (lane == 0) part[warp][t] = acc[t];
+    }
   }
   __syncthreads();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -377,12 +382,54 @@ router_small_kernel(const RouterArgs a) {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (cr != 0) return;
   if (a.top_k <= 8) {
-    if (warp == 0) {                                                       // eight lanes per token, four tokens
-      const int r = lane >> 3;
-      const bool live = r < nt;
-      const int t = token0 + (live ? r : 0);
-      softmax_topk_oct(logit[live ? r : 0], live, E, a.top_k, a.renormalize, lane, a.out_weights + (size_t)t * a.top_k,
-                       a.out_indices + (size_t)t * a.top_k);
+    // Four warps per token: each has the probabilities (lane j: experts j and j + 32) and counts how many of its 16 experts come
+    // before them, so that the order of all 64 is there after one exchange instead of top_k rounds of arg-max.  Sums and ties as in
+    // softmax_topk_oct.
+    const int t = warp >> 2, q = warp & 3;
+    float p[2] = {-2.f, -2.f}, sum = 0.f;
+    if (t < nt) {
+      float l[2], mx;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) l[h] = lane + 32 * h < E ? logit[t][lane + 32 * h] : -INFINITY;
+      mx = fmaxf(l[0], l[1]);
+#pragma unroll
+      for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      float v[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) v[h] = lane + 32 * h < E ? expf(l[h] - mx) : 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum += __shfl_sync(0xffffffffu, v[j >> 2], (lane & 7) + 8 * (j & 3));
+#pragma unroll
+      for (int o = 4; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) p[h] = lane + 32 * h < E ? v[h] / sum : -2.f;
+      int before[2] = {0, 0};
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int j = 16 * q + i;
+        const float pj = __shfl_sync(0xffffffffu, q < 2 ? p[0] : p[1], j & 31);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) before[h] += pj > p[h] || (pj == p[h] && j < lane + 32 * h);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) rank[t][q][lane + 32 * h] = before[h];
+    }
+    __syncthreads();
+    if (t < nt && q == 0) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int e = lane + 32 * h, r = rank[t][0][e] + rank[t][1][e] + rank[t][2][e] + rank[t][3][e];
+        if (e < E && r < a.top_k) { top_p[t][r] = p[h]; top_e[t][r] = e; }
+      }
+      __syncwarp();
+      if (lane < a.top_k) {
+        const bool nan = sum != sum;                        // a NaN or an infinite logit: no expert, as in softmax_topk_oct
+        float all = 0.f;
+        for (int r = 0; r < a.top_k; ++r) all += nan ? -1.f : top_p[t][r];
+        const float mine = nan ? -1.f : top_p[t][lane];
+        a.out_weights[(size_t)(token0 + t) * a.top_k + lane] = a.renormalize ? mine / all : mine;
+        a.out_indices[(size_t)(token0 + t) * a.top_k + lane] = nan ? 0x7fffffff : top_e[t][lane];
+      }
     }
   } else if (warp < nt) {
     const int t = token0 + warp;
