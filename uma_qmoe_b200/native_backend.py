@@ -357,6 +357,8 @@ class MixedTargetNativeBackend:
         layer.used_on(stream, device)
         flat = flat.contiguous()
         out = torch.empty_like(flat)
+        if tokens == 0 and router is not None:
+            ops.route_topk(flat, *router)     # refuses it: a router has no empty result
         if tokens == 0:                       # an empty batch has an empty result; there is nothing to launch
             return out.reshape(hidden_states.shape)
         slot = self._workspace("decode" if tokens == 1 else "prefill", layer, tokens, top_k, shared, device, stream)
