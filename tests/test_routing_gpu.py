@@ -1,9 +1,9 @@
-"""The small router's ranking against the chunked kernel's."""
+"""The small router's ranking against the chunked kernel's, and the sort around its change-overs."""
 
 import pytest
 import torch
 
-from uma_qmoe_b200 import ops
+from uma_qmoe_b200 import _native, ops
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -31,3 +31,28 @@ def test_small_router_ranks_as_the_chunked_one(experts, top_k):
     keep = torch.tensor([0, 1, 2, 3, 5], device=DEV)
     assert torch.equal(idx[keep], clean[1][keep]) and torch.equal(w[keep], clean[0][keep])
     assert (idx[4] == 0x7fffffff).all() and (w[4] == -1).all()
+
+
+@pytest.mark.parametrize("tokens,top_k,experts", [(1, 1, 1), (128, 8, 64), (1025, 1, 60), (512, 8, 64),
+                                                  (2048, 8, 64), (2049, 8, 7), (5000, 4, 128)])
+def test_sort_in_one_launch_and_in_two(tokens, top_k, experts):
+    """Around a CTA's 1024 routes, at the change-over to two launches, and beyond it without scratch (one launch then)."""
+    gen = torch.Generator(device=DEV).manual_seed(tokens)
+    idx = torch.randint(-1, experts, (tokens, top_k), device=DEV, generator=gen)
+    w = torch.rand(tokens, top_k, device=DEV, generator=gen)
+    many = ops.route_sort(idx, w, experts)
+    flat = idx.reshape(-1)
+    order = torch.where(flat < 0, experts, flat).sort(stable=True).indices[:int((flat >= 0).sum())]
+    n = len(order)
+    assert torch.equal(many.sorted_route[:n].long(), order) and torch.equal(many.sorted_weight[:n], w.reshape(-1)[order])
+    one = ops.SortedRoutes(*(torch.zeros_like(t) if torch.is_tensor(t) else t for t in vars(many).values()))
+    code = _native.lib().umaq_route_sort(
+        idx.data_ptr(), 1, w.data_ptr(), tokens, top_k, experts, one.counts.data_ptr(), one.offsets.data_ptr(),
+        one.sorted_route.data_ptr(), one.route_pos.data_ptr(), one.sorted_weight.data_ptr(), one.num_tiles.data_ptr(),
+        one.tile_table.data_ptr(), one.max_tiles, one.status.data_ptr(), None, 0, torch.cuda.current_stream().cuda_stream)
+    assert code == 0
+    tiles = int(one.num_tiles)
+    assert torch.equal(one.counts, many.counts) and torch.equal(one.offsets, many.offsets) and tiles == int(many.num_tiles)
+    assert torch.equal(one.sorted_route[:n], many.sorted_route[:n]) and torch.equal(one.route_pos, many.route_pos)
+    assert torch.equal(one.tile_table.view(3, -1)[:, :tiles], many.tile_table.view(3, -1)[:, :tiles])
+    assert int(one.status) == 0 and int(many.status) == 0

@@ -575,10 +575,10 @@ __global__ void __launch_bounds__(256) router_mma_kernel(const RouterArgs a) {
   }
 }
 
-// ---- stable expert sort of the routes, one CTA --------------------------------------------------------
-// Route i = token * top_k + slot.  Warp w owns a contiguous chunk of routes; a per-warp histogram and
-// a scan over (expert, warp) give every warp its first position inside each expert's run, and ranks
-// inside a 32-route batch come from __match_any_sync, so equal experts keep their route order.
+// ---- stable expert sort of the routes -------------------------------------------------------------------
+// Route i = token * top_k + slot.  A CTA places 1024 of them, one per thread, and counts them all (a few loads per thread, all in
+// flight at once), so that no CTA needs another's result: routes before its own, per-warp histograms of its own with a scan over
+// (expert, warp), and ranks inside a warp from __match_any_sync, so equal experts keep their route order.
 constexpr int kSortThreads = 1024;
 constexpr int kMaxSortExperts = 128;
 
@@ -692,59 +692,68 @@ __device__ __forceinline__ void dense_tiles(const SortArgs& a, int tid, int nthr
   if (tid == 0) *a.dense_num_tiles = tiles;
 }
 
-__global__ void __launch_bounds__(kSortThreads) route_sort_kernel(const SortArgs a) {
+// Up to this many routes by one launch (2048 tokens x 8); above, where counting everything 16 times costs more than a second
+// launch, by the two kernels below.  The 512-token prompt (4096 routes, before: one CTA, four routes per lane one after the other)
+// 575 -> 566 us, 1531 tokens (6124 routes, before: two launches) 1488 -> 1480.
+constexpr long long kSortOneLaunch = 16384;
+constexpr int kHistPitch = kMaxSortExperts + 1;                        // a scan over the warps of one expert reads 32 banks
+__global__ void __launch_bounds__(kSortThreads, 2) route_sort_kernel(const SortArgs a, int sort_ctas) {
   pdl_launch_dependents();
+  __shared__ int hist[32][kHistPitch];          // per-warp counts of this CTA's routes, then the position inside them
+  __shared__ int total[kMaxSortExperts + 1];    // all routes of an expert
+  __shared__ int before[kMaxSortExperts];       // those ahead of this CTA's
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, E = a.experts;
+  if ((int)blockIdx.x < sort_ctas) {
+    for (int i = tid; i < 32 * kHistPitch; i += kSortThreads) (&hist[0][0])[i] = 0;
+    if (tid < kMaxSortExperts) total[tid] = before[tid] = 0;
+  }
   pdl_wait();
-  if (blockIdx.x > 0) return permute_chunk(a, (long long)(blockIdx.x - 1) * kSortThreads + threadIdx.x);
-  __shared__ int hist[32][kMaxSortExperts];     // per-warp counts, then per-warp running positions
-  __shared__ int total[kMaxSortExperts + 1];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int E = a.experts;
-  const long long routes = (long long)a.tokens * a.top_k;
-  const long long chunk = ((routes + 31) / 32 + 31) / 32 * 32;     // routes per warp, multiple of 32
-  const long long begin = min(routes, warp * chunk), end = min(routes, begin + chunk);
-  dense_tiles(a, tid, kSortThreads);
-  for (int i = tid; i < 32 * kMaxSortExperts; i += kSortThreads) (&hist[0][0])[i] = 0;
+  if ((int)blockIdx.x >= sort_ctas) return permute_chunk(a, (long long)(blockIdx.x - sort_ctas) * kSortThreads + tid);
+  const long long routes = (long long)a.tokens * a.top_k, begin = (long long)blockIdx.x * kSortThreads, i = begin + tid;
+  const bool live = i < routes;
+  int mine = live ? load_expert(a.indices, a.idx64, i) : -1;
+  const float weight = live ? a.weights[i] : 0.f;
+  if (blockIdx.x == 0) dense_tiles(a, tid, kSortThreads);
   __syncthreads();
-  bool bad = false;
-  for (long long i = begin + lane; i < end; i += 32) {
-    const int e = load_expert(a.indices, a.idx64, i);
-    if (e == -1) continue;                       // an absent route (padding of a fixed-capacity exchange)
-    if (e < 0 || e >= E) bad = true; else atomicAdd(&hist[warp][e], 1);
-  }
-  if (bad) atomicExch(a.status, (unsigned)ERR_BAD_ARGUMENT);
-  __syncthreads();
-  // per expert: exclusive scan over the warps; totals
-  if (tid < E) {
-    int run = 0;
-    for (int w = 0; w < 32; ++w) { const int c = hist[w][tid]; hist[w][tid] = run; run += c; }
-    total[tid] = run;
-    a.counts[tid] = run;
-  }
-  __syncthreads();
-  __shared__ int start[kMaxSortExperts + 1], tile_base[kMaxSortExperts + 1];
-  emit_offsets_and_tiles(a, total, start, tile_base, true, tid, kSortThreads);
-  __syncthreads();
-  if (tid < E) total[tid] = start[tid];
-  __syncthreads();
-  for (long long base = begin; base < end; base += 32) {
-    const long long i = base + lane;
-    const bool live = i < end;
-    int e = live ? load_expert(a.indices, a.idx64, i) : -1 - lane;     // distinct keys for idle lanes
-    if (live && (e < 0 || e >= E)) { e = -1 - lane; }
-    const unsigned peers = __match_any_sync(0xffffffffu, e);
-    const int rank = __popc(peers & ((1u << lane) - 1u));
-    if (e >= 0) {
-      const int pos = total[e] + hist[warp][e] + rank;
-      a.sorted_route[pos] = (int)i;
-      a.route_pos[i] = pos;
-      a.sorted_weight[pos] = a.weights[i];
-    } else if (live) {
-      a.route_pos[i] = -1;                       // absent or invalid route: no row, the combine skips it
+  const bool alone = sort_ctas == 1;             // its own routes are all there are
+  bool bad = mine < -1 || mine >= E;             // -1: an absent route (padding of a fixed-capacity exchange)
+  if (!alone) {
+#pragma unroll 4
+    for (long long j = tid; j < routes; j += kSortThreads) {
+      const int e = load_expert(a.indices, a.idx64, j);
+      if (e < 0 || e >= E) { bad |= e != -1; continue; }
+      atomicAdd(&total[e], 1);
+      if (j < begin) atomicAdd(&before[e], 1);
     }
-    __syncwarp();
-    if (e >= 0 && rank == 0) hist[warp][e] += __popc(peers);
-    __syncwarp();
+  }
+  if (bad && blockIdx.x == 0) atomicExch(a.status, (unsigned)ERR_BAD_ARGUMENT);
+  if (mine < 0 || mine >= E) mine = -1 - lane;   // no expert: distinct keys
+  const unsigned peers = __match_any_sync(0xffffffffu, mine);
+  const int rank = __popc(peers & ((1u << lane) - 1u));
+  if (mine >= 0 && rank == 0) hist[warp][mine] = __popc(peers);
+  __syncthreads();
+  for (int e = warp; e < E; e += 32) {           // exclusive scan over the warps
+    const int v = hist[lane][e];
+    int in = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, in, o);
+      if (lane >= o) in += up;
+    }
+    hist[lane][e] = in - v;
+    if (alone && lane == 31) total[e] = in;
+  }
+  if (alone) __syncthreads();
+  if (blockIdx.x == 0 && tid < E) a.counts[tid] = total[tid];
+  __shared__ int start[kMaxSortExperts + 1], tile_base[kMaxSortExperts + 1];
+  emit_offsets_and_tiles(a, total, start, tile_base, blockIdx.x == 0, tid, kSortThreads);     // its barrier comes after the scans
+  if (mine >= 0) {
+    const int pos = start[mine] + before[mine] + hist[warp][mine] + rank;
+    a.sorted_route[pos] = (int)i;
+    a.route_pos[i] = pos;
+    a.sorted_weight[pos] = weight;
+  } else if (live) {
+    a.route_pos[i] = -1;                         // absent or invalid route: no row, the combine skips it
   }
 }
 
@@ -1175,8 +1184,9 @@ int launch_route_sort(const SortArgs& a, cudaStream_t stream) {
   const long long routes = (long long)a.tokens * a.top_k;
   const int chunks = (int)((routes + kChunk - 1) / kChunk);
   const unsigned permute_blocks = a.permute_dst ? (unsigned)((a.permute_chunks + kSortThreads - 1) / kSortThreads) : 0;
-  if (chunks <= 2 || !a.scratch || a.scratch_ints < (long long)chunks * a.experts) {
-    return check_launch("route sort", launch_chained(route_sort_kernel, dim3(1 + permute_blocks), dim3(kSortThreads), 0, stream, a));
+  if (routes <= kSortOneLaunch || !a.scratch || a.scratch_ints < (long long)chunks * a.experts) {
+    const unsigned ctas = (unsigned)((routes + kSortThreads - 1) / kSortThreads);
+    return check_launch("route sort", launch_chained(route_sort_kernel, dim3(ctas + permute_blocks), dim3(kSortThreads), 0, stream, a, (int)ctas));
   }
   const int rc = check_launch("route sort", launch_chained(route_hist_kernel, dim3(chunks + permute_blocks), dim3(kSortThreads), 0,
                                                             stream, a, a.scratch, chunks));
