@@ -151,7 +151,7 @@ struct SortArgs {
   // optional: the tile table of dense_rows rows of a single further expert (the shared one), in tiles of dense_cap
   int dense_rows, dense_cap;
   int* dense_num_tiles; int* dense_expert; int* dense_row0; int* dense_tile_rows;
-  int* scratch;                    // optional: ceil(routes / 2048) * experts ints let the sort use many CTAs
+  int* scratch;                    // optional: ceil(routes / 2048) * experts ints for sorts of more than 16,384 routes in two launches
   long long scratch_ints;
 };
 int launch_route_sort(const SortArgs& a, cudaStream_t stream);
