@@ -9,7 +9,6 @@
 #include "common.cuh"
 #include "aux.cuh"
 #include "decode.cuh"
-#include "digits.cuh"
 #include "grouped.cuh"
 
 namespace umaq {
@@ -261,7 +260,7 @@ int umaq_combine_routes(const void* weighted_bf16, const void* expert_indices, i
 
 namespace {
 struct PrefillPlan {
-  size_t status, counts, offsets, num_tiles, tiles, sort_scratch, sorted_route, route_pos, sorted_weight, xs, inter, yw, xs_scales, inter_scales;
+  size_t status, counts, offsets, num_tiles, tiles, sort_scratch, sorted_route, route_pos, sorted_weight, xs, inter, yw;
   long long sort_ints;
   size_t s_num_tiles, s_tiles, s_inter, s_out, s_part, total;
   int max_tiles, s_max_tiles;
@@ -287,8 +286,6 @@ PrefillPlan prefill_plan(long long tokens, int top_k, int experts, int hidden, i
   p.xs = take(routes * hidden * 2);
   p.inter = take(routes * inter * 2);
   p.yw = take(routes * hidden * 2);
-  p.xs_scales = take((size_t)tokens * (hidden / kDigitGroup) * 4);
-  p.inter_scales = take(routes * (inter / kDigitGroup) * 4);
   if (shared_inter) {
     p.s_num_tiles = take(4);
     p.s_tiles = take((size_t)p.s_max_tiles * 12);
@@ -311,7 +308,7 @@ size_t umaq_prefill_workspace_bytes(long long tokens, int top_k, int num_experts
 static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* shared, const void* hidden_bf16,
                         const void* expert_indices, int indices_are_int64, const float* routing_weights, long long tokens,
                         int top_k, void* out_bf16, void* workspace, size_t workspace_bytes, void* stream_,
-                        const SegmentedOut* segments, bool rows_k_permuted = false, bool digits = false, unsigned* host_status = nullptr) {
+                        const SegmentedOut* segments, bool rows_k_permuted = false, unsigned* host_status = nullptr) {
   if (!layer || !hidden_bf16 || !expert_indices || !routing_weights || (!out_bf16 && !segments) || !workspace || tokens <= 0) {
     set_error("umaq_moe_prefill: null argument");
     return ERR_BAD_ARGUMENT;
@@ -334,8 +331,6 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   int* tiles = reinterpret_cast<int*>(at(pl.tiles));
   const long long routes = tokens * top_k;
   const int quant = layer->encoding != ENC_BF16;
-  const bool by_digits = digits && !segments && grouped_gemm_takes_digits(layer->encoding, tokens, top_k, E, H, I) &&
-                         !(reinterpret_cast<uintptr_t>(hidden_bf16) & 15);
 
   SortArgs sa{};
   sa.indices = expert_indices; sa.idx64 = indices_are_int64; sa.weights = routing_weights;
@@ -346,10 +341,8 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   sa.num_tiles = reinterpret_cast<int*>(at(pl.num_tiles));
   sa.tile_expert = tiles; sa.tile_row0 = tiles + pl.max_tiles; sa.tile_rows = tiles + 2 * pl.max_tiles;
   sa.max_tiles = pl.max_tiles; sa.tile_cap = grouped_gemm_tile_cap(layer->encoding, routes, E, 0); sa.status = status;
-  const bool wide = !by_digits && grouped_gemm_takes_wide(layer->encoding, routes, E, H, I);
-  if (by_digits) {
-    sa.tile_cap = kTileCapMin;
-  } else if (wide) {
+  const bool wide = grouped_gemm_takes_wide(layer->encoding, routes, E, H, I);
+  if (wide) {
     sa.tile_cap = kTileCapWide;
   } else if (grouped_gemm_choice_on_device(layer->encoding, routes, E, tokens, 0)) {
     sa.use_ts = reinterpret_cast<int*>(at(pl.status) + 64);
@@ -375,7 +368,6 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
     sa.permute_src = static_cast<const __nv_bfloat16*>(hidden_bf16);
     sa.permute_dst = xs;
     sa.permute_chunks = tokens * (H / 8);
-    if (by_digits) sa.digit_scales = reinterpret_cast<float*>(at(pl.xs_scales));
   }
   int rc = launch_route_sort(sa, stream);
   if (rc) return rc;
@@ -402,22 +394,13 @@ static int prefill_impl(const umaq_layer* layer, const umaq_shared_expert* share
   down.out = reinterpret_cast<__nv_bfloat16*>(at(pl.yw)); down.out_stride = H; down.route_weight = sa.sorted_weight; down.permute_out = 0;
   // Where the sort picks the kernel: both GEMMs on transposed tiles, then both on one-CTA tiles.  The pair that is not wanted
   // returns, and in this order it stands between no two kernels that work.
-  if (by_digits) {
-    g.act_scales = sa.digit_scales;
-    g.out_scales = reinterpret_cast<float*>(at(pl.inter_scales));
-    down.act_scales = g.out_scales;
-    rc = launch_grouped_gemm_digits(g, stream);
-    if (rc) return rc;
-    rc = launch_grouped_gemm_digits(down, stream);
-    if (rc) return rc;
-  }
   if (wide) {
     rc = launch_grouped_gemm_wide(g, stream);
     if (rc) return rc;
     rc = launch_grouped_gemm_wide(down, stream);
     if (rc) return rc;
   }
-  for (int conditional = sa.use_ts ? 1 : 0; !wide && !by_digits && conditional <= (sa.use_ts ? 2 : 0); ++conditional) {
+  for (int conditional = sa.use_ts ? 1 : 0; !wide && conditional <= (sa.use_ts ? 2 : 0); ++conditional) {
     g.conditional = down.conditional = conditional;
     if (conditional) g.tile_cap = down.tile_cap = conditional == 1 ? kTileCapMin : kTileCapMax;
     rc = launch_grouped_gemm(g, stream);
@@ -461,13 +444,6 @@ int umaq_moe_prefill(const umaq_layer* layer, const umaq_shared_expert* shared, 
                       out_bf16, workspace, workspace_bytes, stream_, nullptr);
 }
 
-int umaq_moe_prefill_digits(const umaq_layer* layer, const umaq_shared_expert* shared, const void* hidden_bf16,
-                            const void* expert_indices, int indices_are_int64, const float* routing_weights, long long tokens,
-                            int top_k, void* out_bf16, void* workspace, size_t workspace_bytes, void* stream_) {
-  return prefill_impl(layer, shared, hidden_bf16, expert_indices, indices_are_int64, routing_weights, tokens, top_k,
-                      out_bf16, workspace, workspace_bytes, stream_, nullptr, false, true);
-}
-
 int umaq_moe_step(const umaq_layer* layer, const umaq_shared_expert* shared, const void* hidden_bf16, const void* router_weight_bf16,
                   int router_experts, int renormalize, void* expert_indices, int indices_are_int64, float* routing_weights,
                   long long tokens, int top_k, void* out_bf16, void* workspace, size_t workspace_bytes, unsigned* host_status,
@@ -483,7 +459,7 @@ int umaq_moe_step(const umaq_layer* layer, const umaq_shared_expert* shared, con
   rc = tokens == 1 ? decode_impl(layer, shared, hidden_bf16, expert_indices, indices_are_int64, routing_weights, top_k, out_bf16,
                                  workspace, workspace_bytes, host_status, stream)
                    : prefill_impl(layer, shared, hidden_bf16, expert_indices, indices_are_int64, routing_weights, tokens, top_k,
-                                  out_bf16, workspace, workspace_bytes, stream, nullptr, false, true, host_status);
+                                  out_bf16, workspace, workspace_bytes, stream, nullptr, false, host_status);
   if (rc) return rc;
   if (event) {
     const cudaError_t e = cudaEventRecord(static_cast<cudaEvent_t>(event), static_cast<cudaStream_t>(stream));

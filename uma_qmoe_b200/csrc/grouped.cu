@@ -652,14 +652,6 @@ TileChoice grouped_gemm_choice(int enc, int inter, int hidden) {
   c.den = enc == ENC_Q4 ? 1 : enc == ENC_Q8 ? 5 : 4;
   return c;
 }
-// Q8 layers of a batch: integer digits of the activations (grouped_digits.cu), up to the tokens that need no choice on the device
-// (from there on the transposed and the wide kernel are as fast: OLMoE, us, digits | BF16: 96 tokens 102 | 114, 192: 121 | 124,
-// 512: 200 | 187).  Its 256-row tiles want 1.5 tiles for each SM, of the routes at hand (each may be another expert's) and of the
-// weights that there are: below that the 128-row tiles of the transposed kernel spread better.
-bool grouped_gemm_takes_digits(int enc, long long tokens, int top_k, int experts, int hidden, int inter) {
-  if (enc != ENC_Q8 || hidden % 256 || inter % 128 || hidden > 2048 || inter > 2048 || tokens > kChoiceMinRoutes) return false;
-  return 2 * std::min(tokens * top_k, (long long)experts) * (inter / 128) >= 3 * dense_sms();
-}
 bool grouped_gemm_can_gather(const GroupedGemmArgs& a) { return a.mode == 0 && !takes_pair_kernel(a); }
 int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream) {
   if (takes_pair_kernel(a)) {

@@ -50,9 +50,7 @@ struct GroupedParams {
   // is row gather_route[r] / gather_top_k of gather_src ([tokens, k] BF16, k already in the order the encoding wants)
   const int* gather_route;
   int gather_top_k;
-  const __nv_bfloat16* gather_src;                 // grouped_digits.cu: digits, [rows][groups][hi 128 | lo 128] bytes
-  const float* act_scales;    // grouped_digits.cu: [rows of gather_src, k/128]
-  float* out_scales;          // grouped_digits.cu, mode 0: [routes, n_rows/128], `out` being digits
+  const __nv_bfloat16* gather_src;
   // 1: this launch runs if transposed tiles are wanted, 2: if one-CTA tiles are, 0: always.  The answer is *use_ts, or
   // follows from the tile table (entries of up to 256 routes) where use_ts is null
   int conditional;
@@ -90,9 +88,6 @@ struct GroupedGemmArgs {
   // for sorted route r itself (no gathered copy of the activations)
   const int* gather_route;
   int gather_top_k;
-  // grouped_digits.cu: `act` (and in mode 0 `out`) are digits, these their scales
-  const float* act_scales;
-  float* out_scales;
 };
 
 // true if launch_grouped_gemm would run the kernel that can fetch its activation rows by index
@@ -102,7 +97,6 @@ int launch_grouped_gemm(const GroupedGemmArgs& a, cudaStream_t stream);        /
 int launch_grouped_gemm_single(const GroupedGemmArgs& a, cudaStream_t stream);
 int launch_grouped_gemm_pair(const GroupedGemmArgs& a, cudaStream_t stream);
 int launch_grouped_gemm_ts(const GroupedGemmArgs& a, cudaStream_t stream);
-int launch_grouped_gemm_digits(const GroupedGemmArgs& a, cudaStream_t stream);   // only when asked for: its operands are digits
 int launch_grouped_gemm_wide(const GroupedGemmArgs& a, cudaStream_t stream);   // only when asked for: the table is cut for it
 
 // Whether both GEMMs of a quantised layer run on wide transposed tiles (grouped_wide.cu), the sort cutting its table for them
@@ -112,8 +106,6 @@ int grouped_gemm_tile_cap(int enc, long long rows, int num_experts, int variant)
 // Whether that pick has to be made on the device, from the routes that the experts have; `most`: the most one can have
 bool grouped_gemm_choice_on_device(int enc, long long rows, int num_experts, long long most, int variant);
 TileChoice grouped_gemm_choice(int enc, int inter, int hidden);
-// Whether a layer's GEMMs may run on integer digits of the activations (grouped_digits.cu)
-bool grouped_gemm_takes_digits(int enc, long long tokens, int top_k, int experts, int hidden, int inter);
 // Parts the contraction of a dense BF16 down GEMM (the shared expert's) is cut into
 int grouped_gemm_dense_splits(long long rows, int n_rows, int k);
 // ... and the room they need, in rows of n_rows float32 sums, for every call of up to `rows` rows (0: never more than one part)
@@ -145,9 +137,8 @@ struct SortArgs {
   int tile_cap;                    // routes per tile, unless use_ts is given
   int* use_ts; TileChoice choice;  // optional: the sort picks the kernel, cuts the table for it and writes 1 (transposed) or 0
   unsigned* status;
-  // optional: rows of x in the k order of the quantised GEMMs, or as digits, written by further CTAs of the first launch
+  // optional: rows of x in the k order of the quantised GEMMs, written by further CTAs of the first launch
   const __nv_bfloat16* permute_src; __nv_bfloat16* permute_dst; long long permute_chunks;   // 16-byte chunks
-  float* digit_scales;             // optional: permute_dst receives digits (digits.cuh) and this their scales [rows, hidden/128]
   // optional: the tile table of dense_rows rows of a single further expert (the shared one), in tiles of dense_cap
   int dense_rows, dense_cap;
   int* dense_num_tiles; int* dense_expert; int* dense_row0; int* dense_tile_rows;

@@ -9,7 +9,6 @@
 #include <cstdlib>
 
 #include "common.cuh"
-#include "digits.cuh"
 
 namespace umaq {
 namespace {
@@ -646,36 +645,9 @@ __device__ __forceinline__ void emit_offsets_and_tiles(const SortArgs& a, const 
   }
 }
 
-// The same rows as digits (digits.cuh): half a warp takes a group of 128, 16 bytes of x per lane.
-__device__ __forceinline__ void digits_chunk(const SortArgs& a, long long i) {
-  const bool live = i < a.permute_chunks;          // the same for the lanes of a half: rows are whole groups
-  const uint4 w = live ? reinterpret_cast<const uint4*>(a.permute_src)[i] : make_uint4(0, 0, 0, 0);
-  const uint32_t v[4] = {w.x, w.y, w.z, w.w};
-  uint32_t top = 0;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) top = max(top, max((v[j] << 16) & 0x7fff0000u, v[j] & 0x7fff0000u));
-#pragma unroll
-  for (int o = 8; o; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
-  const DigitScale ds = digit_scale(top);
-  uint32_t hi[2] = {0, 0}, lo[2] = {0, 0};
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    int h, l;
-    to_digits(__uint_as_float(j & 1 ? v[j >> 1] & 0xffff0000u : v[j >> 1] << 16), ds.to_int, h, l);
-    hi[j >> 2] |= (uint32_t)(h & 255) << (8 * (j & 3));
-    lo[j >> 2] |= (uint32_t)(l & 255) << (8 * (j & 3));
-  }
-  if (!live) return;
-  uint8_t* dst = reinterpret_cast<uint8_t*>(a.permute_dst) + (i >> 4) * (2 * kDigitGroup) + (i & 15) * 8;
-  *reinterpret_cast<uint2*>(dst) = make_uint2(hi[0], hi[1]);
-  *reinterpret_cast<uint2*>(dst + kDigitGroup) = make_uint2(lo[0], lo[1]);
-  if ((i & 15) == 0) a.digit_scales[i >> 4] = ds.to_value;
-}
-
 // Rows of x in the k order of the quantised GEMMs ([k0,k4,k1,k5,k2,k6,k3,k7] in every run of 8), 16 bytes per thread: the
 // sort needs one CTA (or a few), the rest of the device does this beside it instead of in a launch of its own.
 __device__ __forceinline__ void permute_chunk(const SortArgs& a, long long i) {
-  if (a.digit_scales) return digits_chunk(a, i);
   if (i >= a.permute_chunks) return;
   const uint4 w = reinterpret_cast<const uint4*>(a.permute_src)[i];
   reinterpret_cast<uint4*>(a.permute_dst)[i] =

@@ -20,7 +20,7 @@ neighbouring expert ids similar popularity and a contiguous split then overloads
 Three exchange schemes share the placement and the kernels:
 
 * :meth:`ExpertParallelMoE.forward` -- exact row counts (one host read per call), routes travel one by
-  one; bit-identical to the single-GPU path on the BF16 kernels (``moe_prefill(..., digits=False)``) for any G.
+  one; bit-identical to the single-GPU path for any G.
 * :meth:`ExpertParallelMoE.forward_fixed` -- the same routes in fixed-capacity segments, no host read.
 * :meth:`ExpertParallelMoE.forward_gather` -- for dense routing (top-8 of 64 over a few ranks reaches
   every rank from almost every token): all-gather the token rows once, every rank runs its own experts
@@ -75,7 +75,7 @@ class CudaKernels:
         if self._ws_rows < n:                   # grow-only: the received row count changes every call
             self._ws_rows = n + n // 4
             self._ws = self.ops.prefill_workspace(self.layer, self._ws_rows, 1, None, rows.device)
-        return self.ops.moe_prefill(self.layer, rows, local_expert.view(n, 1), weight.view(n, 1), self._ws, digits=False)
+        return self.ops.moe_prefill(self.layer, rows, local_expert.view(n, 1), weight.view(n, 1), self._ws)
 
     def combine(self, weighted: torch.Tensor, indices: torch.Tensor, route_pos: torch.Tensor) -> torch.Tensor:
         return self.ops.combine_routes(weighted, indices, route_pos)
@@ -119,7 +119,7 @@ class CudaKernels:
         if self._ws_moe is None or self._ws_moe_shape != (n, top_k):
             self._ws_moe = self.ops.prefill_workspace(self.layer, n, top_k, None, x.device)
             self._ws_moe_shape = (n, top_k)
-        return self.ops.moe_prefill(self.layer, x, local_indices, weights, self._ws_moe, digits=False)
+        return self.ops.moe_prefill(self.layer, x, local_indices, weights, self._ws_moe)
 
 
 class PeerExchange:

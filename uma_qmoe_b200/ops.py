@@ -131,12 +131,8 @@ def prefill_workspace(layer: DeviceLayer, tokens: int, top_k: int, shared: Optio
 
 def moe_prefill(layer: DeviceLayer, hidden: torch.Tensor, indices: torch.Tensor, weights: torch.Tensor,
                 workspace: torch.Tensor, shared: Optional[DeviceSharedExpert] = None,
-                out: Optional[torch.Tensor] = None, digits: bool = True) -> torch.Tensor:
-    """[tokens, H] through the routed experts (and the Qwen shared expert) on the tensor cores.
-
-    ``digits``: whether a Q8 layer may run on integer digits of the activations instead of BF16-rounded weights
-    (``umaq_moe_prefill_digits``: up to 192 tokens, closer to the exact sums, other bits).  Without them a token's bits are the
-    same whichever kernel runs, on any number of ranks."""
+                out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """[tokens, H] through the routed experts (and the Qwen shared expert) on the tensor cores."""
     _require_cuda_bf16(hidden, "hidden_states")
     flat = hidden.reshape(-1, hidden.shape[-1])
     tokens = flat.shape[0]
@@ -150,8 +146,7 @@ def moe_prefill(layer: DeviceLayer, hidden: torch.Tensor, indices: torch.Tensor,
         raise RuntimeError("routes must be contiguous")
     if out is None:
         out = torch.empty_like(flat)
-    native = _native.lib()
-    code = (native.umaq_moe_prefill_digits if digits else native.umaq_moe_prefill)(
+    code = _native.lib().umaq_moe_prefill(
         C.byref(layer.struct()), C.byref(shared.struct()) if shared is not None else None, flat.data_ptr(),
         indices.data_ptr(), int(indices.dtype == torch.int64), weights.data_ptr(), tokens, indices.shape[1],
         out.data_ptr(), workspace.data_ptr(), workspace.numel(), _stream(hidden.device))
