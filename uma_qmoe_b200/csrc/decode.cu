@@ -89,27 +89,14 @@ __device__ __forceinline__ void cp_async8(void* dst_smem, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
 }
 
-// try_wait with a suspend-time hint: the warp sleeps in hardware until the phase completes (or the hint
-// runs out) instead of re-issuing the test -- waiting warps must not take issue slots and shared-memory
-// pipe cycles from the producer warp that shares their scheduler.
-__device__ __forceinline__ bool mbar_try_wait_suspended(uint64_t* bar, uint32_t parity, uint32_t hint_ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(hint_ns)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait that also gives up when another warp of the CTA has already failed.
+// Bounded wait of a whole warp that also gives up when another warp of the CTA has already failed; one answer for all lanes
+// (common.cuh says why).
 __device__ __forceinline__ bool wait_or_fail(uint64_t* bar, uint32_t parity, volatile int* fail) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   const long long t0 = clock64();                 // the SM's own counter: cheap to read
   for (;;) {
-    if (mbar_try_wait_suspended(bar, parity, 100000u)) return true;
-    if (*fail || clock64() - t0 > kDecodeWaitCycles) { *fail = 1; return false; }
+    if (__all_sync(0xffffffffu, mbar_try_wait_suspended(bar, parity, 100000u))) return true;
+    if (__any_sync(0xffffffffu, *fail || clock64() - t0 > kDecodeWaitCycles)) { *fail = 1; return false; }
   }
 }
 
@@ -677,7 +664,7 @@ __global__ void __maxnreg__(64) decode_gateup_kernel(const DecodeParams p) {
     // Issuing a bulk copy costs a warp about 100 ns, so the stages go round the producer warps.
     const int pj = warp - ncons;
     int n = 0;                                 // running stage number: slot n % stages, round n / stages
-    for (int u = ub; u < ue && !*fail; ++u) {
+    for (int u = ub; u < ue && !warp_sees(fail); ++u) {
       const int k = u < U0 ? 0 : 1;
       const DecodeKind& K = P.kind[k];
       const uint8_t *gsrc, *usrc;
@@ -1043,7 +1030,7 @@ __global__ void __maxnreg__(96) decode_down_kernel(const DecodeParams p) {
       }
     } else {
       int n = 0;                               // running stage number; the stages go round the producer warps
-      for (int k = 0; k < kinds && !*fail; ++k) {
+      for (int k = 0; k < kinds && !warp_sees(fail); ++k) {
         const DecodeKind& K = P.kind[k];
         const uint32_t sbytes = 2u * K.groups * 4;
         for (int rp = rp0; rp < rp1; ++rp, ++n) {
@@ -1160,10 +1147,10 @@ __global__ void __maxnreg__(96) decode_down_kernel(const DecodeParams p) {
     Ring ring{0, 0, 0};
     float* red = reinterpret_cast<float*>(smem + P.red_off);
     const bool skip = (p.debug & 1) != 0;
-    if (!s_fail && fast) {
+    if (fast) {                    // after a failed wait as well: every lane takes the same way, nothing of it is used
       if (P.kind[0].enc == ENC_Q4) down_resident<ENC_Q4>(P, P.kind[0], npairs, smem_base, full, red, fail, warp, lane, skip, sreg);
       else down_resident<ENC_Q8>(P, P.kind[0], npairs, smem_base, full, red, fail, warp, lane, skip, sreg);
-    } else if (!s_fail) {
+    } else {
       if (P.kind[0].enc == ENC_Q4) down_pairs<ENC_Q4>(P, P.kind[0], npairs, smem_base, full, empty, red, ring, fail, warp, lane, skip, ncons);
       else if (P.kind[0].enc == ENC_Q8) down_pairs<ENC_Q8>(P, P.kind[0], npairs, smem_base, full, empty, red, ring, fail, warp, lane, skip, ncons);
       else down_pairs<ENC_BF16>(P, P.kind[0], npairs, smem_base, full, empty, red, ring, fail, warp, lane, skip, ncons);

@@ -163,7 +163,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       uint32_t kidx = 0;
       int inflight_from = 0;
       for (int it = first; it < total; it += step) {
-        if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+        if (warp_sees(abort_flag)) break;
         const TileInfo t = tile_of(it);
         const bool two = t.nrows > BM;
         const long long wrow0 = weight_row(t);
@@ -203,7 +203,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       uint32_t kidx = 0;
       int seq = 0;
       for (int it = first; it < total; it += step, ++seq) {
-        if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+        if (warp_sees(abort_flag)) break;
         const TileInfo t = tile_of(it);
         const long long wrow0 = weight_row(t);
         const int sb = seq & 1;
@@ -291,16 +291,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       uint32_t kidx = 0;
       int seq = 0;
       for (int it = first; it < total; it += step, ++seq) {
-        if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+        if (warp_sees(abort_flag)) break;
         const TileInfo t = tile_of(it);
         const bool two = t.nrows > BM;
-        bool ok = seq == 0 || mbar_wait(&sh.acc_empty, (seq - 1) & 1);
+        bool ok = seq == 0 || mbar_wait_warp(&sh.acc_empty, (seq - 1) & 1);
         for (int kc = t.k0; kc < t.k1; ++kc, ++kidx) {
           const uint32_t s = kidx % kInStages;
           const uint32_t sb = ENC == ENC_BF16 ? s : kidx % kBStages;
-          ok = ok && mbar_wait(&sh.in_full[s], (kidx / kInStages) & 1);
-          if (ENC != ENC_BF16) ok = ok && mbar_wait(&sh.b_full[sb], (kidx / kBStages) & 1);
-          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          ok = __all_sync(0xffffffffu, ok && mbar_wait(&sh.in_full[s], (kidx / kInStages) & 1) &&
+                                           (ENC == ENC_BF16 || mbar_wait(&sh.b_full[sb], (kidx / kBStages) & 1)));
+          if (!ok) break;
           tc_fence_after();
           if (gather) fence_proxy_async();               // rows copied by cp.async -> visible to the tensor core
           if (elect_one()) {
@@ -326,20 +326,18 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int r = ct;                                 // B-tile row of this thread (256 rows, 256 threads)
     uint32_t kidx = 0;
     int seq = 0;
-    for (int it = first; it < total && !*abort_flag; it += step, ++seq) {
+    for (int it = first; it < total; it += step, ++seq) {
       const TileInfo t = tile_of(it);
       const bool two = t.nrows > BM;
       const int f0 = t.tile_n * (MODE == 0 ? BN / 2 : BN);
-      bool ok = true;
       if (ENC != ENC_BF16) {
         const int sbuf = seq & 1;
-        ok = mbar_wait(&sh.sc_full[sbuf], (seq >> 1) & 1);
+        mbar_wait_or_flag(&sh.sc_full[sbuf], (seq >> 1) & 1, abort_flag);
         const float* sc = sScales + sbuf * BN * kMaxGroups + r * groups;
-        for (int kc = 0; kc < nk && ok; ++kc, ++kidx) {
+        for (int kc = 0; kc < nk; ++kc, ++kidx) {
           const uint32_t s = kidx % kPStages, sb = kidx % kBStages, use = kidx / kBStages;
-          ok = mbar_wait(&sh.p_full[s], (kidx / kPStages) & 1);
-          if (ok && use > 0) ok = mbar_wait(&sh.b_empty[sb], (use - 1) & 1);
-          if (!ok) break;
+          mbar_wait_or_flag(&sh.p_full[s], (kidx / kPStages) & 1, abort_flag);
+          if (use > 0) mbar_wait_or_flag(&sh.b_empty[sb], (use - 1) & 1, abort_flag);
           const float scale = sc[kc >> 1];
           const Q4Scale qs = q4_scale(scale);
           const bool fused = ENC == ENC_Q4 && __all_sync(0xffffffffu, qs.fused);
@@ -366,14 +364,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           __syncwarp();
           if (lane == 0) { mbar_arrive(&sh.b_full[sb]); mbar_arrive(&sh.p_empty[s]); }
         }
-        if (ok) {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sh.sc_empty[sbuf]);
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.sc_empty[sbuf]);
       }
       // ---- epilogue: warp quarter = warp % 4 (its 32 accumulator lanes), column half = (warp-2)/4 ---
-      if (ok) ok = mbar_wait(&sh.acc_full, seq & 1);
-      if (!ok) { if (lane == 0) fail(); break; }
+      if (!mbar_wait_warp(&sh.acc_full, seq & 1) || warp_sees(abort_flag)) { if (lane == 0) fail(); break; }
       tc_fence_after();
       // The accumulator reads are software-pipelined: the tcgen05.ld of chunk c + 1 is in flight while chunk c
       // is converted and stored, and the accumulators are handed back to the MMA issuer as soon as the last

@@ -305,15 +305,14 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const uint32_t full0 = in_cta(&sh.full[0], 0);
       uint32_t kidx = 0;
       int seq = 0;
-      for (int it = first; it < total && !*abort_flag; it += step, ++seq) {
+      for (int it = first; it < total; it += step, ++seq) {
         const int sb = seq & 1;
-        bool ok = mbar_wait(&sh.sc_full[sb], (seq >> 1) & 1);
+        mbar_wait_or_flag(&sh.sc_full[sb], (seq >> 1) & 1, abort_flag);
         const float* sc = sScales + sb * PM * kPairMaxGroups + row * groups;
-        for (int kc = 0; kc < nk && ok; ++kc, ++kidx) {
+        for (int kc = 0; kc < nk; ++kc, ++kidx) {
           const uint32_t ps = kidx % kPS, s = kidx % kStages, use = kidx / kStages;
-          ok = mbar_wait(&sh.p_full[ps], (kidx / kPS) & 1);
-          if (ok && use > 0) ok = mbar_wait(&sh.free_[s], (use - 1) & 1);
-          if (!ok) break;
+          mbar_wait_or_flag(&sh.p_full[ps], (kidx / kPS) & 1, abort_flag);
+          if (use > 0) mbar_wait_or_flag(&sh.free_[s], (use - 1) & 1, abort_flag);
           const float scale = sc[kc];
           const uint8_t* src = sP + ps * kPackedBytes + row * kPackedRow;
           uint8_t* dstrow = sB + s * kStepBytes + half * kAtom + row * 128;   // this thread: 64 k of one row
@@ -342,8 +341,7 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             mbar_arrive(&sh.p_empty[ps]);
           }
         }
-        if (!ok) { if (lane == 0) fail(); break; }
-        __syncwarp();
+        if (warp_sees(abort_flag)) { if (lane == 0) fail(); break; }
         if (lane == 0) mbar_arrive(&sh.sc_empty[sb]);
       }
     }
@@ -352,10 +350,10 @@ grouped_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int quarter = warp & 3;
     const uint32_t accempty0 = in_cta(&sh.acc_empty[0], 0);
     int seq = 0;
-    for (int it = first; it < total && !*abort_flag; it += step, ++seq) {
+    for (int it = first; it < total; it += step, ++seq) {
       const PairItem w = item_of(it);
       const int buf = seq & 1;
-      if (!mbar_wait(&sh.acc_full[buf], (seq >> 1) & 1)) { if (lane == 0) fail(); break; }
+      if (!mbar_wait_warp(&sh.acc_full[buf], (seq >> 1) & 1) || warp_sees(abort_flag)) { if (lane == 0) fail(); break; }
       tc_fence_after();
       const int row = (int)rank * PM + quarter * 32 + lane;     // route row inside the tile
       const bool valid = row < w.nrows;

@@ -181,20 +181,20 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     const uint64_t b_desc0 = smem_desc_sw128(smem_u32(sB)), w_desc0 = smem_desc_sw128(smem_u32(sP));
     uint32_t seq = 0;
     for (int it = first; it < total; it += step) {
-      if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+      if (warp_sees(abort_flag)) break;
       const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
       if (t.nrows == 0) continue;
       const uint32_t buf = seq % kAccBufs, use = seq / kAccBufs;
       ++seq;
-      bool ok = use == 0 || mbar_wait(&sh.acc_empty[buf], (use - 1) & 1);
+      bool ok = use == 0 || mbar_wait_warp(&sh.acc_empty[buf], (use - 1) & 1);
       const int n16 = (t.nrows + 15) & ~15;
       // kind::f16, BF16 x BF16 -> FP32, K-major operands, M = 128, N = the tile's routes
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n16 >> 3) << 17) | (8u << 24);
       const uint32_t acc = tmem + buf * NMAX;
       for (int kc = t.k0; kc < t.k1; ++kc) {
-        ok = ok && mbar_wait(&sh.in_full[rb.slot], rb.phase);
-        ok = ok && (kQuant ? mbar_wait(&sh.a_full[ra.slot], ra.phase) : mbar_wait(&sh.p_full[rp.slot], rp.phase));
-        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+        ok = __all_sync(0xffffffffu, ok && mbar_wait(&sh.in_full[rb.slot], rb.phase) &&
+                                         (kQuant ? mbar_wait(&sh.a_full[ra.slot], ra.phase) : mbar_wait(&sh.p_full[rp.slot], rp.phase)));
+        if (!ok) break;
         tc_fence_after();
         if (gather) fence_proxy_async();
         if (elect_one()) {
@@ -225,7 +225,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
       uint32_t kidx = 0, seq = 0;
       Ring<kPStages> rp;
       for (int it = first; it < total; it += step) {
-        if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+        if (warp_sees(abort_flag)) break;
         const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
         if (t.nrows == 0) continue;
         const long long wrow0 = (long long)t.expert * p.n_rows + t.col * kFeatures;
@@ -279,7 +279,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
         uint32_t kidx = 0;
         Ring<kBStages> rb;
         for (int it = first; it < total; it += step) {
-          if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+          if (warp_sees(abort_flag)) break;
           const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
           if (t.nrows == 0) continue;
           const int boxes = (t.nrows + kActBox - 1) / kActBox;
@@ -354,19 +354,18 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     uint32_t kidx = 0, seq = 0;
     Ring<kPStages> rp;
     Ring<kAStages> ra;
-    for (int it = first; it < total && !*abort_flag; it += step) {
+    for (int it = first; it < total; it += step) {
       const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
       if (t.nrows == 0) continue;
       const uint32_t sbuf = seq & 1;
-      bool ok = mbar_wait(&sh.sc_full[sbuf], (seq >> 1) & 1);
+      mbar_wait_or_flag(&sh.sc_full[sbuf], (seq >> 1) & 1, abort_flag);
       ++seq;
       const float* sc = sScales + sbuf * kRows * kTsMaxGroups + row * groups;
-      for (int kc = 0; kc < nk && ok; ++kc, ++kidx) {
+      for (int kc = 0; kc < nk; ++kc, ++kidx) {
         const float scale = sc[kc];
         const Q4Scale qs = q4_scale(scale);
         const bool fused = ENC == ENC_Q4 && __all_sync(0xffffffffu, qs.fused);
-        ok = mbar_wait(&sh.p_full[rp.slot], rp.phase);
-        if (!ok) break;
+        mbar_wait_or_flag(&sh.p_full[rp.slot], rp.phase, abort_flag);
         const uint8_t* src = sP + rp.slot * S::kWeightBytes + row * S::kPackedRow;
         uint32_t out[2][16];
 #pragma unroll
@@ -383,8 +382,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.p_empty[rp.slot]);
-        if (kidx >= (uint32_t)kAStages) ok = mbar_wait(&sh.a_empty[ra.slot], ra.phase ^ 1);
-        if (!ok) break;
+        if (kidx >= (uint32_t)kAStages) mbar_wait_or_flag(&sh.a_empty[ra.slot], ra.phase ^ 1, abort_flag);
         tc_fence_after();
 #pragma unroll
         for (int j = 0; j < 2; ++j) tmem_st16(a_lane + ra.slot * (S::kStepK / 2) + j * 16, out[j]);
@@ -395,8 +393,7 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
         rp.next();
         ra.next();
       }
-      if (!ok) { if (lane == 0) fail(); break; }
-      __syncwarp();
+      if (warp_sees(abort_flag)) { if (lane == 0) fail(); break; }
       if (lane == 0) mbar_arrive(&sh.sc_empty[sbuf]);
     }
   } else {
@@ -406,12 +403,12 @@ grouped_ts_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     const int quarter = warp & 3;
     const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
     uint32_t seq = 0;
-    for (int it = first; it < total && !*abort_flag; it += step) {
+    for (int it = first; it < total; it += step) {
       const TsTile t = ts_tile<kSplit, WIDE>(p, it, n_col, nk);
       if (t.nrows == 0) continue;
       const uint32_t buf = seq % kAccBufs, use = seq / kAccBufs;
       ++seq;
-      if (!mbar_wait(&sh.acc_full[buf], use & 1)) { if (lane == 0) fail(); break; }
+      if (!mbar_wait_warp(&sh.acc_full[buf], use & 1) || warp_sees(abort_flag)) { if (lane == 0) fail(); break; }
       tc_fence_after();
       const int chunks = (t.nrows + 15) >> 4;
       const uint32_t acc = lane_base + buf * NMAX;

@@ -142,15 +142,15 @@ grouped_wide_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_co
     uint32_t seq = 0;
     const uint64_t b_desc0 = smem_desc_sw128(smem_u32(sB));
     for (int it = first; it < total; it += step, ++seq) {
-      if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+      if (warp_sees(abort_flag)) break;
       const WideTile t = wide_tile(p, it, n_col);
       const int n16 = (t.nrows + 15) & ~15;
       // kind::f16, BF16 x BF16 -> FP32, K-major operands, M = 128, N = the tile's routes
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n16 >> 3) << 17) | (8u << 24);
-      bool ok = seq == 0 || mbar_wait(&sh.acc_empty, (seq - 1) & 1);
+      bool ok = seq == 0 || mbar_wait_warp(&sh.acc_empty, (seq - 1) & 1);
       for (int kc = 0; kc < nk; ++kc) {
-        ok = ok && mbar_wait(&sh.in_full[rb.slot], rb.phase) && mbar_wait(&sh.a_full[ra.slot], ra.phase);
-        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+        ok = __all_sync(0xffffffffu, ok && mbar_wait(&sh.in_full[rb.slot], rb.phase) && mbar_wait(&sh.a_full[ra.slot], ra.phase));
+        if (!ok) break;
         tc_fence_after();
         if (MODE == 0) fence_proxy_async();
         if (elect_one()) {
@@ -178,7 +178,7 @@ grouped_wide_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_co
       uint32_t kidx = 0, seq = 0;
       Ring<kPStages> rp;
       for (int it = first; it < total; it += step) {
-        if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+        if (warp_sees(abort_flag)) break;
         const WideTile t = wide_tile(p, it, n_col);
         const long long wrow0 = (long long)t.expert * p.n_rows + t.col * kFeatures;
         const uint32_t sb = seq & 1;
@@ -222,7 +222,7 @@ grouped_wide_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_co
         uint32_t kidx = 0;
         Ring<kBStages> rb;
         for (int it = first; it < total; it += step) {
-          if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+          if (warp_sees(abort_flag)) break;
           const WideTile t = wide_tile(p, it, n_col);
           const int boxes = (t.nrows + kActBox - 1) / kActBox;
           bool ok = true;
@@ -287,14 +287,14 @@ grouped_wide_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_co
     uint32_t kidx = 0, seq = 0;
     Ring<kPStages> rp;
     Ring<kAStages> ra;
-    for (int it = first; it < total && !*abort_flag; it += step) {
+    for (int it = first; it < total; it += step) {
       const uint32_t sbuf = seq & 1;
-      bool ok = mbar_wait(&sh.sc_full[sbuf], (seq >> 1) & 1);
+      mbar_wait_or_flag(&sh.sc_full[sbuf], (seq >> 1) & 1, abort_flag);
       ++seq;
       const float* sc = sScales + sbuf * kScaleBuffer + row * groups;
       float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
       Q4Scale qs = q4_scale(0.f);
-      for (int kc = 0; kc < nk && ok; ++kc, ++kidx) {
+      for (int kc = 0; kc < nk; ++kc, ++kidx) {
         if (vec) {                                          // rows 64 bytes apart: four scales per load, a quarter of the conflicts
           if ((kc & 7) == 0) s4 = *reinterpret_cast<const float4*>(sc + (kc >> 1));
         } else if ((kc & 1) == 0) {
@@ -302,8 +302,7 @@ grouped_wide_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_co
         }
         const int j4 = (kc >> 1) & 3;
         const float scale = j4 < 2 ? (j4 == 0 ? s4.x : s4.y) : (j4 == 2 ? s4.z : s4.w);
-        ok = mbar_wait(&sh.p_full[rp.slot], rp.phase);
-        if (!ok) break;
+        mbar_wait_or_flag(&sh.p_full[rp.slot], rp.phase, abort_flag);
         const uint8_t* src = sP + rp.slot * S::kWeightBytes + row * S::kPackedRow;
         if (ENC == ENC_Q4 && (kc & 1) == 0) qs = q4_scale(scale);
         const bool fused = ENC == ENC_Q4 && __all_sync(0xffffffffu, qs.fused);
@@ -320,13 +319,11 @@ grouped_wide_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_co
                        *reinterpret_cast<const uint4*>(src + (((2 * j + 1) ^ sw) << 4)), scale, out);
           }
           if (j == 0) {
-            if (kidx >= (uint32_t)kAStages) ok = mbar_wait(&sh.a_empty[ra.slot], ra.phase ^ 1);
-            if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+            if (kidx >= (uint32_t)kAStages) mbar_wait_or_flag(&sh.a_empty[ra.slot], ra.phase ^ 1, abort_flag);
             tc_fence_after();
           }
           tmem_st16(a_lane + ra.slot * kAStageCols + j * 16, out);
         }
-        if (!ok) break;
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.p_empty[rp.slot]);
         tmem_st_wait();
@@ -336,8 +333,7 @@ grouped_wide_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_co
         rp.next();
         ra.next();
       }
-      if (!ok) { if (lane == 0) fail(); break; }
-      __syncwarp();
+      if (warp_sees(abort_flag)) { if (lane == 0) fail(); break; }
       if (lane == 0) mbar_arrive(&sh.sc_empty[sbuf]);
     }
   } else {
@@ -356,7 +352,7 @@ grouped_wide_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_co
     bool ok = true;
     for (int it = first; it < total; it += step, ++seq) {
       const WideTile t = wide_tile(p, it, n_col);
-      ok = mbar_wait(&sh.acc_full, seq & 1);
+      ok = mbar_wait_warp(&sh.acc_full, seq & 1);
       // the group's warps agree whether to go on: none may be left waiting at a chunk's barrier
       if (named_bar_or(2 + group, kGroupThreads, !ok || *abort_flag != 0)) break;
       tc_fence_after();
