@@ -1,0 +1,59 @@
+"""How the back end keeps the workspaces of its calls, with the device calls replaced."""
+
+import contextlib
+import weakref
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from uma_qmoe_b200 import _native, native_backend, ops
+
+
+class _Buffer(torch.Tensor):
+    """A workspace that can be watched going away."""
+
+
+@pytest.fixture
+def world(monkeypatch):
+    state = SimpleNamespace(capturing=False, calls=[], made=[], on_step=None)
+    backend = native_backend.MixedTargetNativeBackend(native_backend.PLATFORM, _native.lib())
+    layer = SimpleNamespace(hidden=2048, intermediate=1024, num_experts=64, used_on=lambda *_: None)
+    monkeypatch.setattr(backend, "_device_layer", lambda *_: layer)
+    monkeypatch.setattr(native_backend, "acquire_expert_pack", lambda handle: contextlib.nullcontext())
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 7, raising=False)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: state.capturing)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: None)
+    event = lambda: SimpleNamespace(cuda_event=1, record=lambda stream=None: None, synchronize=lambda: None)
+    monkeypatch.setattr(torch.cuda, "Event", event)
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda self: self)
+
+    def workspace(layer, tokens, *_):
+        buffer = torch.zeros(4096, dtype=torch.uint8).as_subclass(_Buffer)
+        state.made.append(weakref.ref(buffer))
+        return buffer
+
+    def step(layer, hidden, indices, weights, out, buffer, shared, router, renormalize, host, event, stream):
+        if state.on_step:
+            state.on_step(buffer)
+        state.calls.append((buffer.data_ptr(), host))
+
+    monkeypatch.setattr(ops, "prefill_workspace", workspace)
+    monkeypatch.setattr(ops, "decode_workspace", lambda layer, top_k, *_: workspace(layer, 1))
+    monkeypatch.setattr(ops, "moe_step", step)
+    state.backend = backend
+    state.run = lambda tokens, pack=1: backend._run(
+        "olmoe", torch.zeros(tokens, 2048, dtype=torch.bfloat16), torch.zeros(tokens, 8, dtype=torch.int64),
+        torch.zeros(tokens, 8), 0, pack)
+    return state
+
+
+@pytest.mark.parametrize("tokens,word", [(1, 2), (4, 0)])
+def test_a_waiting_check_sees_an_error_that_the_hosts_copy_missed(world, tokens, word):
+    """The last kernel's first CTA may have copied the status word before another CTA of it gave up."""
+    world.run(tokens)
+    world.made[0]()[:16].view(torch.int32)[word] = -4         # UMAQ_ERR_DEVICE_TIMEOUT
+    with pytest.raises(RuntimeError, match="failed on the device"):
+        world.backend.check_device_status()
+    world.backend.check_device_status()                       # reported once
+    world.run(tokens)

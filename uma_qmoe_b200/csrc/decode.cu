@@ -1193,6 +1193,7 @@ __global__ void __maxnreg__(96) decode_down_kernel(const DecodeParams p) {
     }
   } else if (tid == 0) {
     atomicExch(p.sync + kSyncStatus, (unsigned)ERR_DEVICE_TIMEOUT);
+    if (p.host_status) *reinterpret_cast<volatile unsigned*>(p.host_status) = (unsigned)ERR_DEVICE_TIMEOUT;   // CTA 0 may be gone
     __nanosleep(100000);
   }
   if (p.host_status && blockIdx.x == 0 && tid == 0) {       // the gate/up kernel's reports are behind its counter

@@ -71,9 +71,10 @@ class _Workspace:
     """A kernel workspace owned by one (shape, device, stream), room for the routes of a call that routes itself, and the host's
     view of the workspace's sticky status word.
 
-    The last kernel of a call copies the word to mapped host memory if it is set, and an event is recorded behind the call;
-    the next call on this workspace looks at the host's copy, `cache_summary()` and `release_pack()` do once the event has
-    completed.  Nothing on the hot path waits for the device."""
+    The last kernel of a call copies the word to mapped host memory if it is set, and an event is recorded behind the call.
+    The next call on this workspace looks at the host's copy; `cache_summary()` and `release_pack()` wait for the event and
+    then look at the word itself as well, which every CTA of the call has written by then.  Nothing on the hot path waits for
+    the device."""
 
     __slots__ = ("kind", "buffer", "host", "word", "event", "used", "tokens", "indices", "weights", "lock")
 
@@ -111,6 +112,8 @@ class _Workspace:
             return
         self.event.synchronize()                     # all work on the buffer has finished
         code = int(self.word[0])
+        if wait and code == 0:
+            code = int(self.buffer[:16].view(torch.int32)[0 if self.kind == "prefill" else 2])
         if code == 0:
             return
         # sticky on the device: clear it so that the error is reported once
