@@ -117,3 +117,24 @@ def test_bf16_routing_weights_are_accepted(olmoe_pack):
     b = torch.ops.uma_qmoe.moe_forward(x, idx, wb.float(), 0, handle, True)
     assert torch.equal(a, b)
     assert_parity(a.cpu(), torch.ops.uma_qmoe.moe_forward(x, idx, w, 0, handle, True).cpu(), max_abs=6e-2, cosine=0.999)
+
+
+def test_a_graph_replays_after_its_streams_workspace_has_grown(olmoe_pack):
+    """Captured at 7 tokens with a workspace that a larger eager call on the same stream then replaces; memory allocated after
+    that must not be the graph's."""
+    _backend, handle = olmoe_pack
+    x = syn.activations(SEED + 30, 300).to(DEV)
+    idx, w = _routes(300, SEED + 30)
+    want = torch.ops.uma_qmoe.moe_forward(x[:7], idx[:7], w[:7], 0, handle, True)
+    side = torch.cuda.Stream(device=DEV)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.ops.uma_qmoe.moe_forward(x[:7], idx[:7], w[:7], 0, handle, True)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            got = torch.ops.uma_qmoe.moe_forward(x[:7], idx[:7], w[:7], 0, handle, True)
+        torch.ops.uma_qmoe.moe_forward(x, idx, w, 0, handle, True)
+        others = [torch.full((1 << n,), 85, dtype=torch.uint8, device=DEV) for n in range(8, 24) for _ in range(4)]
+        graph.replay()
+    side.synchronize()
+    assert torch.equal(got, want) and all(bool((t == 85).all()) for t in others)

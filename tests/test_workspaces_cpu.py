@@ -1,6 +1,7 @@
 """How the back end keeps the workspaces of its calls, with the device calls replaced."""
 
 import contextlib
+import gc
 import weakref
 from types import SimpleNamespace
 
@@ -57,3 +58,22 @@ def test_a_waiting_check_sees_an_error_that_the_hosts_copy_missed(world, tokens,
         world.backend.check_device_status()
     world.backend.check_device_status()                       # reported once
     world.run(tokens)
+
+
+def test_a_captured_workspace_outlives_its_replacement(world):
+    """Capture at 7 tokens, then an eager prompt of 300 on the same stream: the graph still holds the first buffer's address."""
+    world.run(7)
+    world.capturing = True
+    world.run(7)
+    world.capturing = False
+    world.run(300)
+    gc.collect()
+    assert len(world.made) == 2 and world.made[0]() is not None
+    world.run(600)                                            # the one for 300 was not captured: it goes
+    gc.collect()
+    assert world.made[0]() is not None and world.made[1]() is None
+    world.backend._drop_layers(2)                             # another pack
+    assert world.made[0]() is not None
+    world.backend._drop_layers(1)                             # the graph's weights go as well now
+    gc.collect()
+    assert world.made[0]() is None

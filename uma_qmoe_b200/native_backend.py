@@ -76,7 +76,7 @@ class _Workspace:
     then look at the word itself as well, which every CTA of the call has written by then.  Nothing on the hot path waits for
     the device."""
 
-    __slots__ = ("kind", "buffer", "host", "word", "event", "used", "tokens", "indices", "weights", "lock")
+    __slots__ = ("kind", "buffer", "host", "word", "event", "used", "tokens", "indices", "weights", "lock", "captured")
 
     def __init__(self, kind: str, buffer: Any, tokens: int, top_k: int, stream: Any) -> None:
         import torch
@@ -88,15 +88,17 @@ class _Workspace:
         if not torch.cuda.is_current_stream_capturing():
             self.event.record(stream)                # creates it
         self.used = False
+        self.captured: set[int] = set()              # packs with a captured call, whose graph holds this slot's addresses
         self.lock = threading.Lock()                 # the launches of a call stay together on the stream
         self.indices = torch.empty((tokens, top_k), dtype=torch.int64, device=buffer.device)
         self.weights = torch.empty((tokens, top_k), dtype=torch.float32, device=buffer.device)
 
-    def report(self, device: Any) -> tuple[Optional[int], Optional[int]]:
+    def report(self, device: Any, pack_handle: int) -> tuple[Optional[int], Optional[int]]:
         """Where a call leaves its status and which event it records; a captured call reports through the workspace only."""
         import torch
 
         if torch.cuda.is_current_stream_capturing():
+            self.captured.add(pack_handle)
             return None, None
         if not self.event.cuda_event:                # made during a capture
             self.event.record(torch.cuda.current_stream(device))
@@ -141,6 +143,7 @@ class MixedTargetNativeBackend:
         self.extension = extension
         self._cache = _LayerCache()
         self._workspaces: dict[tuple, _Workspace] = {}
+        self._outgrown: list[_Workspace] = []                    # replaced by larger ones, but captured graphs use them
         self._pending: dict[tuple[int, int, str], Any] = {}      # layers being staged: (DeviceLayer, wait)
         self._linear_cache: dict[tuple[int, str, str], Any] = {}  # single tensors staged for q4_linear / q8_linear
         self._workspace_lock = threading.Lock()
@@ -301,12 +304,17 @@ class MixedTargetNativeBackend:
                 del self._cache.layers[key]
             for key in [k for k in self._linear_cache if k[0] == pack_handle]:
                 del self._linear_cache[key]
+        with self._workspace_lock:
+            for slot in [*self._workspaces.values(), *self._outgrown]:
+                slot.captured.discard(pack_handle)
+            self._outgrown = [slot for slot in self._outgrown if slot.captured]
 
     # ---- execution ------------------------------------------------------------------------
     def _workspace(self, kind: str, layer: Any, tokens: int, top_k: int, shared: Any, device: Any, stream: int) -> _Workspace:
         """The workspace of this shape on this stream.  Calls on different streams (or threads, which have their own
         current stream only if they set one) never share a workspace, so they may overlap on the device; a stream
-        keeps one prefill workspace per layer shape, grown to the largest token count seen."""
+        keeps one prefill workspace per layer shape, grown to the largest token count seen.  One that a graph has captured
+        stays until the packs of the captured calls are released: without their weights no such graph can run."""
         from . import ops
 
         family = (kind, device.index, stream, layer.hidden, layer.intermediate, layer.num_experts, top_k,
@@ -325,6 +333,8 @@ class MixedTargetNativeBackend:
         fresh = _Workspace(kind, buffer, tokens, top_k, torch.cuda.current_stream(device))
         with self._workspace_lock:
             self._workspaces[family] = fresh
+            if slot is not None and slot.captured:
+                self._outgrown.append(slot)
         return fresh
 
     def _run(self, model: str, hidden_states: Any, expert_indices: Any, routing_weights: Any, layer_index: int,
@@ -373,7 +383,7 @@ class MixedTargetNativeBackend:
             indices, weights = slot.indices, slot.weights
             if slot.tokens != tokens:
                 indices, weights = indices[:tokens], weights[:tokens]
-        host, event = slot.report(device)
+        host, event = slot.report(device, pack_handle)
         with slot.lock:
             ops.moe_step(layer, flat, indices, weights, out, slot.buffer, shared, None if router is None else router[0],
                          router is not None and router[2], host, event, stream)
