@@ -77,3 +77,38 @@ def test_a_captured_workspace_outlives_its_replacement(world):
     world.backend._drop_layers(1)                             # the graph's weights go as well now
     gc.collect()
     assert world.made[0]() is None
+
+
+@pytest.mark.parametrize("before", [None, 4])
+def test_no_call_runs_on_a_workspace_that_another_thread_has_replaced(world, before):
+    """Its host copy of the status would be given back while the call may still write to it, and nobody would look there."""
+    if before:
+        world.run(before)
+    find, pending = world.backend._workspace, [True]
+
+    def find_and_be_overtaken(*args):
+        slot = find(*args)
+        if pending:
+            pending.clear()
+            world.run(300)                                    # the other thread's call, on the same stream
+        return slot
+
+    world.backend._workspace = find_and_be_overtaken
+    world.run(4)
+    kept = {slot.buffer.data_ptr() for slot in world.backend._workspaces.values()}
+    assert world.calls[-1][0] in kept and world.calls[-2][0] in kept
+
+
+def test_two_threads_first_calls_share_one_workspace(world, monkeypatch):
+    make, pending = ops.prefill_workspace, [True]
+
+    def make_and_be_overtaken(*args):
+        if pending:
+            pending.clear()
+            world.run(4)
+        return make(*args)
+
+    monkeypatch.setattr(ops, "prefill_workspace", make_and_be_overtaken)
+    world.run(4)
+    kept = {slot.buffer.data_ptr() for slot in world.backend._workspaces.values()}
+    assert {call[0] for call in world.calls} == kept

@@ -18,6 +18,7 @@ per projection; nothing is dequantised, ``dequantized_weight_bytes`` stays 0.
 
 from __future__ import annotations
 
+import contextlib
 import threading
 import warnings
 from pathlib import Path
@@ -76,7 +77,8 @@ class _Workspace:
     then look at the word itself as well, which every CTA of the call has written by then.  Nothing on the hot path waits for
     the device."""
 
-    __slots__ = ("kind", "buffer", "host", "word", "event", "used", "tokens", "indices", "weights", "lock", "captured")
+    __slots__ = ("kind", "buffer", "host", "word", "event", "used", "tokens", "indices", "weights", "lock", "captured",
+                 "outgrown")
 
     def __init__(self, kind: str, buffer: Any, tokens: int, top_k: int, stream: Any) -> None:
         import torch
@@ -89,6 +91,7 @@ class _Workspace:
             self.event.record(stream)                # creates it
         self.used = False
         self.captured: set[int] = set()              # packs with a captured call, whose graph holds this slot's addresses
+        self.outgrown = False                        # a larger slot has taken its place: no further call
         self.lock = threading.Lock()                 # the launches of a call stay together on the stream
         self.indices = torch.empty((tokens, top_k), dtype=torch.int64, device=buffer.device)
         self.weights = torch.empty((tokens, top_k), dtype=torch.float32, device=buffer.device)
@@ -272,7 +275,7 @@ class MixedTargetNativeBackend:
     def check_device_status(self) -> None:
         """Wait for the calls submitted so far and raise if one of them recorded a device-side error."""
         with self._workspace_lock:
-            slots = list(self._workspaces.values())
+            slots = [*self._workspaces.values(), *self._outgrown]
         for slot in slots:
             slot.raise_if_failed(wait=True)
 
@@ -319,23 +322,30 @@ class MixedTargetNativeBackend:
 
         family = (kind, device.index, stream, layer.hidden, layer.intermediate, layer.num_experts, top_k,
                   0 if shared is None else shared.gate.shape[0])
-        with self._workspace_lock:
-            slot = self._workspaces.get(family)
-            if slot is not None and (kind == "decode" or slot.tokens >= tokens):
-                return slot
-        import torch
-        if slot is not None:
-            slot.raise_if_failed(wait=True)          # the smaller buffer is about to be dropped
-        if kind == "decode":
-            buffer, tokens = ops.decode_workspace(layer, top_k, shared, device), 1
-        else:
-            buffer = ops.prefill_workspace(layer, tokens, top_k, shared, device)
-        fresh = _Workspace(kind, buffer, tokens, top_k, torch.cuda.current_stream(device))
-        with self._workspace_lock:
-            self._workspaces[family] = fresh
-            if slot is not None and slot.captured:
-                self._outgrown.append(slot)
-        return fresh
+        while True:
+            with self._workspace_lock:
+                slot = self._workspaces.get(family)
+                if slot is not None and (kind == "decode" or slot.tokens >= tokens):
+                    return slot
+            import torch
+            with contextlib.nullcontext() if slot is None else slot.lock:    # no call is being issued on it meanwhile
+                if slot is not None:
+                    slot.raise_if_failed(wait=True)  # the smaller buffer is about to be dropped
+                if kind == "decode":
+                    buffer, room = ops.decode_workspace(layer, top_k, shared, device), 1
+                else:
+                    buffer, room = ops.prefill_workspace(layer, tokens, top_k, shared, device), tokens
+                fresh = _Workspace(kind, buffer, room, top_k, torch.cuda.current_stream(device))
+                with self._workspace_lock:
+                    if self._workspaces.get(family) is not slot:             # another thread was quicker
+                        continue
+                    self._workspaces[family] = fresh
+                    if slot is not None:
+                        slot.outgrown = True
+                        # (under a capture nobody has waited for the calls that may still write to the host's copy)
+                        if slot.captured or torch.cuda.is_current_stream_capturing():
+                            self._outgrown.append(slot)
+                return fresh
 
     def _run(self, model: str, hidden_states: Any, expert_indices: Any, routing_weights: Any, layer_index: int,
              pack_handle: int, shared: Optional[Any] = None, router: Optional[tuple] = None):
@@ -374,19 +384,23 @@ class MixedTargetNativeBackend:
             ops.route_topk(flat, *router)     # refuses it: a router has no empty result
         if tokens == 0:                       # an empty batch has an empty result; there is nothing to launch
             return out.reshape(hidden_states.shape)
-        slot = self._workspace("decode" if tokens == 1 else "prefill", layer, tokens, top_k, shared, device, stream)
-        slot.raise_if_failed(wait=False)      # an error an earlier call on this workspace left behind, if already known
         if router is None:
             indices = expert_indices.contiguous()
             weights = routing_weights.to(dtype=torch.float32).contiguous()     # float32 routing weights, no BF16 rounding
-        else:
-            indices, weights = slot.indices, slot.weights
-            if slot.tokens != tokens:
-                indices, weights = indices[:tokens], weights[:tokens]
-        host, event = slot.report(device, pack_handle)
-        with slot.lock:
-            ops.moe_step(layer, flat, indices, weights, out, slot.buffer, shared, None if router is None else router[0],
-                         router is not None and router[2], host, event, stream)
+        while True:
+            slot = self._workspace("decode" if tokens == 1 else "prefill", layer, tokens, top_k, shared, device, stream)
+            slot.raise_if_failed(wait=False)  # an error an earlier call on this workspace left behind, if already known
+            with slot.lock:
+                if slot.outgrown:             # by another thread on this stream, between the two lines above
+                    continue
+                if router is not None:
+                    indices, weights = slot.indices, slot.weights
+                    if slot.tokens != tokens:
+                        indices, weights = indices[:tokens], weights[:tokens]
+                host, event = slot.report(device, pack_handle)
+                ops.moe_step(layer, flat, indices, weights, out, slot.buffer, shared, None if router is None else router[0],
+                             router is not None and router[2], host, event, stream)
+                break
         return out.reshape(hidden_states.shape)
 
     # ---- one projection as a linear layer -----------------------------------------------------
