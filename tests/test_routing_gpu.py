@@ -56,3 +56,18 @@ def test_sort_in_one_launch_and_in_two(tokens, top_k, experts):
     assert torch.equal(one.sorted_route[:n], many.sorted_route[:n]) and torch.equal(one.route_pos, many.route_pos)
     assert torch.equal(one.tile_table.view(3, -1)[:, :tiles], many.tile_table.view(3, -1)[:, :tiles])
     assert int(one.status) == 0 and int(many.status) == 0
+
+
+@pytest.mark.parametrize("hidden", [4096, 5632, 5888, 6144, 8192])
+@pytest.mark.parametrize("tokens", [1, 7, 192, 193])
+def test_router_takes_hidden_sizes_around_48_kb_of_rows(hidden, tokens):
+    """Four rows and the ranks beside them pass what an ordinary launch may use.  Weights against float64: a logit of 64 terms of size
+    one is rounded to BF16 (2^-9 of at most 4 here), which a softmax passes on as a relative error of 2^-7."""
+    gen = torch.Generator(device=DEV).manual_seed(hidden)
+    x = torch.randn(tokens, hidden, device=DEV, generator=gen).to(torch.bfloat16)
+    weight = torch.zeros(64, hidden, device=DEV)
+    weight[:, torch.randperm(hidden, device=DEV, generator=gen)[:64]] = torch.randn(64, 64, device=DEV, generator=gen) / 8
+    weight = weight.to(torch.bfloat16)
+    w, idx = ops.route_topk(x, weight, 8, False)
+    exact = (x.double() @ weight.double().T).softmax(1).gather(1, idx)
+    assert ((w.double() - exact).abs() <= 2.0 ** -6 * exact).all()

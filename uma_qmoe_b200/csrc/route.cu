@@ -1131,7 +1131,8 @@ int launch_router_topk(const RouterArgs& a, cudaStream_t stream) {
     static thread_local int small_configured = -1, small_bytes = 0;
     int dev = 0;
     cudaGetDevice(&dev);
-    if (small_smem > 48 * 1024 && (small_configured != dev || small_bytes < (int)small_smem)) {
+    // The 48 KB of an ordinary launch hold the static part (6 KB) as well, so ask well below them.
+    if (small_smem > 32 * 1024 && (small_configured != dev || small_bytes < (int)small_smem)) {
       cudaError_t e = cudaFuncSetAttribute(router_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem);
       if (e != cudaSuccess) { set_error("router: cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return ERR_LAUNCH; }
       small_configured = dev; small_bytes = (int)small_smem;
