@@ -617,6 +617,12 @@ long long grouped_gemm_dense_part_rows(long long rows, int n_rows, int k) {
 //   OLMoE Q8   88 routes per expert 217 | 182 / 234 | 188   128: 242 | 196 / 234 | 230   256: 345 | 324 / 346 | 344   512: 532 | 543 / 520 | 552
 //   Qwen  Q8  102 routes per expert 270 | 226 / 281 | 238   136: 310 | 243 / 291 | 273   273: 488 | 422 / 421 | 420   546: 814 | 724 / 715 | 746
 // Around 192 (a tile and a little more for many experts) they lose: 192, OLMoE Q4 212 | 232 / 241 | 228, Q8 258 | 288 / 290 | 284.
+// Between 400 and 490 they lose as well where routes spread evenly and win or draw where they do not: 467, Qwen Q4 493 | 535 / 554 | 532;
+// 475, OLMoE Q4 392 | 444 / 457 | 452; 380 and 512, Qwen Q4 464 | 435 / 460 | 436 and 614 | 559 / 622 | 578.
+// Routes on a few experts only are not seen here and can lose: time with them over time without, 440 routings of both models at random
+// sizes, evenly 0.75 to 1.14, skewed 0.80 to 1.06, on 4 to 60 experts 0.78 to 1.31 (0.98 on average).  The ratio of waves would tell:
+// wide tiles win below 1.3 times the waves of 256-row tiles, 0.1 % off the better one on average.  But the counts are on the device,
+// and asking there takes four GEMM launches in place of two.
 constexpr long long kWideGapFrom = 160, kWideGapTo = 248, kWideMaxRoutesQ4 = 512, kWideMaxRoutesQ8 = 288;
 bool grouped_gemm_takes_wide(int enc, long long rows, int experts, int hidden, int inter) {
   if (enc == ENC_BF16 || hidden % 256 || inter % 128 || hidden > 2048 || inter > 2048) return false;
