@@ -71,3 +71,27 @@ def test_router_takes_hidden_sizes_around_48_kb_of_rows(hidden, tokens):
     w, idx = ops.route_topk(x, weight, 8, False)
     exact = (x.double() @ weight.double().T).softmax(1).gather(1, idx)
     assert ((w.double() - exact).abs() <= 2.0 ** -6 * exact).all()
+
+
+@pytest.mark.parametrize("tokens,top_k,experts", [(303104, 1, 64), (303105, 1, 64), (50003, 7, 60), (700001, 1, 128), (40000, 8, 1)])
+def test_sort_without_scratch_of_more_routes_than_run_at_once(tokens, top_k, experts):
+    """A CTA then places several batches of 1024 routes; some of the last one's may be empty."""
+    gen = torch.Generator(device=DEV).manual_seed(tokens)
+    idx = torch.randint(-1, experts, (tokens, top_k), device=DEV, generator=gen)
+    w = torch.rand(tokens, top_k, device=DEV, generator=gen)
+    r = ops.route_sort(idx, w, experts)
+    for t in (r.counts, r.offsets, r.sorted_route, r.route_pos, r.sorted_weight, r.num_tiles, r.tile_table):
+        t.zero_()
+    code = _native.lib().umaq_route_sort(
+        idx.data_ptr(), 1, w.data_ptr(), tokens, top_k, experts, r.counts.data_ptr(), r.offsets.data_ptr(), r.sorted_route.data_ptr(),
+        r.route_pos.data_ptr(), r.sorted_weight.data_ptr(), r.num_tiles.data_ptr(), r.tile_table.data_ptr(), r.max_tiles,
+        r.status.data_ptr(), None, 0, torch.cuda.current_stream().cuda_stream)
+    flat = idx.reshape(-1)
+    order = torch.where(flat < 0, experts, flat).sort(stable=True).indices[:int((flat >= 0).sum())]
+    n = len(order)
+    pos = torch.full_like(flat, -1)
+    pos[order] = torch.arange(n, device=DEV)
+    assert code == 0 and int(r.status) == 0
+    assert torch.equal(r.counts.long(), torch.bincount(flat[flat >= 0], minlength=experts))
+    assert torch.equal(r.sorted_route[:n].long(), order) and torch.equal(r.route_pos.long(), pos)
+    assert torch.equal(r.sorted_weight[:n], w.reshape(-1)[order])
