@@ -57,3 +57,40 @@ def test_block_gives_the_bits_of_router_and_operator(model, tokens):
         custom_op.unregister_expert_pack(handle)
     with pytest.raises(RuntimeError, match="unknown or closed ExpertPack handle"):
         block(x)
+
+
+@pytest.mark.parametrize("tokens", [1, 9])
+def test_block_shows_its_operator_to_modes_profilers_and_autograd(tokens):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Seen(TorchDispatchMode):
+        def __init__(self):
+            super().__init__()
+            self.names = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.names.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    shape = syn.OLMOE
+    backend = native_backend.install_mixed_target_backend()
+    handle = custom_op.register_target_pack(InMemoryPack({0: "q4_group128"}))
+    try:
+        backend.preload_layer(handle, 0, DEV, random_layer(shape, "q4_group128", 3, DEV))
+        gate = SimpleNamespace(weight=syn.router_weight(1, 0, shape, skew=1.0).to(DEV), top_k=8, norm_topk_prob=False)
+        block = QuantizedMoEBlock(gate, layer_index=0, pack_handle=handle, performance_mode=True)
+        x = torch.randn(1, tokens, shape.hidden, device=DEV).to(torch.bfloat16)
+        want = block(x)
+        with Seen() as seen:
+            assert torch.equal(block(x), want)
+        assert any(name.startswith("uma_qmoe.moe_forward") for name in seen.names)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as profile:
+            block(x)
+        assert any(event.key == "uma_qmoe::moe_forward" for event in profile.key_averages())
+        leaf = x.clone().requires_grad_()
+        out = block(leaf)
+        assert out.requires_grad and torch.equal(out.detach(), want)
+        with torch.no_grad():
+            assert not block(leaf).requires_grad
+    finally:
+        custom_op.unregister_expert_pack(handle)

@@ -5,7 +5,8 @@
 They run what the ``torch.ops.uma_qmoe`` operators run, with the path around it fused: the router
 (softmax / top-k / renormalisation) is one kernel, for Qwen the shared expert, its sigmoid gate and the
 final add run inside the expert kernels instead of as separate cuBLAS and element-wise launches, and the
-back end issues all of it from one native call.
+back end issues all of it from one native call.  Where the OLMoE operator would be seen (dispatch modes,
+profilers, autograd) the block calls the router and the operator one after the other, with the same bits.
 """
 
 from __future__ import annotations
@@ -23,6 +24,12 @@ def _router_params(gate: Any) -> tuple[torch.Tensor, int, bool]:
     return gate.weight, int(gate.top_k), bool(getattr(gate, "norm_topk_prob", False))
 
 
+def _unobserved(hidden: torch.Tensor) -> bool:
+    """Nobody looks at the operators of this call: no dispatch mode or tensor subclass, no profiler, no autograd history to keep."""
+    return (type(hidden) is torch.Tensor and not torch._C._len_torch_dispatch_stack()
+            and not torch.autograd._profiler_enabled() and not (hidden.requires_grad and torch.is_grad_enabled()))
+
+
 class QuantizedMoEBlock(torch.nn.Module):
     """OLMoE router plus the compressed routed experts."""
 
@@ -37,7 +44,7 @@ class QuantizedMoEBlock(torch.nn.Module):
         weight, top_k, renorm = _router_params(self.gate)
         flat = hidden_states.reshape(-1, hidden_states.shape[-1])
         whole = getattr(_backend_for(platform_of(torch, flat)), "block_forward", None)
-        if callable(whole):                       # router and experts in one native call
+        if callable(whole) and _unobserved(flat):             # router and experts in one native call
             with acquire_expert_pack(self.pack_handle):
                 return whole("olmoe", flat, weight, top_k, renorm, self.layer_index, self.pack_handle).view(hidden_states.shape)
         routing_weights, selected = ops.route_topk(flat, weight, top_k, renorm)
