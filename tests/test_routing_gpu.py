@@ -95,3 +95,27 @@ def test_sort_without_scratch_of_more_routes_than_run_at_once(tokens, top_k, exp
     assert torch.equal(r.counts.long(), torch.bincount(flat[flat >= 0], minlength=experts))
     assert torch.equal(r.sorted_route[:n].long(), order) and torch.equal(r.route_pos.long(), pos)
     assert torch.equal(r.sorted_weight[:n], w.reshape(-1)[order])
+
+
+@pytest.mark.parametrize("experts,top_k", [(64, 8), (60, 4), (9, 8), (33, 1)])
+@pytest.mark.parametrize("tokens", [1, 2, 3, 5, 9, 150, 192, 193])
+def test_every_row_is_ranked_by_its_own_logits(experts, top_k, tokens):
+    """Whatever run of sums the logits come from: the softmax of the logits that the same call returns, ties to the lower expert.
+    A logit is the BF16 rounding of a sum that is off by 2^-20 of its terms' sizes at most, so it lies between the roundings of the ends.
+    Weights: float32 exponentials, a sum of 64 and a quotient, 2^-20 together."""
+    gen = torch.Generator(device=DEV).manual_seed(100 * experts + tokens)
+    x = torch.randn(tokens, 2048, device=DEV, generator=gen).to(torch.bfloat16)
+    weight = (torch.randn(experts, 2048, device=DEV, generator=gen) * 0.05).to(torch.bfloat16)
+    weight[experts // 2] = weight[1]
+    weight[experts - 1] = weight[0]
+    exact = x.double() @ weight.double().T
+    off = 2.0 ** -20 * (x.double().abs() @ weight.double().abs().T)
+    for renormalize in (False, True):
+        w, idx, logits = ops.route_topk(x, weight, top_k, renormalize, return_logits=True)
+        assert ((logits >= (exact - off).to(torch.bfloat16)) & (logits <= (exact + off).to(torch.bfloat16))).all()
+        order = logits.float().sort(dim=1, descending=True, stable=True).indices[:, :top_k]
+        assert torch.equal(idx, order)
+        p = logits.double().softmax(1).gather(1, order)
+        if renormalize:
+            p = p / p.sum(1, keepdim=True)
+        assert ((w.double() - p).abs() <= 2.0 ** -20 * p).all()
