@@ -112,3 +112,17 @@ def test_two_threads_first_calls_share_one_workspace(world, monkeypatch):
     world.run(4)
     kept = {slot.buffer.data_ptr() for slot in world.backend._workspaces.values()}
     assert {call[0] for call in world.calls} == kept
+
+
+@pytest.mark.parametrize("tokens", [1, 4])
+@pytest.mark.parametrize("which", ["indices", "weights"])
+def test_routes_on_another_device_are_refused(world, tokens, which):
+    """The kernels would follow a host pointer."""
+    indices, weights = torch.zeros(tokens, 8, dtype=torch.int64), torch.zeros(tokens, 8)
+    if which == "indices":
+        indices = indices.to("meta")
+    else:
+        weights = weights.to("meta")
+    with pytest.raises(RuntimeError, match="must be on the device of hidden_states"):
+        world.backend._run("olmoe", torch.zeros(tokens, 2048, dtype=torch.bfloat16), indices, weights, 0, 1)
+    assert not world.calls

@@ -373,6 +373,8 @@ class MixedTargetNativeBackend:
                 raise RuntimeError("expert_indices must use int32 or int64")
             if tuple(routing_weights.shape) != tuple(expert_indices.shape):
                 raise RuntimeError("expert_indices and routing_weights shapes must match")
+            if expert_indices.device != flat.device or routing_weights.device != flat.device:
+                raise RuntimeError("expert_indices and routing_weights must be on the device of hidden_states")
         device = flat.device
         with acquire_expert_pack(pack_handle) as reader:
             layer = self._device_layer(pack_handle, layer_index, device, reader, model)
