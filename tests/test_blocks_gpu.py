@@ -94,3 +94,22 @@ def test_block_shows_its_operator_to_modes_profilers_and_autograd(tokens):
             assert not block(leaf).requires_grad
     finally:
         custom_op.unregister_expert_pack(handle)
+
+
+@pytest.mark.parametrize("tokens", [1, 9, 300])
+def test_block_takes_activations_that_start_anywhere(tokens):
+    shape = syn.OLMOE
+    backend = native_backend.install_mixed_target_backend()
+    handle = custom_op.register_target_pack(InMemoryPack({0: "q4_group128"}))
+    try:
+        backend.preload_layer(handle, 0, DEV, random_layer(shape, "q4_group128", 3, DEV))
+        gate = SimpleNamespace(weight=syn.router_weight(1, 0, shape, skew=1.0).to(DEV), top_k=8, norm_topk_prob=False)
+        block = QuantizedMoEBlock(gate, layer_index=0, pack_handle=handle, performance_mode=True)
+        x = torch.randn(1, tokens, shape.hidden, device=DEV).to(torch.bfloat16)
+        want = block(x)
+        shifted = torch.empty(x.numel() + 1, dtype=torch.bfloat16, device=DEV)[1:].view(x.shape).copy_(x)
+        assert torch.equal(block(shifted), want)
+        weights, selected = ops.route_topk(shifted.view(tokens, -1), gate.weight, 8, False)
+        assert torch.equal(torch.ops.uma_qmoe.moe_forward(shifted, selected, weights, 0, handle, True), want)
+    finally:
+        custom_op.unregister_expert_pack(handle)

@@ -37,7 +37,7 @@ def world(monkeypatch):
     def step(layer, hidden, indices, weights, out, buffer, shared, router, renormalize, host, event, stream):
         if state.on_step:
             state.on_step(buffer)
-        state.calls.append((buffer.data_ptr(), host))
+        state.calls.append((buffer.data_ptr(), host, hidden.data_ptr()))
 
     monkeypatch.setattr(ops, "prefill_workspace", workspace)
     monkeypatch.setattr(ops, "decode_workspace", lambda layer, top_k, *_: workspace(layer, 1))
@@ -126,3 +126,12 @@ def test_routes_on_another_device_are_refused(world, tokens, which):
     with pytest.raises(RuntimeError, match="must be on the device of hidden_states"):
         world.backend._run("olmoe", torch.zeros(tokens, 2048, dtype=torch.bfloat16), indices, weights, 0, 1)
     assert not world.calls
+
+
+@pytest.mark.parametrize("tokens", [1, 4])
+@pytest.mark.parametrize("offset", [1, 4, 8])
+def test_activations_reach_the_kernels_on_a_16_byte_boundary(world, tokens, offset):
+    """A contiguous view may start anywhere in its storage."""
+    hidden = torch.zeros(tokens * 2048 + offset, dtype=torch.bfloat16)[offset:].view(tokens, 2048)
+    world.backend._run("olmoe", hidden, torch.zeros(tokens, 8, dtype=torch.int64), torch.zeros(tokens, 8), 0, 1)
+    assert world.calls[-1][2] % 16 == 0

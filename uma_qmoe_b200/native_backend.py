@@ -381,6 +381,8 @@ class MixedTargetNativeBackend:
         stream = torch._C._cuda_getCurrentRawStream(device.index)
         layer.used_on(stream, device)
         flat = flat.contiguous()
+        if flat.data_ptr() & 15:              # the kernels read 16 bytes at a time
+            flat = flat.clone()
         out = torch.empty_like(flat)
         if tokens == 0 and router is not None:
             ops.route_topk(flat, *router)     # refuses it: a router has no empty result

@@ -179,6 +179,8 @@ def route_topk(hidden: torch.Tensor, router_weight: torch.Tensor, top_k: int, re
     _require_cuda_bf16(hidden, "hidden_states")
     _require_cuda_bf16(router_weight, "router weight")
     flat = hidden.reshape(-1, hidden.shape[-1])
+    if flat.data_ptr() & 15:              # the kernels read 16 bytes at a time
+        flat = flat.clone()
     tokens, experts = flat.shape[0], router_weight.shape[0]
     w = torch.empty((tokens, top_k), dtype=torch.float32, device=hidden.device)
     idx = torch.empty((tokens, top_k), dtype=torch.int64, device=hidden.device)
