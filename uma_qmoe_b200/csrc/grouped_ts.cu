@@ -15,7 +15,7 @@
 // BF16 layers need no conversion: TMA writes the swizzled A tile to shared memory.
 //
 // Measured (B200, OLMoE shape, 64 tokens = 8 routes per expert, gate/up | down, us; the kernels of grouped.cu in brackets):
-// Q4 45 | 26 (106 | 58), Q8 70 | 38 (138 | 71) = 4.0 TB/s of codes.  What bounds the quantised encodings is the conversion:
+// Q4 46 | 27 (106 | 58), Q8 71 | 38 (138 | 71) = 4.0 TB/s of codes.  What bounds the quantised encodings is the conversion:
 // of 1850 clocks a 128-k step takes a CTA, 760 (Q4) are its arithmetic, 460 its loop, 160 the tcgen05.st.  With 64-k steps
 // and a lone lane computing descriptors the MMA issuer was the bound (1200 clocks a step for four MMAs): 54 | 29.  Qwen BF16,
 // 512 tokens: 126 | 61 (132 | 70), gate/up at 0.83 of the copy bandwidth.
